@@ -515,13 +515,20 @@ hfx_status hfx_debug_plan(const hfx_job* job, int mixed, int* ngroups, double* r
     return guarded([&] {
         if (!job || !ngroups) throw Error(HFX_ERR_INVALID, "null argument");
         const auto& groups = job->job->plan_groups(mixed != 0);
-        *ngroups = (int)groups.size();
+        const auto& team = job->job->plan_team(mixed != 0);
+        *ngroups = (int)(groups.size() + team.size());
         if (!rows) return;
         for (size_t g = 0; g < groups.size(); ++g) {
             const LaunchGroup& x = groups[g];
             double* r = rows + 10 * g;
             r[0] = x.kind; r[1] = x.pcb; r[2] = x.pck; r[3] = x.fp32 ? 1 : 0; r[4] = (double)x.n;
             r[5] = x.flops; r[6] = x.prims; r[7] = x.grid; r[8] = x.slice; r[9] = x.warps_per_cta;
+        }
+        for (size_t g = 0; g < team.size(); ++g) {
+            const TeamGroup& x = team[g];
+            double* r = rows + 10 * (groups.size() + g);
+            r[0] = 2; r[1] = x.L; r[2] = x.team; r[3] = 0; r[4] = (double)x.n;
+            r[5] = x.cost; r[6] = 0; r[7] = job->job->team_grid(x); r[8] = x.slice; r[9] = 4;
         }
     });
 }

@@ -142,21 +142,6 @@ __host__ __device__ inline Task make_task(int bra, int ket, int i0, int i1, int 
     return t;
 }
 
-// Arguments of the unique-ERI kernel (hfx_kernels.cu).
-struct LaunchArgs {
-    const DPair* pairs;
-    const PairGeo* pp_geo;
-    const double* epool;
-    const double* boys;      // [kBoysN][kBoysM]
-    const Task* tasks;
-    int ntasks;
-    int* counter;            // work-queue head (zeroed before launch)
-    int K;
-    double thr;              // BF-level Schwarz threshold (< 0: none)
-    const double* Qbf;
-    double* eri;             // packed unique ERIs, eri_index order
-};
-
 // Arguments of the small-class (thread-per-shell-quartet) kernels.
 template <typename T>
 struct SmallArgs {

@@ -203,12 +203,7 @@ void Job::init(const hfx_options& opt)
     cuda_check(cudaEventCreate(&ev1_), "event");
     cuda_check(cudaEventCreate(&evk0_), "event");
     cuda_check(cudaEventCreate(&evk1_), "event");
-    d_counter_.alloc(4);
 
-    const std::vector<double>& tab = boys_table_host();
-    d_boys_.upload(tab, stream_);
-    d_boys32_.upload(boys_table32_host(), stream_);
-    d_boys64_.upload(boys_table64_host(), stream_);
     for (int s = 0; s < 3; ++s) {
         cudaStream_t st;
         cuda_check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -226,18 +221,10 @@ void Job::init(const hfx_options& opt)
         return std::chrono::duration<double, std::milli>(b - a).count();
     };
     auto t0 = tnow();
-    build_pairs();
+    build_super();
     auto t1 = tnow();
     compute_schwarz();
     auto t2 = tnow();
-    {
-        std::vector<float> q32(qbf_.begin(), qbf_.end());
-        d_qbf32_.upload(q32, stream_);
-    }
-    // shell-pair Schwarz maxima into the device pair records (density screening)
-    for (size_t p = 0; p < dpairs_host_.size(); ++p) dpairs_host_[p].qmax = qsh_[p];
-    d_pairs_.upload(dpairs_host_, stream_);
-    d_dsh_.alloc(std::max<size_t>(1, dpairs_host_.size()));
     {
         const int F = frags_.count();
         std::vector<int> fk(F);
@@ -262,12 +249,11 @@ void Job::init(const hfx_options& opt)
         // that builds (the allocation-free entry point included) allocate nothing
         d_d32_.alloc((size_t)3 * nmat());
     }
-    d_counters_.alloc(std::max<size_t>(1, std::max(gs_fp64_.groups.size(), gs_mixed_.groups.size())));
+    d_counters_.alloc(std::max<size_t>(1, std::max(gs_fp64_.launches(), gs_mixed_.launches())));
     cuda_check(cudaStreamSynchronize(stream_), "job setup");
     if (trace)
-        std::fprintf(stderr, "job setup (K=%d): pairs %.1f ms, Schwarz %.1f ms, pair upload %.1f ms, FP64 plan %.1f ms, "
-                             "rest %.1f ms\n",
-                     basis_.K, ms(t0, t1), ms(t1, t2), ms(t2, t3), ms(t3, t4), ms(t4, tnow()));
+        std::fprintf(stderr, "job setup (K=%d): super pairs %.1f ms, Schwarz %.1f ms, FP64 plan %.1f ms, rest %.1f ms\n",
+                     basis_.K, ms(t0, t1), ms(t1, t2), ms(t3, t4), ms(t4, tnow()));
 }
 
 Job::~Job()
@@ -300,28 +286,6 @@ const std::vector<double>& boys_table_host()
     return tab;
 }
 
-const std::vector<double>& boys_table64_host()
-{
-    static const std::vector<double> t64 = [] {
-        const std::vector<double>& t = boys_table_host();
-        std::vector<double> v((size_t)(kBoys64MaxL + 1) * kBoysN * kBoys64Row, 0.0);
-        double fac = 1.0;
-        double inv_fact[7];
-        for (int j = 0; j < 7; ++j) {
-            inv_fact[j] = 1.0 / fac;
-            fac *= (double)(j + 1);
-        }
-        for (int L = 0; L <= kBoys64MaxL; ++L)
-            for (int k = 0; k < kBoysN; ++k) {
-                double* r = &v[((size_t)L * kBoysN + k) * kBoys64Row];
-                for (int j = 0; j < 7; ++j) r[j] = t[(size_t)k * kBoysM + L + j] * inv_fact[j];
-                r[7] = t[(size_t)k * kBoysM + (kBoysM - 1)];
-            }
-        return v;
-    }();
-    return t64;
-}
-
 const std::vector<float>& boys_table32_host()
 {
     static const std::vector<float> t32 = [] {
@@ -347,8 +311,7 @@ const std::vector<float>& boys_table32_host()
 // With `shape` (thread-kernel groups: bra x ket primitive-pair counts of the
 // task, 8 bits each), tasks of one cost bin are further ordered by shape, so
 // that the 32 threads of a warp run loops of the same trip counts.
-static std::vector<size_t> order_by_cost_desc(const std::vector<double>& cost,
-                                              const std::vector<unsigned short>* shape = nullptr)
+std::vector<size_t> order_by_cost_desc(const std::vector<double>& cost, const std::vector<unsigned short>* shape)
 {
     constexpr int kBins = 1024;
     const size_t n = cost.size();
@@ -382,23 +345,9 @@ static std::vector<size_t> order_by_cost_desc(const std::vector<double>& cost,
     return idx;
 }
 
-// The classes whose class kernels split their ket component pairs over
-// several threads per task (or, (dd|ss), hold 36 accumulators): in FP64 they
-// beat the warp kernel on lightly contracted quartets (benzene/cc-pVDZ build
-// 21.4 -> 17.9 ms) but not on heavily contracted ones (NaCl/cc-pVTZ 20.0 ->
-// 22.2 ms), whose quartets the plan keeps on the warp kernel.
-static bool is_ket_blocked_class(int pcb, int pck)
-{
-    static const int blocked[][2] = {{2, 2}, {3, 2}, {4, 1}, {4, 2}, {4, 3}, {4, 4}, {5, 0}, {5, 1}, {5, 2}, {5, 3}};
-    for (auto& c : blocked)
-        if (c[0] == pcb && c[1] == pck) return true;
-    return false;
-}
-
 bool is_small_class(int pcb, int pck)
 {
-    // every class up to (dd|ds) with at most d functions, in both precisions;
-    // the larger ones split their ket component pairs over several threads
+    // FP32: every class up to (dd|ds) with at most d functions; the larger ones split their ket component pairs over several threads
     // per task
     static const int small[][2] = {{0, 0}, {1, 0}, {1, 1}, {2, 0}, {2, 1}, {3, 0}, {3, 1}, {3, 3}, {4, 0},
                                    {2, 2}, {3, 2}, {4, 1}, {4, 2}, {4, 3}, {4, 4}, {5, 0}, {5, 1}, {5, 2}, {5, 3}};
@@ -444,15 +393,9 @@ const ClassTables& class_tables()
     return ct;
 }
 
-// Primitive pairs below this fraction of their shell pair's largest
-// coefficient are left out (build_pair_data).
-constexpr double kPrimPairCut = 1e-18;
-
-namespace {
-// f(i) for i in [0, n) on up to 16 host threads, indices handed out one at a
-// time; the first exception is rethrown after every thread has joined.
-template <typename F>
-void parallel_for(int n, F&& f)
+// Indices handed out one at a time; the first exception is rethrown after
+// every thread has joined.
+void host_parallel_for(int n, const std::function<void(int)>& f)
 {
     const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
     const int nt = std::min(std::min(n, hw), 16);
@@ -482,7 +425,6 @@ void parallel_for(int n, F&& f)
     for (auto& th : pool) th.join();
     if (err) std::rethrow_exception(err);
 }
-}  // namespace
 
 PairData build_pair_data(const Basis& basis, const Fragments& fr)
 {
@@ -504,7 +446,7 @@ PairData build_pair_data(const Basis& basis, const Fragments& fr)
     };
     std::vector<PairOut> outs(items.size());
     constexpr int kPairsPerUnit = 16;
-    parallel_for((int)((items.size() + kPairsPerUnit - 1) / kPairsPerUnit), [&](int u) {
+    host_parallel_for((int)((items.size() + kPairsPerUnit - 1) / kPairsPerUnit), [&](int u) {
         std::vector<double> Ex, Ey, Ez;
         const size_t i1 = std::min(items.size(), (size_t)(u + 1) * kPairsPerUnit);
         for (size_t it = (size_t)u * kPairsPerUnit; it < i1; ++it) {
@@ -645,17 +587,17 @@ PairData build_pair_data(const Basis& basis, const Fragments& fr)
     return pd;
 }
 
+// Shell-pair records of the FP32 launches; built for mixed-precision jobs.
 void Job::build_pairs()
 {
     PairData pd = build_pair_data(basis_, frags_);
-    hpairs_ = std::move(pd.hpairs);
-    dpairs_host_ = pd.dpairs;
-    d_pairs_.upload(pd.dpairs, stream_);
-    d_ppgeo_.upload(pd.geo, stream_);
-    d_epool_.upload(pd.epool, stream_);
-    d_rec64_.upload(pd.rec, stream_);
+    dpairs_host_ = std::move(pd.dpairs);
+    for (size_t p = 0; p < dpairs_host_.size(); ++p) dpairs_host_[p].qmax = qsh_[p];
+    d_pairs_.upload(dpairs_host_, stream_);
+    d_dsh_.alloc(std::max<size_t>(1, dpairs_host_.size()));
     std::vector<float> r32(pd.rec.begin(), pd.rec.end());
     d_rec32_.upload(r32, stream_);
+    d_boys32_.upload(boys_table32_host(), stream_);
     const ClassTables& ct = class_tables();
     d_pct_.upload(ct.tab, stream_);
     d_abs_.upload(ct.ab_start, stream_);
@@ -664,176 +606,284 @@ void Job::build_pairs()
     cuda_check(cudaStreamSynchronize(stream_), "pair upload");
 }
 
-LaunchArgs Job::base_args() const
+TeamArgs Job::team_args(const TeamPlanDev& plan, const TeamGroup& g, int* counter) const
 {
-    LaunchArgs a{};
-    a.pairs = d_pairs_.p;
-    a.pp_geo = d_ppgeo_.p;
-    a.epool = d_epool_.p;
-    a.boys = d_boys_.p;
-    a.counter = d_counter_.p;
-    a.K = basis_.K;
-    a.thr = opt_.screening_threshold;
-    a.Qbf = d_qbf_.p;
+    TeamArgs a{};
+    a.pairs = d_super_.p;
+    a.order = plan.order.p;
+    a.tasks = plan.tasks.p + g.off;
+    a.ntasks = (int)g.n;
+    a.counter = counter;
+    a.kcode = d_scode_.p;
+    a.ridx = reinterpret_cast<const uint4*>(d_sridx_.p);
+    std::copy(team_ridx().at, team_ridx().at + 49, a.ridx_at);
+    a.boys = team_boys_->p;
+    a.slice = g.slice;
     return a;
 }
 
-void Job::run_eri_tasks(const DevBuf<Task>& tasks, int ntasks, int maxacc, int maxw, int maxr, LaunchArgs a)
+void team_thresholds(TeamArgs& a, double thr, double dthr)
 {
-    if (ntasks == 0) return;
-    a.tasks = tasks.p;
-    a.ntasks = ntasks;
-    cuda_check(cudaMemsetAsync(d_counter_.p, 0, sizeof(int), stream_), "memset counter");
-    size_t sm = generic_smem_bytes(maxacc, maxw, maxr);
-    int per_sm = (int)std::max<size_t>(1, std::min<size_t>(16, (220 * 1024) / std::max<size_t>(sm, 1)));
-    int grid = std::min(ntasks, nsm_ * per_sm);
-    cuda_check(launch_eri(a, maxacc, maxw, maxr, grid, stream_), "ERI kernel launch");
+    a.thr = thr;
+    a.screen = thr >= 0.0;
+    a.thr_lo = (float)(thr * 0.99999);
+    a.thr_hi = (float)(thr * 1.00001);
+    a.dthr = dthr;
+    a.dscreen = dthr > 0.0;
 }
 
+void TeamPlanDev::upload(const TeamPlanHost& h, cudaStream_t st)
+{
+    groups = h.groups;
+    tasks.upload(h.tasks, st);
+    order.upload(h.order, st);
+}
+
+// One launch per group of `plan`, in order on the main stream.
+void Job::run_team(const TeamPlanDev& plan, int mode, double thr, double* out)
+{
+    DevBuf<int> ctr;
+    ctr.alloc(std::max<size_t>(1, plan.groups.size()));
+    cuda_check(cudaMemsetAsync(ctr.p, 0, sizeof(int) * ctr.n, stream_), "memset counters");
+    StreamSink sk = stream_sink();
+    sk.fork();
+    for (size_t gi = 0; gi < plan.groups.size(); ++gi) {
+        TeamArgs a = team_args(plan, plan.groups[gi], ctr.p + gi);
+        a.mode = mode;
+        team_thresholds(a, thr, 0.0);
+        a.out = out;
+        KernelSpec ks;
+        cuda_check(team_spec(plan.groups[gi], nsm_, &ks), "team kernel");
+        void* prm[] = {&a};
+        sk.kernel((int)(gi % (aux_.size() + 1)), ks, prm);
+    }
+    sk.join();
+    cuda_check(cudaStreamSynchronize(stream_), "team kernel");
+}
+
+// Schwarz bounds from the diagonal quartets of the super pairs.
 void Job::compute_schwarz()
 {
-    // Diagonal shell quartets (AB|AB) on the warp kernel (NK = 0 writes the
-    // BF-pair bounds sqrt((ab|ab)) and the per-pair maximum), tiered by the
-    // shared-memory slice each class needs.
-    const int np = (int)hpairs_.size();
-    size_t npair_bf = (size_t)frags_.qoff.back();
+    const size_t npair_bf = (size_t)frags_.qoff.back();
     d_qbf_.alloc(npair_bf);
-    d_qsh_.alloc(np);
+    d_qbf32_.alloc(npair_bf);
     cuda_check(cudaMemsetAsync(d_qbf_.p, 0, npair_bf * sizeof(double), stream_), "memset");
-    cuda_check(cudaMemsetAsync(d_qsh_.p, 0, np * sizeof(unsigned long long), stream_), "memset");
-    std::map<int, std::vector<Task>> tiers;
-    std::map<int, int> tier_slice;
-    for (int p = 0; p < np; ++p) {
-        const HostPair& h = hpairs_[p];
-        int sl = warp_slice_elems(h.l0, h.l1, h.l0, h.l1, h.npp, kDefaultLaneMinNpp);
-        int tier = 0;
-        while ((512 << tier) < sl) ++tier;
-        tiers[tier].push_back(make_task(p, p, 0, h.npp, 0, h.npp));   // whole quartet: the pass writes, not adds
-        tier_slice[tier] = std::max(tier_slice[tier], sl);
-    }
-    std::vector<DevBuf<Task>> dts(tiers.size());
-    DevBuf<int> ctr;
-    ctr.alloc(tiers.size());
-    cuda_check(cudaMemsetAsync(ctr.p, 0, sizeof(int) * tiers.size(), stream_), "memset");
-    size_t ti = 0;
-    for (auto& kv : tiers) {
-        dts[ti].upload(kv.second, stream_);
-        const int slice = (tier_slice[kv.first] + 1) & ~1;
-        const int wpc = (int)std::max<size_t>(1, std::min<size_t>(8, (200 * 1024 - kWarpSmemHeader) / (slice * sizeof(double))));
-        const size_t sm = kWarpSmemHeader + sizeof(double) * (size_t)slice * wpc;
-        const int ctas_per_sm = (int)std::max<size_t>(1, (228 * 1024) / (sm + 1024));
-        const long long need = ((long long)kv.second.size() + wpc - 1) / wpc;
-        const int grid = (int)std::min<long long>(need, (long long)nsm_ * ctas_per_sm);
-        WarpArgs<double> a{};
-        a.pairs = d_pairs_.p;
-        a.rec = d_rec64_.p;
-        a.pct = d_pct_.p;
-        a.ab_start = d_abs_.p;
-        a.k_herm = d_kh_.p;
-        a.k_lin = d_kl_.p;
-        a.tasks = dts[ti].p;
-        a.ntasks = (int)kv.second.size();
-        a.counter = ctr.p + ti;
-        a.boys = d_boys64_.p;
-        a.thr = -1.0;
-        a.K = basis_.K;
-        a.slice = slice;
-        a.lane_min_npp = kDefaultLaneMinNpp;
-        a.Qout_bf = d_qbf_.p;
-        a.Qout_sh = d_qsh_.p;
-        cuda_check(launch_warp(false, &a, 0, grid, wpc, stream_), "schwarz launch");
-        ++ti;
+    cuda_check(cudaMemsetAsync(d_qbf32_.p, 0, npair_bf * sizeof(float), stream_), "memset");
+    const TeamPlanHost h = build_team_diagonal(sup_, nsm_);
+    TeamPlanDev plan;
+    plan.upload(h, stream_);
+    DevBuf<double> part;
+    DevBuf<int> first;
+    DevBuf<long long> qoff;
+    part.alloc(std::max(1, h.first.back()));
+    first.upload(h.first, stream_);
+    qoff.upload(frags_.qoff, stream_);
+    run_team(plan, kTeamDiag, -1.0, part.p);
+    {
+        const SuperPair* pr = d_super_.p;
+        int np = (int)sup_.pairs.size();
+        const int* fi = first.p;
+        const double* pa = part.p;
+        const long long* qo = qoff.p;
+        double* q = d_qbf_.p;
+        float* q32 = d_qbf32_.p;
+        void* prm[] = {&pr, &np, &fi, &pa, &qo, &q, &q32};
+        KernelSpec ks = team_bounds_spec(np);
+        cuda_check(cudaLaunchKernel(ks.func, ks.grid, ks.block, prm, 0, stream_), "Schwarz bounds");
     }
     qbf_.resize(npair_bf);
-    std::vector<unsigned long long> qs(np);
     cuda_check(cudaMemcpyAsync(qbf_.data(), d_qbf_.p, npair_bf * sizeof(double), cudaMemcpyDeviceToHost, stream_),
                "download Q");
-    cuda_check(cudaMemcpyAsync(qs.data(), d_qsh_.p, np * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream_),
-               "download Q");
     cuda_check(cudaStreamSynchronize(stream_), "schwarz");
-    qsh_.resize(np);
-    for (int p = 0; p < np; ++p) {
-        double v;
-        std::memcpy(&v, &qs[p], sizeof(double));
-        qsh_[p] = v;
+    // per shell pair, per super pair: the largest
+    qsh_.assign(hpairs_.size(), 0.0);
+    for (size_t p = 0; p < hpairs_.size(); ++p) {
+        const HostPair& h2 = hpairs_[p];
+        const double* Q = qbf_.data() + frags_.qoff[h2.frag];
+        const int b0 = frags_.bf[h2.frag];
+        const Shell &s0 = basis_.shells[h2.s0], &s1 = basis_.shells[h2.s1];
+        for (int i = s0.bf0 - b0; i < s0.bf0 - b0 + ncart(s0.L); ++i)
+            for (int j = s1.bf0 - b0; j < s1.bf0 - b0 + ncart(s1.L); ++j)
+                qsh_[p] = std::max(qsh_[p], Q[(long long)std::max(i, j) * (std::max(i, j) + 1) / 2 + std::min(i, j)]);
     }
+    qsup_.assign(sup_.pairs.size(), 0.0);
+    for (size_t p = 0; p < sup_.pairs.size(); ++p) {
+        for (int m : sup_.members[p]) qsup_[p] = std::max(qsup_[p], qsh_[m]);
+        SuperPair& d = sup_.pairs[p];
+        d.qmax = qsup_[p];
+        d.Qbf = d_qbf_.p + frags_.qoff[d.frag];
+        d.Qbf32 = d_qbf32_.p + frags_.qoff[d.frag];
+    }
+    std::vector<double> mq;
+    std::vector<size_t> at(sup_.pairs.size());
+    for (size_t p = 0; p < sup_.pairs.size(); ++p) {
+        at[p] = mq.size();
+        const SuperPair& d = sup_.pairs[p];
+        // members of one super shell with itself: only the ordered ones exist
+        mq.resize(mq.size() + d.nmem, 0.0);
+        for (size_t m = 0; m < sup_.members[p].size(); ++m)
+            mq[at[p] + sup_.member_at[p][m]] = qsh_[sup_.members[p][m]];
+    }
+    d_smq_.upload(mq, stream_);
+    for (size_t p = 0; p < sup_.pairs.size(); ++p) sup_.pairs[p].mq = d_smq_.p + at[p];
+    d_super_.upload(sup_.pairs, stream_);
+    cuda_check(cudaStreamSynchronize(stream_), "super pair upload");
 }
 
 void Job::schwarz_host(std::vector<double>& Q) const { Q = qbf_; }
 
-// Calls f(X, Y) for every unique shell-pair pair X >= Y of the same molecule
-// with Q_X Q_Y >= thr (all pairs if thr < 0), visiting only the survivors:
-// a molecule's pairs are scanned in decreasing Q order and the scan for X
-// stops at the first Q_Y below thr / Q_X.
-template <typename F>
-void Job::for_each_surviving_quartet(double thr, F&& f) const
+// Super pairs of the job and their device tables; the shell pairs' list.
+void Job::build_super()
 {
-    for (int fr = 0; fr < frags_.count(); ++fr) {
-        const int p0 = frags_.pbase[fr], p1 = frags_.pbase[fr + 1];
-        if (thr < 0.0) {
-            for (int X = p0; X < p1; ++X)
-                for (int Y = p0; Y <= X; ++Y) f(X, Y);
-            continue;
-        }
-        std::vector<int> order(p1 - p0);
-        std::iota(order.begin(), order.end(), p0);
-        std::sort(order.begin(), order.end(), [&](int a, int b) { return qsh_[a] > qsh_[b]; });
-        for (int X = p0; X < p1; ++X) {
-            if (qsh_[X] <= 0.0) continue;
-            const double need = thr / qsh_[X];
-            for (int Y : order) {
-                if (qsh_[Y] < need) break;
-                if (Y <= X) f(X, Y);
+    sup_ = build_super_data(basis_, frags_);
+    const size_t np = sup_.pairs.size();
+    hpairs_.clear();
+    for (int f = 0; f < frags_.count(); ++f)
+        for (int A = frags_.sh[f]; A < frags_.sh[f + 1]; ++A)
+            for (int B = frags_.sh[f]; B <= A; ++B) {
+                const bool swap = basis_.shells[A].L < basis_.shells[B].L;
+                HostPair h{};
+                h.frag = f;
+                h.s0 = swap ? B : A;
+                h.s1 = swap ? A : B;
+                h.l0 = basis_.shells[h.s0].L;
+                h.l1 = basis_.shells[h.s1].L;
+                h.same = A == B;
+                hpairs_.push_back(h);
             }
+    for (size_t p = 0; p < np; ++p)
+        for (size_t m = 0; m < sup_.members[p].size(); ++m) {
+            hpairs_[sup_.members[p][m]].npp = sup_.member_npp[p][m];
         }
+    d_shdr_.upload(sup_.hdr, stream_);
+    d_scoef_.upload(sup_.coef, stream_);
+    d_stab_.upload(sup_.tab, stream_);
+    d_stypes_.upload(sup_.types, stream_);
+    d_scode_.upload(team_codes(), stream_);
+    d_sridx_.upload(team_ridx().words, stream_);
+    for (size_t p = 0; p < np; ++p) {
+        SuperPair& d = sup_.pairs[p];
+        d.hdr = d_shdr_.p + (size_t)d.hdr;
+        d.coef = d_scoef_.p + (size_t)d.coef;
+        d.tab = d_stab_.p + (size_t)d.tab;
+        d.type = d_stypes_.p + (size_t)d.type;
     }
+    d_super_.upload(sup_.pairs, stream_);
+    d_tdsh_.alloc(std::max<size_t>(1, np));
+    team_boys_ = team_boys_device(device_, stream_);
+    cuda_check(cudaStreamSynchronize(stream_), "super pair upload");
+    for (auto* v : {&sup_.hdr, &sup_.coef}) std::vector<double>().swap(*v);
+    std::vector<int>().swap(sup_.tab);
 }
 
-void Job::build_tasks(double thr, std::vector<Task>& tasks, int& maxacc, int& maxw, int& maxr, double* flops,
-                      double* prims) const
+std::shared_ptr<DevBuf<double>> team_boys_device(int device, cudaStream_t st)
 {
-    // order pairs so that the pair with the larger (L, l0) is the bra
-    auto key = [&](int p) { return (hpairs_[p].l0 + hpairs_[p].l1) * 16 + hpairs_[p].l0; };
-    std::vector<double> cost;
-    tasks.clear();
-    maxacc = maxw = maxr = 1;
-    for_each_surviving_quartet(thr, [&](int X, int Y) {
-        int bra = X, ket = Y;
-        if (key(Y) > key(X)) std::swap(bra, ket);
-        tasks.push_back(make_task(bra, ket, 0, hpairs_[bra].npp, 0, hpairs_[ket].npp));
-    });
-    std::vector<double> c(tasks.size());
-    double fsum = 0.0, psum = 0.0;
-    for (size_t t = 0; t < tasks.size(); ++t) {
-        const HostPair& b = hpairs_[tasks[t].bra];
-        const HostPair& k = hpairs_[tasks[t].ket];
-        c[t] = (double)b.npp * k.npp * flops_per_prim(b.l0, b.l1, k.l0, k.l1);
-        fsum += c[t];
-        psum += (double)b.npp * k.npp;
-        int L1 = b.l0 + b.l1, L2 = k.l0 + k.l1;
-        int nab = ncart(b.l0) * ncart(b.l1), ncd = ncart(k.l0) * ncart(k.l1);
-        maxacc = std::max(maxacc, nab * ncd);
-        maxw = std::max(maxw, nherm(L1) * ncd);
-        maxr = std::max(maxr, nherm(L1 + L2));
+    static std::mutex mu;
+    static std::map<int, std::weak_ptr<DevBuf<double>>> tables;
+    std::lock_guard<std::mutex> lk(mu);
+    std::shared_ptr<DevBuf<double>> t = tables[device].lock();
+    if (!t) {
+        t = std::make_shared<DevBuf<double>>();
+        t->upload(team_boys_host(), st);
+        cuda_check(cudaStreamSynchronize(st), "Boys table upload");
+        tables[device] = t;
     }
-    if (flops) *flops = fsum;
-    if (prims) *prims = psum;
-    std::vector<size_t> idx(tasks.size());
-    std::iota(idx.begin(), idx.end(), 0);
-    std::stable_sort(idx.begin(), idx.end(), [&](size_t x, size_t y) { return c[x] > c[y]; });
-    std::vector<Task> sorted(tasks.size());
-    for (size_t t = 0; t < idx.size(); ++t) sorted[t] = tasks[idx[t]];
-    tasks.swap(sorted);
+    return t;
 }
 
+// Surviving shell quartets, their primitive quartets and algorithmic flops,
+// counted per class pair on bounds sorted in decreasing order (every quartet
+// is one unordered pair of a molecule's shell pairs with Q_X Q_Y >= thr).
+void Job::count_quartets(GroupSet& gs) const
+{
+    const double thr = opt_.screening_threshold;
+    constexpr int kPC = (kMaxL + 1) * (kMaxL + 2) / 2;
+    double quartets = 0.0;
+    gs.prims = gs.flops64 = 0.0;
+    for (int fr = 0; fr < frags_.count(); ++fr) {
+        struct Entry {
+            double q, npp;
+        };
+        std::vector<Entry> cls[kPC];
+        int l0[kPC], l1[kPC];
+        for (int p = frags_.pbase[fr]; p < frags_.pbase[fr + 1]; ++p) {
+            const HostPair& h = hpairs_[p];
+            const int c = pair_class(h.l0, h.l1);
+            l0[c] = h.l0;
+            l1[c] = h.l1;
+            if (qsh_[p] > 0.0) cls[c].push_back({qsh_[p], (double)h.npp});
+        }
+        std::vector<double> sum[kPC];
+        for (int c = 0; c < kPC; ++c) {
+            std::sort(cls[c].begin(), cls[c].end(), [](const Entry& a, const Entry& b) { return a.q > b.q; });
+            sum[c].assign(1, 0.0);
+            for (const Entry& e : cls[c]) sum[c].push_back(sum[c].back() + e.npp);
+        }
+        for (int a = 0; a < kPC; ++a)
+            for (int b = 0; b <= a; ++b) {
+                if (cls[a].empty() || cls[b].empty()) continue;
+                double n = 0.0, pr = 0.0;
+                size_t m = cls[b].size();
+                for (const Entry& e : cls[a]) {
+                    while (m > 0 && cls[b][m - 1].q < thr / e.q) --m;
+                    n += (double)m;
+                    pr += e.npp * sum[b][m];
+                }
+                if (a == b) {
+                    for (const Entry& e : cls[a])
+                        if (e.q >= thr / e.q) {
+                            n += 1.0;
+                            pr += e.npp * e.npp;
+                        }
+                    n *= 0.5;
+                    pr *= 0.5;
+                }
+                quartets += n;
+                gs.prims += pr;
+                gs.flops64 += pr * flops_per_prim(l0[a], l1[a], l0[b], l1[b]);
+            }
+    }
+    gs.nquartets = (int)quartets;
+}
 
-// FP64 quartets of the ket-blocked classes with more primitive quartets than
-// this run on the warp kernel.
-constexpr long long kKetBlockMaxPrims64 = 64;
+int Job::team_grid(const TeamGroup& g) const
+{
+    KernelSpec ks;
+    cuda_check(team_spec(g, nsm_, &ks), "team kernel");
+    return (int)ks.grid.x;
+}
 
+// The plan of one precision mode: FP64 quartets as tasks of the team kernel
+// over super pairs, and in a mixed plan the FP32 quartets (those whose own
+// bound is below the FP32 cut) as shell-quartet launch groups; the team kernel
+// leaves these out of the super quartets' digestion.
 void Job::build_jk_groups(bool mixed, GroupSet& gs)
 {
     clear_graphs();   // graphs hold the previous plan's task pointers
+    gs.groups.clear();
+    gs.ntasks = 0;
+    gs.flops32 = gs.quartets32 = 0.0;
+    if (mixed && dpairs_host_.empty()) build_pairs();
+    if (mixed) build_fp32_groups(gs);
+    const auto t0 = std::chrono::steady_clock::now();
+    count_quartets(gs);
+    gs.flops64 -= gs.flops32;
+    if (mixed) {
+        for (SuperPair& d : sup_.pairs) d.cut32 = opt_.fp32_threshold;
+        d_super_.upload(sup_.pairs, stream_);
+    }
+    const double thr = opt_.screening_threshold, tau = opt_.fp32_threshold;
+    TeamPlanHost tp = build_team_plan(sup_, qsup_, mixed ? std::max(thr, tau) : thr, nsm_);
+    gs.team.upload(tp, stream_);
+    cuda_check(cudaStreamSynchronize(stream_), "plan upload");
+    if (std::getenv("HFX_TRACE_SETUP"))
+        std::fprintf(stderr, "team plan (%s): %zu tasks, %zu launches, %.1f ms\n", mixed ? "mixed" : "fp64",
+                     tp.tasks.size(), tp.groups.size(),
+                     std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
+}
+
+void Job::build_fp32_groups(GroupSet& gs)
+{
     const double thr = opt_.screening_threshold;
     const double tau = opt_.fp32_threshold;
     const int np = (int)hpairs_.size();
@@ -849,17 +899,14 @@ void Job::build_jk_groups(bool mixed, GroupSet& gs)
             pl1[pair_class(l0, l1)] = l1;
         }
     bool small_ok[kPC][kPC];
-    bool ket_blocked[kPC][kPC];   // the ten classes beyond the nine single-block ones
     double fpp_tab[kPC][kPC];
     for (int a = 0; a < kPC; ++a)
         for (int b = 0; b < kPC; ++b) {
             small_ok[a][b] = is_small_class(a, b);
-            ket_blocked[a][b] = is_ket_blocked_class(a, b);
             fpp_tab[a][b] = flops_per_prim(pl0[a], pl1[a], pl0[b], pl1[b]);
         }
-    // buckets: small classes per (fp32, pcb, pck) at fp32 * 100 + pcb * 10 + pck;
-    // the warp kernel's per fp32 at kWarpBucket + fp32
-    constexpr int kWarpBucket = 200, kBuckets = 202;
+    // buckets: small classes per (pcb, pck) at pcb * 10 + pck, then the warp kernel's
+    constexpr int kWarpBucket = 100, kBuckets = 101;
     // Work units of the enumeration: ranges of bra-side shell pairs X of one
     // molecule.  Every unit lists its surviving quartets per bucket in the
     // serial visiting order (X ascending, Y by decreasing Schwarz bound), so
@@ -891,7 +938,7 @@ void Job::build_jk_groups(bool mixed, GroupSet& gs)
     }
     const int nu = (int)units.size();
     const auto tp0 = std::chrono::steady_clock::now();
-    parallel_for(nu, [&](int u) {
+    host_parallel_for(nu, [&](int u) {
         Unit& un = units[u];
         un.q.resize(kBuckets);
         un.prims.assign(kBuckets, 0.0);
@@ -902,18 +949,10 @@ void Job::build_jk_groups(bool mixed, GroupSet& gs)
             for (int Y : order) {
                 if (qsh_[Y] < need) break;
                 if (Y > X) continue;
-                const double bound = qsh_[X] * qsh_[Y];
+                if (qsh_[X] * qsh_[Y] >= tau) continue;   // FP64
                 int bra = X, ket = Y;
                 if (pcls[Y] > pcls[X]) std::swap(bra, ket);
-                const int f32 = mixed && bound < tau ? 1 : 0;
-                const int pcb = pcls[bra], pck = pcls[ket];
-                // FP64 quartets of the ket-block classes with many primitive
-                // quartets go to the warp kernel: every ket block of a class
-                // kernel task recomputes R and the Boys function
-                const bool sm = small_ok[pcb][pck] &&
-                                (f32 || !ket_blocked[pcb][pck] ||
-                                 (long long)hpairs_[bra].npp * hpairs_[ket].npp <= kKetBlockMaxPrims64);
-                const int b = sm ? f32 * 100 + pcb * 10 + pck : kWarpBucket + f32;
+                const int b = small_ok[pcls[bra]][pcls[ket]] ? pcls[bra] * 10 + pcls[ket] : kWarpBucket;
                 un.q[b].push_back({bra, ket});
                 un.prims[b] += (double)hpairs_[bra].npp * hpairs_[ket].npp;
             }
@@ -945,7 +984,7 @@ void Job::build_jk_groups(bool mixed, GroupSet& gs)
                                        std::min<long long>(cap, (long long)std::ceil(bprims[b] / fill)));
     }
     const auto tp1 = std::chrono::steady_clock::now();
-    parallel_for(nu, [&](int u) {
+    host_parallel_for(nu, [&](int u) {
         Unit& un = units[u];
         un.t.resize(kBuckets);
         un.cost.resize(kBuckets);
@@ -985,7 +1024,7 @@ void Job::build_jk_groups(bool mixed, GroupSet& gs)
     };
     std::vector<Bucket> bk(kBuckets);
     const auto tp2 = std::chrono::steady_clock::now();
-    parallel_for(kBuckets, [&](int b) {
+    host_parallel_for(kBuckets, [&](int b) {
         size_t n = 0;
         for (const Unit& un : units) n += un.t[b].size();
         if (n == 0) return;
@@ -1016,27 +1055,24 @@ void Job::build_jk_groups(bool mixed, GroupSet& gs)
     std::vector<LaunchGroup>& groups = gs.groups;
     groups.clear();
     std::vector<Span> spans;
-    for (int f = 0; f < 2; ++f)
-        for (int pcb = 0; pcb < 10; ++pcb)
-            for (int pck = 0; pck <= pcb; ++pck) {
-                const int b = f * 100 + pcb * 10 + pck;
-                if (bk[b].t.empty()) continue;
-                LaunchGroup g{};
-                g.kind = 0;
-                g.pcb = pcb;
-                g.pck = pck;
-                g.fp32 = f == 1;
-                g.n = bk[b].t.size();
-                groups.push_back(g);
-                spans.push_back(Span{b, {}});
-            }
-    const size_t elem[2] = {sizeof(double), sizeof(float)};
-    for (int f = 0; f < 2; ++f) {
-        const Bucket& B = bk[kWarpBucket + f];
-        if (B.t.empty()) continue;
+    for (int pcb = 0; pcb < 10; ++pcb)
+        for (int pck = 0; pck <= pcb; ++pck) {
+            const int b = pcb * 10 + pck;
+            if (bk[b].t.empty()) continue;
+            LaunchGroup g{};
+            g.kind = 0;
+            g.pcb = pcb;
+            g.pck = pck;
+            g.fp32 = true;
+            g.n = bk[b].t.size();
+            groups.push_back(g);
+            spans.push_back(Span{b, {}});
+        }
+    if (!bk[kWarpBucket].t.empty()) {
+        const Bucket& B = bk[kWarpBucket];
         const size_t n = B.t.size();
         std::vector<int> sl(n);
-        parallel_for((int)((n + 65535) / 65536), [&](int c) {
+        host_parallel_for((int)((n + 65535) / 65536), [&](int c) {
             for (size_t i = (size_t)c * 65536; i < std::min(n, (size_t)(c + 1) * 65536); ++i) {
                 const HostPair& hb = hpairs_[B.t[i].bra];
                 const HostPair& hk = hpairs_[B.t[i].ket];
@@ -1054,18 +1090,18 @@ void Job::build_jk_groups(bool mixed, GroupSet& gs)
         for (auto& kv : tiers) {
             LaunchGroup g{};
             g.kind = 1;
-            g.fp32 = f == 1;
+            g.fp32 = true;
             g.n = kv.second.first.size();
             g.slice = (kv.second.second + 1) & ~1;
             g.lane_min_npp = shape_.lane_min_npp;
             g.warps_per_cta = (int)std::max<size_t>(
-                1, std::min<size_t>((size_t)shape_.warp_max_warps, (200 * 1024 - kWarpSmemHeader) / (g.slice * elem[f])));
-            size_t sm = kWarpSmemHeader + elem[f] * (size_t)g.slice * g.warps_per_cta;
+                1, std::min<size_t>((size_t)shape_.warp_max_warps, (200 * 1024 - kWarpSmemHeader) / (g.slice * sizeof(float))));
+            size_t sm = kWarpSmemHeader + sizeof(float) * (size_t)g.slice * g.warps_per_cta;
             int ctas_per_sm = (int)std::max<size_t>(1, (228 * 1024) / (sm + 1024));
             long long need = ((long long)g.n + g.warps_per_cta - 1) / g.warps_per_cta;
             g.grid = (int)std::min<long long>(need, (long long)nsm_ * ctas_per_sm);
             groups.push_back(g);
-            spans.push_back(Span{kWarpBucket + f, std::move(kv.second.first)});
+            spans.push_back(Span{kWarpBucket, std::move(kv.second.first)});
         }
     }
     size_t total = 0;
@@ -1086,7 +1122,7 @@ void Job::build_jk_groups(bool mixed, GroupSet& gs)
         for (size_t r = 0; r < groups[gi].n; r += 65536)
             chunks.push_back(Chunk{gi, r, std::min(groups[gi].n, r + 65536)});
     std::unique_ptr<Task[]> all(new Task[std::max<size_t>(1, total)]);
-    parallel_for((int)chunks.size(), [&](int c) {
+    host_parallel_for((int)chunks.size(), [&](int c) {
         Chunk& ch = chunks[c];
         const Span& sp = spans[ch.group];
         const Bucket& B = bk[sp.bucket];
@@ -1100,21 +1136,12 @@ void Job::build_jk_groups(bool mixed, GroupSet& gs)
             if (t.i0 == 0 && t.k0 == 0) ++ch.whole;
         }
     });
-    gs.flops64 = gs.flops32 = gs.prims = gs.quartets32 = 0.0;
-    gs.nquartets = 0;
     for (const Chunk& ch : chunks) {
         LaunchGroup& g = groups[ch.group];
         g.flops += ch.flops;
         g.prims += ch.prims;
-        gs.nquartets += (int)ch.whole;
-        if (g.fp32) gs.quartets32 += (double)ch.whole;
-    }
-    for (const auto& g : groups) {
-        if (g.fp32)
-            gs.flops32 += g.flops;
-        else
-            gs.flops64 += g.flops;
-        gs.prims += g.prims;
+        gs.quartets32 += (double)ch.whole;
+        gs.flops32 += ch.flops;
     }
     gs.ntasks = (int)total;
     const auto tp4 = std::chrono::steady_clock::now();
@@ -1129,8 +1156,8 @@ void Job::build_jk_groups(bool mixed, GroupSet& gs)
             return std::chrono::duration<double, std::milli>(b - a).count();
         };
         const auto tp5 = std::chrono::steady_clock::now();
-        std::fprintf(stderr, "plan (%s, %d tasks): enumerate %.1f ms, tile %.1f ms, order %.1f ms, assemble %.1f ms, "
-                             "upload %.1f ms\n", mixed ? "mixed" : "fp64", gs.ntasks, ms(tp0, tp1), ms(tp1, tp2),
+        std::fprintf(stderr, "FP32 plan (%d tasks): enumerate %.1f ms, tile %.1f ms, order %.1f ms, assemble %.1f ms, "
+                             "upload %.1f ms\n", gs.ntasks, ms(tp0, tp1), ms(tp1, tp2),
                      ms(tp2, tp3), ms(tp3, tp4), ms(tp4, tp5));
     }
 }
@@ -1234,7 +1261,8 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
     const double* Dsh = nullptr;
     int K = basis_.K;
     const unsigned char* active = d_active_.p;
-    if (dthr > 0.0 && !dpairs_host_.empty()) {
+    const double* Tsh = nullptr;
+    if (dthr > 0.0 && !groups.empty()) {
         const DPair* pr = d_pairs_.p;
         int np = (int)dpairs_host_.size();
         double* out = d_dsh_.p;
@@ -1242,10 +1270,18 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
         sk.kernel(0, density_blocks_spec(np), prm);
         Dsh = d_dsh_.p;
     }
+    if (dthr > 0.0 && !gs.team.groups.empty()) {
+        const SuperPair* pr = d_super_.p;
+        int np = (int)sup_.pairs.size();
+        double* out = d_tdsh_.p;
+        void* prm[] = {&pr, &np, &Dk, &Dk2, &out};
+        sk.kernel(0, team_density_spec(np), prm);
+        Tsh = d_tdsh_.p;
+    }
     // float copies of the densities for the FP32 groups' block digestion
     const float *Dj32 = nullptr, *Dk32 = nullptr, *Dk232 = nullptr;
     bool any32 = false;
-    for (const auto& g : groups) any32 = any32 || (g.fp32 && g.n > 0);
+    for (const auto& g : groups) any32 = any32 || g.n > 0;
     if (any32) {
         long long n = nmat();
         d_d32_.alloc((size_t)3 * n);
@@ -1271,12 +1307,31 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
         Dk232 = dst[2];
     }
     int* ctr = counters ? counters : d_counters_.p;
-    sk.zero(0, ctr, sizeof(int) * std::max<size_t>(1, groups.size()));
+    sk.zero(0, ctr, sizeof(int) * std::max<size_t>(1, gs.launches()));
     sk.fork();
-    // warp groups (the long ones) on the main lane, small classes spread over
-    // the others (running the FP32 warp groups on a lane of their own, beside
-    // the FP64 ones, measured slower: the persistent grids contend for SMs)
     const int naux = (int)aux_.size();
+    // FP64: the team kernel's launches over all lanes, the largest first
+    for (size_t gi = 0; gi < gs.team.groups.size(); ++gi) {
+        const TeamGroup& g = gs.team.groups[gi];
+        KernelSpec ks;
+        cuda_check(team_spec(g, nsm_, &ks), "team kernel");
+        TeamArgs a = team_args(gs.team, g, ctr + groups.size() + gi);
+        a.mode = kTeamFock;
+        a.mixed = mixed_plan && mixed();
+        a.Dj = Dj;
+        a.Dk = Dk;
+        a.Dk2 = Dk2;
+        a.J = J;
+        a.Kx = Kx;
+        a.Kx2 = Kx2;
+        a.Dsh = Tsh;
+        team_thresholds(a, opt_.screening_threshold, dthr);
+        a.active = active;
+        a.nk = nk;
+        void* prm[] = {&a};
+        sk.kernel((int)(gi % (naux + 1)), ks, prm);
+    }
+    // FP32: warp groups on the main lane, small classes spread over the others
     int next_aux = 0;
     for (size_t gi = 0; gi < groups.size(); ++gi) {
         const LaunchGroup& g = groups[gi];
@@ -1285,40 +1340,19 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
         if (g.kind == 0) {
             const int lane = 1 + next_aux;
             next_aux = (next_aux + 1) % naux;
-            if (g.fp32) {
-                SmallArgs<float> a{d_pairs_.p, d_rec32_.p, tasks + g.off, (int)g.n, d_boys32_.p,
-                                   opt_.screening_threshold, d_qbf_.p, K, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr, active,
-                                   Dj32, Dk32, Dk232, d_qbf32_.p};
-                cuda_check(small_spec_f32(g.pcb, g.pck, nk, (int)g.n, &ks), "small-class kernel");
-                void* prm[] = {&a};
-                sk.kernel(lane, ks, prm);
-            } else {
-                SmallArgs<double> a{d_pairs_.p, d_rec64_.p, tasks + g.off, (int)g.n, d_boys64_.p,
-                                    opt_.screening_threshold, d_qbf_.p, K, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr,
-                                    active, nullptr, nullptr, nullptr};
-                cuda_check(small_spec_f64(g.pcb, g.pck, nk, (int)g.n, &ks), "small-class kernel");
-                void* prm[] = {&a};
-                sk.kernel(lane, ks, prm);
-            }
+            SmallArgs<float> a{d_pairs_.p, d_rec32_.p, tasks + g.off, (int)g.n, d_boys32_.p, opt_.screening_threshold,
+                               d_qbf_.p, K, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, d_qbf32_.p};
+            cuda_check(small_spec_f32(g.pcb, g.pck, nk, (int)g.n, &ks), "small-class kernel");
+            void* prm[] = {&a};
+            sk.kernel(lane, ks, prm);
         } else {
-            cuda_check(warp_spec(g.fp32, nk, g.grid, g.warps_per_cta, g.slice, &ks), "warp kernel");
-            if (g.fp32) {
-                WarpArgs<float> a{d_pairs_.p, d_rec32_.p, d_pct_.p, d_abs_.p, d_kh_.p, d_kl_.p,
-                                  tasks + g.off, (int)g.n, ctr + gi, d_boys32_.p,
-                                  opt_.screening_threshold, d_qbf_.p, K, Dj, Dk, Dk2, J, Kx, Kx2, g.slice,
-                                  g.lane_min_npp,
-                                  Dsh, dthr, nullptr, nullptr, active, Dj32, Dk32, Dk232, d_qbf32_.p};
-                void* prm[] = {&a};
-                sk.kernel(0, ks, prm);
-            } else {
-                WarpArgs<double> a{d_pairs_.p, d_rec64_.p, d_pct_.p, d_abs_.p, d_kh_.p, d_kl_.p,
-                                   tasks + g.off, (int)g.n, ctr + gi, d_boys64_.p,
-                                   opt_.screening_threshold, d_qbf_.p, K, Dj, Dk, Dk2, J, Kx, Kx2, g.slice,
-                                   g.lane_min_npp,
-                                   Dsh, dthr, nullptr, nullptr, active, nullptr, nullptr, nullptr};
-                void* prm[] = {&a};
-                sk.kernel(0, ks, prm);
-            }
+            cuda_check(warp_spec(true, nk, g.grid, g.warps_per_cta, g.slice, &ks), "warp kernel");
+            WarpArgs<float> a{d_pairs_.p, d_rec32_.p, d_pct_.p, d_abs_.p, d_kh_.p, d_kl_.p, tasks + g.off, (int)g.n,
+                              ctr + gi, d_boys32_.p, opt_.screening_threshold, d_qbf_.p, K, Dj, Dk, Dk2, J, Kx, Kx2,
+                              g.slice, g.lane_min_npp, Dsh, dthr, nullptr, nullptr, active, Dj32, Dk32, Dk232,
+                              d_qbf32_.p};
+            void* prm[] = {&a};
+            sk.kernel(0, ks, prm);
         }
     }
     sk.join();
@@ -1447,7 +1481,7 @@ void Job::fock_rhf_device_ex(const double* dP, double* dG, bool mixed_plan, doub
     }
     cuda_check(cudaEventRecord(ev1_, stream_), "event");
     cuda_check(cudaStreamSynchronize(stream_), "fock build");
-    record_stats_plan((int)plan(mixed_plan).groups.size() + 1, plan(mixed_plan));
+    record_stats_plan((int)plan(mixed_plan).launches() + 1, plan(mixed_plan));
 }
 
 void Job::fock_rhf_device_scratch(const double* dP, double* dG, double* Jacc, double* Kacc, int* counters)
@@ -1465,7 +1499,7 @@ void Job::fock_rhf_device_scratch(const double* dP, double* dG, double* Jacc, do
     enqueue_finish_rhf(sk, Jacc, Kacc, dG);
     cuda_check(cudaEventRecord(ev1_, stream_), "event");
     cuda_check(cudaStreamSynchronize(stream_), "fock build");
-    record_stats((int)plan(mixed()).groups.size() + 1);
+    record_stats((int)plan(mixed()).launches() + 1);
 }
 
 void Job::set_launch_shape(const hfx_launch_shape& s)
@@ -1476,7 +1510,7 @@ void Job::set_launch_shape(const hfx_launch_shape& s)
     shape_ = s;
     build_jk_groups(false, gs_fp64_);
     if (mixed()) build_jk_groups(true, gs_mixed_);
-    d_counters_.alloc(std::max<size_t>(1, std::max(gs_fp64_.groups.size(), gs_mixed_.groups.size())));
+    d_counters_.alloc(std::max<size_t>(1, std::max(gs_fp64_.launches(), gs_mixed_.launches())));
 }
 
 // Coordinate search over the launch shape: for each parameter in turn (small
@@ -1546,7 +1580,7 @@ double Job::autotune_fp32_threshold(const double* P, double target_dE, double* d
     for (double tau : cand) {
         opt_.fp32_threshold = tau;
         build_jk_groups(true, gs_mixed_);
-        d_counters_.alloc(std::max<size_t>(1, std::max(gs_fp64_.groups.size(), gs_mixed_.groups.size())));
+        d_counters_.alloc(std::max<size_t>(1, std::max(gs_fp64_.launches(), gs_mixed_.launches())));
         fock_rhf_ex(P, Gm.data(), true, 0.0);
         double dE = 0.0;
         for (size_t i = 0; i < n; ++i) dE += P[i] * (Gm[i] - G64[i]);
@@ -1567,7 +1601,7 @@ double Job::autotune_fp32_threshold(const double* P, double target_dE, double* d
         opt_.fp32_threshold = tau0;
         if (mixed()) build_jk_groups(true, gs_mixed_);
     }
-    d_counters_.alloc(std::max<size_t>(1, std::max(gs_fp64_.groups.size(), gs_mixed_.groups.size())));
+    d_counters_.alloc(std::max<size_t>(1, std::max(gs_fp64_.launches(), gs_mixed_.launches())));
     if (dE_out) *dE_out = best_dE;
     if (ms64) *ms64 = t64;
     if (msmx) *msmx = best_ms;
@@ -1609,7 +1643,7 @@ void Job::fock_uhf_device_ex(const double* dPa, const double* dPb, double* dJ, d
     }
     cuda_check(cudaEventRecord(ev1_, stream_), "event");
     cuda_check(cudaStreamSynchronize(stream_), "fock build");
-    record_stats_plan((int)plan(mixed_plan).groups.size() + 2, plan(mixed_plan));
+    record_stats_plan((int)plan(mixed_plan).launches() + 2, plan(mixed_plan));
 }
 
 void Job::fock_rhf(const double* P, double* G) { fock_rhf_ex(P, G, mixed(), 0.0); }
@@ -1659,16 +1693,10 @@ void Job::eri_unique(double thr, double* out)
     DevBuf<double> d_out;
     d_out.alloc(nq);
     cuda_check(cudaMemsetAsync(d_out.p, 0, nq * sizeof(double), stream_), "memset");
-    std::vector<Task> tasks;
-    int maxacc, maxw, maxr;
-    // every quartet whose shell-level bound can pass the BF-level test
-    build_tasks(thr, tasks, maxacc, maxw, maxr);
-    DevBuf<Task> dt;
-    dt.upload(tasks, stream_);
-    LaunchArgs a = base_args();
-    a.thr = thr;
-    a.eri = d_out.p;
-    run_eri_tasks(dt, (int)tasks.size(), maxacc, maxw, maxr, a);
+    // every super quartet whose bound can pass the BF-level test
+    TeamPlanDev plan;
+    plan.upload(build_team_plan(sup_, qsup_, thr, nsm_), stream_);
+    run_team(plan, kTeamEri, thr, d_out.p);
     cuda_check(cudaMemcpyAsync(out, d_out.p, nq * sizeof(double), cudaMemcpyDeviceToHost, stream_), "D2H");
     cuda_check(cudaStreamSynchronize(stream_), "eri_unique");
 }

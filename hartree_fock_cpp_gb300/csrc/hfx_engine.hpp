@@ -4,18 +4,19 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <map>
+#include <memory>
 #include <tuple>
 #include <vector>
 
 #include "hfx_device.cuh"
 #include "hfx_internal.hpp"
+#include "hfx_team.hpp"
 
 namespace hfx {
 
 // device launch helpers (hfx_kernels.cu)
-size_t generic_smem_bytes(int maxacc, int maxw, int maxr);
-cudaError_t launch_eri(const LaunchArgs& a, int maxacc, int maxw, int maxr, int grid, cudaStream_t st);
 // symmetrisation of packed accumulators: one grid row (blockIdx.y) per
 // molecule, Kmax = the largest molecule's K
 KernelSpec finish_rhf_spec(int Kmax, int nfrag);   // k_finish_rhf(Jacc, Kacc, G, fk, fmoff, active)
@@ -24,7 +25,6 @@ KernelSpec add_spec(long long n);    // k_add(A, B, C, n)
 KernelSpec to_float_spec(long long n);   // k_to_float(A, B, n)
 KernelSpec density_blocks_spec(int npairs);   // k_density_blocks(pairs, npairs, D1, D2, Dsh)
 KernelSpec rebase_tasks_spec(long long n);    // k_rebase_tasks(tasks, n, delta): bra, ket += delta
-cudaError_t small_spec_f64(int pcb, int pck, int nk, int ntasks, KernelSpec* s);   // k_small(SmallArgs<double>)
 cudaError_t small_spec_f32(int pcb, int pck, int nk, int ntasks, KernelSpec* s);   // k_small(SmallArgs<float>)
 cudaError_t warp_spec(bool fp32, int nk, int grid, int warps_per_cta, int slice, KernelSpec* s);
 cudaError_t launch_warp(bool fp32, const void* args, int nk, int grid, int warps_per_cta, cudaStream_t st);
@@ -37,8 +37,6 @@ bool is_small_class(int pcb, int pck);
 const std::vector<double>& boys_table_host();
 // The FP32 kernels' Boys table: 8 floats per (L <= kBoys32MaxL, k), see hfx_device.cuh.
 const std::vector<float>& boys_table32_host();
-// The FP64 Fock kernels' Boys table: 8 doubles per (L <= kBoys64MaxL, k), see hfx_device.cuh.
-const std::vector<double>& boys_table64_host();
 
 void cuda_check(cudaError_t e, const char* what);
 
@@ -81,6 +79,10 @@ struct DevBuf {
         if (!v.empty()) cuda_check(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st), "upload");
     }
 };
+
+// The team kernel's Boys table on the current device, shared by the jobs and
+// sessions alive there and freed with the last of them.
+std::shared_ptr<DevBuf<double>> team_boys_device(int device, cudaStream_t st);
 
 struct HostPair {
     int frag;         // molecule of a packed job
@@ -140,10 +142,35 @@ Fragments single_fragment(const Basis& b);
 
 PairData build_pair_data(const Basis& b, const Fragments& fr);
 
+// Primitive pairs below this fraction of their shell pair's largest
+// coefficient are left out (build_pair_data, build_super_data).
+constexpr double kPrimPairCut = 1e-18;
+
+// f(i) for i in [0, n) on up to 16 host threads.
+void host_parallel_for(int n, const std::function<void(int)>& f);
+// Indices by decreasing cost (counting sort on 1/16-octave bins, stable); with
+// `shape`, equal bins are ordered by shape.
+std::vector<size_t> order_by_cost_desc(const std::vector<double>& cost,
+                                       const std::vector<unsigned short>* shape = nullptr);
+
+// Screening thresholds of a launch (density screening off at dthr = 0).
+void team_thresholds(TeamArgs& a, double thr, double dthr);
+
+// A team-kernel plan on the device.
+struct TeamPlanDev {
+    std::vector<TeamGroup> groups;
+    DevBuf<TeamTask> tasks;
+    DevBuf<int> order;
+    void upload(const TeamPlanHost& h, cudaStream_t st);
+};
+
 // The launch plan of one precision mode.
 struct GroupSet {
     std::vector<LaunchGroup> groups;
     DevBuf<Task> tasks;
+    // FP64 quartets: tasks of the team kernel over super pairs
+    TeamPlanDev team;
+    size_t launches() const { return groups.size() + team.groups.size(); }
     int ntasks = 0, nquartets = 0;
     double flops64 = 0.0, flops32 = 0.0, prims = 0.0, quartets32 = 0.0;
 };
@@ -263,9 +290,11 @@ public:
     void set_launch_shape(const hfx_launch_shape& s);
     // pick the launch shape by timing builds at density P (host, K x K); returns the best build ms
     double autotune_launch_shape(const double* P, int builds, hfx_launch_shape* out);
-    int num_launch_groups() const { return (int)plan(true).groups.size(); }
+    int num_launch_groups() const { return (int)plan(true).launches(); }
     // launch groups of a plan (FP64 or, for a mixed job, mixed)
     const std::vector<LaunchGroup>& plan_groups(bool mixed_plan) const { return plan(mixed_plan).groups; }
+    const std::vector<TeamGroup>& plan_team(bool mixed_plan) const { return plan(mixed_plan).team.groups; }
+    int team_grid(const TeamGroup& g) const;
     void fock_uhf_device(const double* dPa, const double* dPb, double* dJ, double* dKa, double* dKb);
     void fock_rhf(const double* P, double* G);
     void fock_uhf(const double* Pa, const double* Pb, double* J, double* Ka, double* Kb);
@@ -278,12 +307,8 @@ private:
     void init(const hfx_options& opt);
     void build_pairs();
     void compute_schwarz();
-    void build_tasks(double thr, std::vector<Task>& tasks, int& maxacc, int& maxw, int& maxr, double* flops = nullptr,
-                     double* prims = nullptr) const;
-    void run_eri_tasks(const DevBuf<Task>& tasks, int ntasks, int maxacc, int maxw, int maxr, LaunchArgs a);
-    LaunchArgs base_args() const;
-    template <typename F>
-    void for_each_surviving_quartet(double thr, F&& f) const;
+    TeamArgs team_args(const TeamPlanDev& plan, const TeamGroup& g, int* counter) const;
+    void run_team(const TeamPlanDev& plan, int mode, double thr, double* out);
     void record_stats(int launches);
 
     Basis basis_;
@@ -294,6 +319,9 @@ private:
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr, evk0_ = nullptr, evk1_ = nullptr;
 
     void build_jk_groups(bool mixed, GroupSet& gs);
+    void build_super();
+    void count_quartets(GroupSet& gs) const;
+    void build_fp32_groups(GroupSet& gs);
     void launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, const double* Dk2, double* J, double* Kx,
                    double* Kx2, int* counters = nullptr, bool mixed_plan = false, double dthr = 0.0);
     const GroupSet& plan(bool mixed_plan) const { return mixed_plan && mixed() ? gs_mixed_ : gs_fp64_; }
@@ -320,13 +348,23 @@ private:
     bool packed_ = false;              // built by the packed (several-molecule) constructor
     hfx_launch_shape shape_{256, 4096, 8, kDefaultLaneMinNpp, {0, 0, 0, 0}};
 
+    // super pairs (hfx_team.hpp): host image without the pools, device tables
+    SuperData sup_;
+    std::vector<double> qsup_;      // per super pair: largest bound of its members
+    DevBuf<SuperPair> d_super_;
+    DevBuf<double> d_shdr_, d_scoef_, d_smq_;
+    DevBuf<int> d_stab_, d_stypes_;
+    DevBuf<short> d_scode_;
+    DevBuf<unsigned> d_sridx_;
+    std::shared_ptr<DevBuf<double>> team_boys_;
+    DevBuf<double> d_tdsh_;         // per super pair max |D| (density screening)
+
     std::vector<HostPair> hpairs_;
     GroupSet gs_fp64_, gs_mixed_;
     DevBuf<int> d_counters_;
     DevBuf<double> d_dsh_;
     DevBuf<float> d_d32_;           // float copies of the build's densities (FP32 groups)
     std::vector<DPair> dpairs_host_;
-    DevBuf<double> d_rec64_;
     DevBuf<float> d_rec32_;
     DevBuf<float> d_boys32_;
     DevBuf<PairClassTab> d_pct_;
@@ -335,24 +373,12 @@ private:
     std::vector<cudaStream_t> aux_;
     std::vector<cudaEvent_t> aux_ev_;
     cudaEvent_t fork_ev_ = nullptr;
-    double flops32_ = 0.0, quartets32_ = 0.0;
     std::vector<double> qsh_;     // per pair
     std::vector<double> qbf_;     // per BF pair
     DevBuf<DPair> d_pairs_;
-    DevBuf<PairGeo> d_ppgeo_;
-    DevBuf<double> d_epool_;
-    DevBuf<double> d_boys_;     // [kBoysN][kBoysM] (k_quartet_eri)
-    DevBuf<double> d_boys64_;   // per-L rows (FP64 Fock and Schwarz kernels)
     DevBuf<double> d_qbf_;
     DevBuf<float> d_qbf32_;         // float copy of d_qbf_ (the FP32 kernels' screen)
-    DevBuf<unsigned long long> d_qsh_;
-    DevBuf<Task> d_tasks_;
-    int ntasks_ = 0;
-    int nquartets_ = 0;
-    int maxacc_ = 0, maxw_ = 0, maxr_ = 0;
-    DevBuf<int> d_counter_;
     DevBuf<double> d_D_, d_D2_, d_Dj_, d_J_, d_K_, d_K2_, d_out1_, d_out2_, d_out3_;
-    double prim_quartets_ = 0.0, flops_ = 0.0;
 };
 
 }  // namespace hfx

@@ -9,15 +9,16 @@
 // SCF cycle on its quartets are part of the session's launches.
 //
 // Layout.  The members' device tables stay where their jobs put them.  The
-// session builds a combined pair table whose records address every member's
-// arrays as anchor + offset (the offsets are taken in the device's single
-// address space; anchor64_ / anchor32_ are small session allocations), with
+// session builds combined pair tables: the FP32 one's records address every
+// member's arrays as anchor + offset (the offsets are taken in the device's
+// single address space; anchor32_ is a small session allocation), the super
+// pairs of the FP64 launches hold their arrays' addresses; both with
 // the member's matrices at its own offset of the session's packed density /
 // accumulator / output buffers and its pair indices shifted to its block of
 // the combined table.  The members' launch-group task lists are concatenated
-// per class (small classes by bra/ket class and precision, the warp kernel by
-// precision and shared-memory tier) and their pair indices shifted by a
-// device pass.  The layout is rebuilt whenever a member joins or leaves.
+// per launch (FP64: the team kernel by angular momentum, team size and
+// shared-memory tier; FP32: small classes by bra/ket class, the warp kernel by
+// shared-memory tier) and their pair indices shifted by a device pass.  The layout is rebuilt whenever a member joins or leaves.
 //
 // Cycle.  A member that needs a build waits until every live member has
 // asked; the last one runs the session's builds -- one per distinct
@@ -58,9 +59,10 @@ FockSession::FockSession(int device, int nspin, double screening_threshold)
     cuda_check(cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming), "event");
     cuda_check(cudaEventCreate(&ev0_), "event");
     cuda_check(cudaEventCreate(&ev1_), "event");
-    anchor64_.alloc(32);
     anchor32_.alloc(64);
-    boys64_.upload(boys_table64_host(), stream_);
+    team_boys_ = team_boys_device(device_, stream_);
+    scode_.upload(team_codes(), stream_);
+    sridx_.upload(team_ridx().words, stream_);
     boys32_.upload(boys_table32_host(), stream_);
     const ClassTables& ct = class_tables();
     pct_.upload(ct.tab, stream_);
@@ -156,7 +158,9 @@ void FockSession::relayout()
         if (slots_[s].live) live_.push_back((int)s);
     nmat_ = 0;
     npairs_ = 0;
-    std::vector<DPair> h64, h32;
+    nsuper_ = 0;
+    std::vector<DPair> h32;
+    std::vector<SuperPair> hs;
     std::vector<int> fk;
     std::vector<long long> fm;
     lane_min_npp_ = -1;
@@ -166,27 +170,30 @@ void FockSession::relayout()
         m.frag = (int)f;
         m.moff = nmat_;
         m.pair_off = npairs_;
+        m.super_off = nsuper_;
         const int K = j.K();
         nmat_ += (long long)K * K;
-        const long long d64 = elem_offset(j.d_rec64_.p, anchor64_.p, sizeof(double));
         const long long d32 = elem_offset(j.d_rec32_.p, anchor32_.p, sizeof(float));
-        const long long dq = elem_offset(j.d_qbf_.p, anchor64_.p, sizeof(double));
         const long long dq32 = elem_offset(j.d_qbf32_.p, anchor32_.p, sizeof(float));
         for (const DPair& src : j.dpairs_host_) {
             DPair x = src;
             x.moff = m.moff;
-            x.qoff = dq + src.qoff;
             x.pbase = m.pair_off + src.pbase;
             x.id = m.pair_off + src.id;
             x.frag = (int)f;
             x.kdim = K;
-            DPair a = x, b = x;
-            a.rec_off = d64 + src.rec_off;
-            b.rec_off = d32 + src.rec_off;
-            b.qoff = dq32 + src.qoff;   // the FP32 kernels screen with the float table
-            h64.push_back(a);
-            h32.push_back(b);
+            x.rec_off = d32 + src.rec_off;
+            x.qoff = dq32 + src.qoff;   // the FP32 kernels screen with the float table
+            h32.push_back(x);
         }
+        for (SuperPair x : j.sup_.pairs) {
+            x.moff = m.moff;
+            x.frag = (int)f;
+            x.id += m.super_off;
+            x.pbase += m.super_off;
+            hs.push_back(x);
+        }
+        nsuper_ += (int)j.sup_.pairs.size();
         npairs_ += (int)j.dpairs_host_.size();
         fk.push_back(K);
         fm.push_back(m.moff);
@@ -195,13 +202,15 @@ void FockSession::relayout()
     }
     if (lane_min_npp_ < 0) lane_min_npp_ = kDefaultLaneMinNpp;
     if (live_.empty()) {
-        plan64_.groups.clear();
-        plan_mixed_.groups.clear();
+        for (Combined* c : {&plan64_, &plan_mixed_}) {
+            c->groups.clear();
+            c->team.groups.clear();
+        }
         dirty_ = false;
         return;
     }
-    pairs64_.upload(h64, stream_);
     pairs32_.upload(h32, stream_);
+    super_.upload(hs, stream_);
     fk_.upload(fk, stream_);
     fmoff_.upload(fm, stream_);
     active_.alloc(live_.size());
@@ -211,19 +220,22 @@ void FockSession::relayout()
     for (int s = 0; s < nspin_ + 1; ++s) acc_[s].alloc(n);
     for (int s = 0; s < 2 * nspin_ - 1; ++s) out_[s].alloc(n);
     dsh_.alloc((size_t)std::max(1, npairs_));
+    tdsh_.alloc((size_t)std::max(1, nsuper_));
     d32_.alloc(3 * n);
     combine(false, plan64_);
     combine(true, plan_mixed_);
-    counters_.alloc(std::max<size_t>(1, std::max(plan64_.groups.size(), plan_mixed_.groups.size())));
+    counters_.alloc(std::max<size_t>(1, std::max(plan64_.launches(), plan_mixed_.launches())));
     cuda_check(cudaStreamSynchronize(stream_), "session layout");
     dirty_ = false;
 }
 
-// The members' launch groups of one plan, merged by class: small classes by
-// (bra class, ket class, precision), the warp kernel by (precision,
-// shared-memory tier); task lists concatenated, pair indices shifted.
+// The members' launch groups of one plan, merged by launch: the team kernel by
+// (angular momentum, team size, shared-memory tier), small classes by (bra
+// class, ket class), the FP32 warp kernel by shared-memory tier; task lists
+// concatenated, pair indices shifted.
 void FockSession::combine(bool mixed_plan, Combined& c)
 {
+    combine_team(mixed_plan, c);
     struct Part {
         int member;
         const GroupSet* gs;
@@ -249,7 +261,6 @@ void FockSession::combine(bool mixed_plan, Combined& c)
     c.groups.clear();
     c.tasks.alloc(std::max<size_t>(1, total));
     size_t off = 0;
-    const size_t elem[2] = {sizeof(double), sizeof(float)};
     for (auto& kv : parts) {
         LaunchGroup cg{};
         const LaunchGroup& g0 = *kv.second.front().g;
@@ -278,18 +289,78 @@ void FockSession::combine(bool mixed_plan, Combined& c)
             cg.slice = std::max(cg.slice, g.slice);
         }
         if (cg.kind == 1) {
-            const int f = cg.fp32 ? 1 : 0;
             cg.slice = (cg.slice + 1) & ~1;
             cg.lane_min_npp = lane_min_npp_;
             cg.warps_per_cta = (int)std::max<size_t>(
-                1, std::min<size_t>(8, (200 * 1024 - kWarpSmemHeader) / ((size_t)cg.slice * elem[f])));
-            const size_t sm = kWarpSmemHeader + elem[f] * (size_t)cg.slice * cg.warps_per_cta;
+                1, std::min<size_t>(8, (200 * 1024 - kWarpSmemHeader) / ((size_t)cg.slice * sizeof(float))));
+            const size_t sm = kWarpSmemHeader + sizeof(float) * (size_t)cg.slice * cg.warps_per_cta;
             const int ctas_per_sm = (int)std::max<size_t>(1, (228 * 1024) / (sm + 1024));
             const long long need = ((long long)cg.n + cg.warps_per_cta - 1) / cg.warps_per_cta;
             cg.grid = (int)std::min<long long>(need, (long long)nsm_ * ctas_per_sm);
         }
         c.groups.push_back(cg);
     }
+}
+
+void FockSession::combine_team(bool mixed_plan, Combined& c)
+{
+    struct Part {
+        int member, order_off;
+        const GroupSet* gs;
+        const TeamGroup* g;
+    };
+    std::map<std::tuple<int, int, int>, std::vector<Part>> parts;
+    size_t ntask = 0, norder = 0;
+    for (int slot : live_) {
+        const GroupSet& gs = slots_[slot].job->plan(mixed_plan);
+        for (const TeamGroup& g : gs.team.groups) {
+            int tier = 0;
+            while ((512 << tier) < g.slice) ++tier;
+            parts[{g.L, g.team, tier}].push_back(Part{slot, (int)norder, &gs, &g});
+            ntask += g.n;
+        }
+        norder += gs.team.order.n;
+    }
+    c.team.groups.clear();
+    c.team.tasks.alloc(std::max<size_t>(1, ntask));
+    c.team.order.alloc(std::max<size_t>(1, norder));
+    size_t off = 0;
+    for (int slot : live_) {
+        const GroupSet& gs = slots_[slot].job->plan(mixed_plan);
+        long long n = (long long)gs.team.order.n;
+        if (n == 0) continue;
+        int* o = c.team.order.p + off;
+        int delta = slots_[slot].super_off;
+        cuda_check(cudaMemcpyAsync(o, gs.team.order.p, n * sizeof(int), cudaMemcpyDeviceToDevice, stream_), "session order");
+        KernelSpec ks = team_rebase_order_spec(n);
+        void* prm[] = {&o, &n, &delta};
+        cuda_check(cudaLaunchKernel(ks.func, ks.grid, ks.block, prm, 0, stream_), "session rebase");
+        off += (size_t)n;
+    }
+    off = 0;
+    for (auto& kv : parts) {
+        TeamGroup cg = *kv.second.front().g;
+        cg.off = off;
+        cg.n = 0;
+        cg.cost = 0.0;
+        for (const Part& p : kv.second) {
+            long long n = (long long)p.g->n;
+            TeamTask* t = c.team.tasks.p + off;
+            int dpair = slots_[p.member].super_off, dorder = p.order_off;
+            cuda_check(cudaMemcpyAsync(t, p.gs->team.tasks.p + p.g->off, n * sizeof(TeamTask), cudaMemcpyDeviceToDevice,
+                                       stream_),
+                       "session tasks");
+            KernelSpec ks = team_rebase_spec(n);
+            void* prm[] = {&t, &n, &dpair, &dorder};
+            cuda_check(cudaLaunchKernel(ks.func, ks.grid, ks.block, prm, 0, stream_), "session rebase");
+            off += (size_t)n;
+            cg.n += p.g->n;
+            cg.cost += p.g->cost;
+            cg.slice = std::max(cg.slice, p.g->slice);
+        }
+        c.team.groups.push_back(cg);
+    }
+    std::stable_sort(c.team.groups.begin(), c.team.groups.end(), [](const TeamGroup& a, const TeamGroup& b) { return a.cost > b.cost; });
 }
 
 // One build of the live members switched on in active_ (J/K into acc_,
@@ -317,18 +388,25 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
     double* Kx = acc_[1].p;
     double* Kx2 = nk == 2 ? acc_[2].p : nullptr;
     const double* Dsh = nullptr;
-    if (dthr > 0.0 && npairs_ > 0) {
-        const DPair* pr = pairs64_.p;
+    if (dthr > 0.0 && !c.groups.empty()) {
+        const DPair* pr = pairs32_.p;
         int np = npairs_;
         double* out = dsh_.p;
         void* prm[] = {&pr, &np, &Dk, &Dk2, &out};
         sk.kernel(0, density_blocks_spec(np), prm);
         Dsh = dsh_.p;
     }
+    const double* Tsh = nullptr;
+    if (dthr > 0.0 && !c.team.groups.empty()) {
+        const SuperPair* pr = super_.p;
+        int np = nsuper_;
+        double* out = tdsh_.p;
+        void* prm[] = {&pr, &np, &Dk, &Dk2, &out};
+        sk.kernel(0, team_density_spec(np), prm);
+        Tsh = tdsh_.p;
+    }
     const float *Dj32 = nullptr, *Dk32 = nullptr, *Dk232 = nullptr;
-    bool any32 = false;
-    for (const auto& g : c.groups) any32 = any32 || g.fp32;
-    if (any32) {
+    if (!c.groups.empty()) {
         long long nn = (long long)n;
         const double* src[3] = {Dj, Dk, Dk2};
         const float* dst[3] = {nullptr, nullptr, nullptr};
@@ -353,10 +431,40 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
     }
     const unsigned char* active = active_.p;
     int* ctr = counters_.p;
-    sk.zero(0, ctr, sizeof(int) * std::max<size_t>(1, c.groups.size()));
+    sk.zero(0, ctr, sizeof(int) * std::max<size_t>(1, c.launches()));
     sk.fork();
     const Task* tasks = c.tasks.p;
     const int naux = (int)aux_.size();
+    for (size_t gi = 0; gi < c.team.groups.size(); ++gi) {
+        const TeamGroup& g = c.team.groups[gi];
+        KernelSpec ks;
+        cuda_check(team_spec(g, nsm_, &ks), "session team kernel");
+        TeamArgs a{};
+        a.pairs = super_.p;
+        a.order = c.team.order.p;
+        a.tasks = c.team.tasks.p + g.off;
+        a.ntasks = (int)g.n;
+        a.counter = ctr + c.groups.size() + gi;
+        a.kcode = scode_.p;
+        a.ridx = reinterpret_cast<const uint4*>(sridx_.p);
+        std::copy(team_ridx().at, team_ridx().at + 49, a.ridx_at);
+        a.boys = team_boys_->p;
+        team_thresholds(a, thr_, dthr);
+        a.mode = kTeamFock;
+        a.mixed = mixed_plan;
+        a.Dj = Dj;
+        a.Dk = Dk;
+        a.Dk2 = Dk2;
+        a.J = J;
+        a.Kx = Kx;
+        a.Kx2 = Kx2;
+        a.Dsh = Tsh;
+        a.active = active;
+        a.nk = nk;
+        a.slice = g.slice;
+        void* prm[] = {&a};
+        sk.kernel((int)(gi % (naux + 1)), ks, prm);
+    }
     int next_aux = 0;
     for (size_t gi = 0; gi < c.groups.size(); ++gi) {
         const LaunchGroup& g = c.groups[gi];
@@ -364,34 +472,18 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
         if (g.kind == 0) {
             const int lane = 1 + next_aux;
             next_aux = (next_aux + 1) % naux;
-            if (g.fp32) {
-                SmallArgs<float> a{pairs32_.p, anchor32_.p, tasks + g.off, (int)g.n, boys32_.p, thr_, nullptr,
-                                   0, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p};
-                cuda_check(small_spec_f32(g.pcb, g.pck, nk, (int)g.n, &ks), "session small-class kernel");
-                void* prm[] = {&a};
-                sk.kernel(lane, ks, prm);
-            } else {
-                SmallArgs<double> a{pairs64_.p, anchor64_.p, tasks + g.off, (int)g.n, boys64_.p, thr_, anchor64_.p,
-                                    0, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr, active, nullptr, nullptr, nullptr};
-                cuda_check(small_spec_f64(g.pcb, g.pck, nk, (int)g.n, &ks), "session small-class kernel");
-                void* prm[] = {&a};
-                sk.kernel(lane, ks, prm);
-            }
+            SmallArgs<float> a{pairs32_.p, anchor32_.p, tasks + g.off, (int)g.n, boys32_.p, thr_, nullptr,
+                               0, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p};
+            cuda_check(small_spec_f32(g.pcb, g.pck, nk, (int)g.n, &ks), "session small-class kernel");
+            void* prm[] = {&a};
+            sk.kernel(lane, ks, prm);
         } else {
-            cuda_check(warp_spec(g.fp32, nk, g.grid, g.warps_per_cta, g.slice, &ks), "session warp kernel");
-            if (g.fp32) {
-                WarpArgs<float> a{pairs32_.p, anchor32_.p, pct_.p, abs_.p, kh_.p, kl_.p, tasks + g.off, (int)g.n,
-                                  ctr + gi, boys32_.p, thr_, nullptr, 0, Dj, Dk, Dk2, J, Kx, Kx2, g.slice,
-                                  g.lane_min_npp, Dsh, dthr, nullptr, nullptr, active, Dj32, Dk32, Dk232, anchor32_.p};
-                void* prm[] = {&a};
-                sk.kernel(0, ks, prm);
-            } else {
-                WarpArgs<double> a{pairs64_.p, anchor64_.p, pct_.p, abs_.p, kh_.p, kl_.p, tasks + g.off, (int)g.n,
-                                   ctr + gi, boys64_.p, thr_, anchor64_.p, 0, Dj, Dk, Dk2, J, Kx, Kx2, g.slice,
-                                   g.lane_min_npp, Dsh, dthr, nullptr, nullptr, active, nullptr, nullptr, nullptr};
-                void* prm[] = {&a};
-                sk.kernel(0, ks, prm);
-            }
+            cuda_check(warp_spec(true, nk, g.grid, g.warps_per_cta, g.slice, &ks), "session warp kernel");
+            WarpArgs<float> a{pairs32_.p, anchor32_.p, pct_.p, abs_.p, kh_.p, kl_.p, tasks + g.off, (int)g.n,
+                              ctr + gi, boys32_.p, thr_, nullptr, 0, Dj, Dk, Dk2, J, Kx, Kx2, g.slice,
+                              g.lane_min_npp, Dsh, dthr, nullptr, nullptr, active, Dj32, Dk32, Dk232, anchor32_.p};
+            void* prm[] = {&a};
+            sk.kernel(0, ks, prm);
         }
     }
     sk.join();

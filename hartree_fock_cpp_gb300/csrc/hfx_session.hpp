@@ -62,6 +62,7 @@ private:
         bool live = false;
         long long moff = 0;   // first element of its matrices in the session buffers
         int pair_off = 0;     // first combined pair
+        int super_off = 0;    // first combined super pair
         int frag = 0;         // index in the live list (active flags, finish tables)
     };
     struct Req {
@@ -74,10 +75,13 @@ private:
     struct Combined {
         std::vector<LaunchGroup> groups;
         DevBuf<Task> tasks;
+        TeamPlanDev team;                 // FP64: team kernel over the members' super pairs
+        size_t launches() const { return groups.size() + team.groups.size(); }
     };
 
     void relayout();                      // combined tables of the live members (mu_ held)
     void combine(bool mixed_plan, Combined& c);
+    void combine_team(bool mixed_plan, Combined& c);
     void run_locked();
     void launch(int nk, bool mixed_plan, double dthr);
 
@@ -92,25 +96,28 @@ private:
     std::vector<int> live_;               // live slots in layout order
     bool dirty_ = true;
     long long nmat_ = 0;
-    int npairs_ = 0;
+    int npairs_ = 0, nsuper_ = 0;
     int lane_min_npp_ = kDefaultLaneMinNpp;
 
-    // anchors of the combined pair table's offsets: each member's record and
-    // Schwarz arrays are addressed as anchor + offset (one address space)
-    DevBuf<double> anchor64_;
+    // anchor of the combined pair table's offsets (FP32 launches): each
+    // member's record and Schwarz arrays are addressed as anchor + offset (one
+    // address space); the super pairs hold their arrays' addresses
     DevBuf<float> anchor32_;
-    DevBuf<DPair> pairs64_, pairs32_;
+    DevBuf<DPair> pairs32_;
+    DevBuf<SuperPair> super_;
     DevBuf<int> fk_;
     DevBuf<long long> fmoff_;
     DevBuf<unsigned char> active_;
     Combined plan64_, plan_mixed_;
     DevBuf<int> counters_;
-    DevBuf<double> boys64_;
+    std::shared_ptr<DevBuf<double>> team_boys_;
+    DevBuf<short> scode_;
+    DevBuf<unsigned> sridx_;
     DevBuf<float> boys32_;
     DevBuf<PairClassTab> pct_;
     DevBuf<int> abs_;
     DevBuf<short> kh_, kl_;
-    DevBuf<double> in_[2], dj_, acc_[3], out_[3], dsh_;
+    DevBuf<double> in_[2], dj_, acc_[3], out_[3], dsh_, tdsh_;
     DevBuf<float> d32_;
 
     mutable std::mutex mu_;
