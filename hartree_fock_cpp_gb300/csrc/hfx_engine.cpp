@@ -204,7 +204,7 @@ void Job::init(const hfx_options& opt)
     cuda_check(cudaEventCreate(&evk0_), "event");
     cuda_check(cudaEventCreate(&evk1_), "event");
 
-    for (int s = 0; s < 3; ++s) {
+    for (int s = 0; s < kAuxLanes; ++s) {
         cudaStream_t st;
         cuda_check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
         aux_.push_back(st);
@@ -1310,7 +1310,8 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
     sk.zero(0, ctr, sizeof(int) * std::max<size_t>(1, gs.launches()));
     sk.fork();
     const int naux = (int)aux_.size();
-    // FP64: the team kernel's launches over all lanes, the largest first
+    // FP64: the team kernel's launches, the largest first
+    const int n64 = groups.empty() ? naux + 1 : kFp64Lanes;
     for (size_t gi = 0; gi < gs.team.groups.size(); ++gi) {
         const TeamGroup& g = gs.team.groups[gi];
         KernelSpec ks;
@@ -1329,17 +1330,17 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
         a.active = active;
         a.nk = nk;
         void* prm[] = {&a};
-        sk.kernel((int)(gi % (naux + 1)), ks, prm);
+        sk.kernel((int)(gi % n64), ks, prm);
     }
-    // FP32: warp groups on the main lane, small classes spread over the others
+    // FP32: on the lanes left, warp groups on the last
     int next_aux = 0;
     for (size_t gi = 0; gi < groups.size(); ++gi) {
         const LaunchGroup& g = groups[gi];
         if (g.n == 0) continue;
         KernelSpec ks;
         if (g.kind == 0) {
-            const int lane = 1 + next_aux;
-            next_aux = (next_aux + 1) % naux;
+            const int lane = naux - next_aux;
+            next_aux = (next_aux + 1) % (naux + 1 - kFp64Lanes);
             SmallArgs<float> a{d_pairs_.p, d_rec32_.p, tasks + g.off, (int)g.n, d_boys32_.p, opt_.screening_threshold,
                                d_qbf_.p, K, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, d_qbf32_.p};
             cuda_check(small_spec_f32(g.pcb, g.pck, nk, (int)g.n, &ks), "small-class kernel");
@@ -1352,7 +1353,7 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
                               g.slice, g.lane_min_npp, Dsh, dthr, nullptr, nullptr, active, Dj32, Dk32, Dk232,
                               d_qbf32_.p};
             void* prm[] = {&a};
-            sk.kernel(0, ks, prm);
+            sk.kernel(naux, ks, prm);
         }
     }
     sk.join();

@@ -175,6 +175,13 @@ struct GroupSet {
     double flops64 = 0.0, flops32 = 0.0, prims = 0.0, quartets32 = 0.0;
 };
 
+// Streams of a build beside the main one, and how many of all of them the FP64
+// launches of a mixed build share (an FP64 build uses all): its 30-40 launches
+// end in tails of a few CTAs that only other launches can fill. 3 + all
+// against 11 + 8, ms: water/cc-pVTZ 1.14 / 0.92, NaCl/cc-pVTZ 3.73 / 3.4,
+// benzene/cc-pVDZ 8.10 / 7.84, n-decane/6-31G* mixed 3.20 / 3.02.
+constexpr int kAuxLanes = 11, kFp64Lanes = 8;
+
 // Destination of a Fock build's device work.  Lane 0 is the job's main
 // stream, lanes 1..n its auxiliary streams; fork() makes every auxiliary lane
 // wait for what lane 0 has issued so far, join() makes lane 0 wait for all of

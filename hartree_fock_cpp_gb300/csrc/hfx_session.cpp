@@ -48,7 +48,7 @@ FockSession::FockSession(int device, int nspin, double screening_threshold)
     cuda_check(cudaSetDevice(device_), "cudaSetDevice");
     cuda_check(cudaDeviceGetAttribute(&nsm_, cudaDevAttrMultiProcessorCount, device_), "SM count");
     cuda_check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
-    for (int s = 0; s < 3; ++s) {
+    for (int s = 0; s < kAuxLanes; ++s) {
         cudaStream_t st;
         cuda_check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
         aux_.push_back(st);
@@ -463,15 +463,15 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
         a.nk = nk;
         a.slice = g.slice;
         void* prm[] = {&a};
-        sk.kernel((int)(gi % (naux + 1)), ks, prm);
+        sk.kernel((int)(gi % (c.groups.empty() ? naux + 1 : kFp64Lanes)), ks, prm);
     }
     int next_aux = 0;
     for (size_t gi = 0; gi < c.groups.size(); ++gi) {
         const LaunchGroup& g = c.groups[gi];
         KernelSpec ks;
         if (g.kind == 0) {
-            const int lane = 1 + next_aux;
-            next_aux = (next_aux + 1) % naux;
+            const int lane = naux - next_aux;
+            next_aux = (next_aux + 1) % (naux + 1 - kFp64Lanes);
             SmallArgs<float> a{pairs32_.p, anchor32_.p, tasks + g.off, (int)g.n, boys32_.p, thr_, nullptr,
                                0, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p};
             cuda_check(small_spec_f32(g.pcb, g.pck, nk, (int)g.n, &ks), "session small-class kernel");
@@ -483,7 +483,7 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
                               ctr + gi, boys32_.p, thr_, nullptr, 0, Dj, Dk, Dk2, J, Kx, Kx2, g.slice,
                               g.lane_min_npp, Dsh, dthr, nullptr, nullptr, active, Dj32, Dk32, Dk232, anchor32_.p};
             void* prm[] = {&a};
-            sk.kernel(0, ks, prm);
+            sk.kernel(naux, ks, prm);
         }
     }
     sk.join();

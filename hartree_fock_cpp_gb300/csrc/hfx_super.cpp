@@ -318,10 +318,17 @@ SuperData build_super_data(const Basis& b, const Fragments& fr)
                 }
             }
             Out& o = outs[p];
-            std::vector<int> place(nq, -1);
+            // primitive pairs of more members first: a short member's list
+            // then lies in the first batches of a long ket loop
+            std::vector<int> place(nq, -1), seq;
+            for (int q = 0; q < nq; ++q)
+                if (keep[q]) seq.push_back(q);
+            std::vector<int> uses(nq, 0);
+            for (int m = 0; m < nm; ++m)
+                for (int q = 0; q < nq; ++q) uses[q] += has[m][q] != 0;
+            std::stable_sort(seq.begin(), seq.end(), [&](int x, int y) { return uses[x] > uses[y]; });
             int n = 0;
-            for (int q = 0; q < nq; ++q) {
-                if (!keep[q]) continue;
+            for (int q : seq) {
                 place[q] = n++;
                 o.hdr.insert(o.hdr.end(), geo.begin() + 4 * (size_t)q, geo.begin() + 4 * (size_t)q + 4);
                 o.hdr.push_back(5.914967172795613 / geo[4 * (size_t)q]);   // sqrt(2 pi^{5/2}) / p
@@ -353,7 +360,7 @@ SuperData build_super_data(const Basis& b, const Fragments& fr)
                 o.tab[m] = (int)o.tab.size();
                 o.tab[2 * nm + m] = (int)o.coef.size();
                 int n = 0;
-                for (int q = 0; q < nq; ++q) {
+                for (int q : seq) {
                     if (!has[m][q]) continue;
                     n += has[m][q];
                     o.tab.push_back(place[q]);
@@ -429,62 +436,73 @@ struct StepCosts {
 // `cap` doubles where the smallest batch allows it.  One bra pair: the rows
 // per batch with the fewest instructions per row; the threads of a round take
 // items in decreasing work, so a round costs as much as its first one.
-Geometry geometry(int L1, int L2, int nab, int ncd, int rows, int npk, int nb, int maxrows, int lanes, int cap,
+Geometry geometry(int L1, int L2, const SuperPair& bra, const SuperPair& ket, int rows, int npk, int nb, int maxrows, int lanes, int cap,
                   const StepCosts& c)
 {
-    Geometry g;
-    // rows of a bra pair shared by several threads where its block alone
-    // leaves threads idle
-    auto parts = [&](int slots, int r) {
-        int p = 1;
-        while (2 * p <= std::min(r, 16) && 2 * p * slots * nab * ncd <= lanes) p *= 2;
-        return p;
+    const int nab = bra.nA * bra.nB, ncd = ket.nA * ket.nB, nmk = ket.nmem;
+    auto slice_of = [&](int nr, int nkb, int nw, int slots, int parts) {
+        return team_slice(L1, L2, bra.nA, bra.nB, ket.nA, ket.nB, nr, nkb, nw, slots, nb, parts, nmk);
     };
+    Geometry g;
+    auto group = [&](int n) { return n >= team_cd_group(ncd) * lanes ? team_cd_group(ncd) : 1; };
     if (nb > 1) {
         // several bra pairs: every primitive quartet of the task in one R
-        // batch; rounds of as many bra pairs as the slice holds
+        // batch; rounds of as many bra pairs as the slice holds; the rows of
+        // a bra pair shared by several threads where its block alone leaves
+        // threads idle
+        auto parts = [&](int slots) {
+            int p = 1;
+            while (2 * p <= std::min(maxrows, 16) && p * slots * nab * ncd < 2 * lanes) p *= 2;
+            return p;
+        };
         g.nr = rows;
         g.nkb = npk;
         g.slots = 1;
         auto fits = [&](int s) {
-            return team_slice(L1, L2, nab, ncd, rows, npk, s * maxrows, s, nb, parts(s, maxrows)) <= cap;
+            return slice_of(rows, npk, s * maxrows, s, parts(s)) <= cap;
         };
         while (g.slots < nb && fits(g.slots + 1)) ++g.slots;
         const int rounds = (nb + g.slots - 1) / g.slots;
         g.slots = (nb + rounds - 1) / rounds;
         g.nw = g.slots * maxrows;
+        g.parts = parts(g.slots);
     } else {
-        g.slots = 1;
-        auto size = [&](int nr, int nkb) { return team_slice(L1, L2, nab, ncd, nr, nkb, nr, 1, 1, parts(1, nr)); };
-        int nblk = 1;
-        while (nblk < npk && size(1, (npk + nblk - 1) / nblk) > cap) ++nblk;
-        g.nkb = (npk + nblk - 1) / nblk;
         const int H1 = team_nherm(L1), J = H1 == 1 ? 1 : team_tuv_group(H1), ng = (H1 + J - 1) / J;
-        auto cost = [&](int r) {
-            double w = nblk * ((r * g.nkb + lanes - 1) / lanes * c.r + 30.0) + 60.0;
-            for (int x = 0; x < ncd * r * ng; x += lanes) w += (double)J * (*c.ket)[x / (r * ng)] * npk / c.nket;
-            const int n = nab * ncd * parts(1, r);
-            const int JC = ncd % 4 == 0 && n >= 4 * lanes ? 4 : ncd % 3 == 0 && n >= 3 * lanes ? 3 : 1;
-            const int per = ncd / JC * parts(1, r);
-            for (int x = 0; x < nab * per; x += lanes)
-                w += (double)JC * (*c.bra)[x / per] * r / c.nbra / parts(1, r);
-            return w * ((rows + r - 1) / r);
-        };
-        int best = 1;
-        double least = 0.0;
-        for (int r = 1; r <= std::min(rows, 96); ++r) {
-            if (r > 1 && size(r, g.nkb) > cap) break;
-            const double w = cost(r);
-            if (r == 1 || w < 0.995 * least) {
-                least = w;
-                best = r;
+        double least = -1.0;
+        g.slots = 1;
+        for (int nblk = 1; nblk <= npk; nblk = nblk < 4 ? nblk + 1 : nblk * 3 / 2) {
+            const int nkb = (npk + nblk - 1) / nblk;
+            const bool last = nblk * 3 / 2 > npk;
+            for (int r = 1; r <= std::min(rows, 64); ++r) {
+                bool fits = false;
+                for (int p = 1; p <= std::min(r, 8); p *= 2) {
+                    const int size = slice_of(r, nkb, r, 1, p);
+                    if (size > cap && !(last && r == 1 && least < 0.0)) break;
+                    fits = true;
+                    double w = nblk * ((double)((r * nkb + lanes - 1) / lanes) * c.r + 20.0);
+                    for (int x = 0; x < ncd * r * ng; x += lanes)
+                        w += (double)J * (*c.ket)[x / (r * ng)] * npk / c.nket + 2.0 * nblk;
+                    const int JC = group(nab * ncd * p), per = ncd / JC * p;
+                    for (int x = 0; x < nab * per; x += lanes)
+                        w += (double)JC * (*c.bra)[x / per] / c.nbra * ((r + p - 1) / p) + 2.0;
+                    w = w * ((rows + r - 1) / r) + (double)(p - 1) * ((nab * ncd + lanes - 1) / lanes);
+                    if (least < 0.0 || w < 0.995 * least) {
+                        least = w;
+                        g.nr = g.nw = r;
+                        g.nkb = nkb;
+                        g.parts = p;
+                    }
+                }
+                if (!fits) break;
             }
+            if (nblk > 40 && least > 0.0) break;
         }
-        g.nr = best;
-        g.nw = best;
+        if (least < 0.0) {
+            g.nr = g.nw = g.parts = 1;
+            g.nkb = 1;
+        }
     }
-    g.parts = parts(g.slots, nb > 1 ? maxrows : g.nr);
-    g.slice = team_slice(L1, L2, nab, ncd, g.nr, g.nkb, g.nw, g.slots, nb, g.parts);
+    g.slice = slice_of(g.nr, g.nkb, g.nw, g.slots, g.parts);
     return g;
 }
 
@@ -539,19 +557,12 @@ TeamPlanHost build_team_plan(const SuperData& sd, const std::vector<double>& q, 
 {
     TeamPlanHost plan;
     const int np = (int)sd.pairs.size();
-    // Classes ranked by coefficients per Hermite function: the ket transform
-    // costs (ket coefficients) x (bra Hermite functions) per primitive
-    // quartet, so the ket is the side with the smaller ratio.
-    std::vector<int> rank(sd.ncls), by(sd.ncls), cL(sd.ncls, 0), cab(sd.ncls, 0);
+    std::vector<int> cL(sd.ncls, 0), cab(sd.ncls, 0), sample(sd.ncls, 0);
     for (int p = 0; p < np; ++p) {
         cL[sd.cls[p]] = sd.pairs[p].L;
         cab[sd.cls[p]] = sd.pairs[p].nA * sd.pairs[p].nB;
+        sample[sd.cls[p]] = p;
     }
-    std::iota(by.begin(), by.end(), 0);
-    std::stable_sort(by.begin(), by.end(), [&](int x, int y) {
-        return sd.cls_nnz[x] / team_nherm(cL[x]) < sd.cls_nnz[y] / team_nherm(cL[y]);
-    });
-    for (int i = 0; i < sd.ncls; ++i) rank[by[i]] = i;
     // per (molecule, class): its pairs by decreasing bound
     const int F = (int)sd.pbase.size() - 1;
     std::vector<int> start((size_t)F * sd.ncls + 1, 0);
@@ -590,23 +601,32 @@ TeamPlanHost build_team_plan(const SuperData& sd, const std::vector<double>& q, 
         double total = 0.0;
     };
     std::vector<Unit> units;
-    for (int fr = 0; fr < F; ++fr)
-        for (int i = 0; i < sd.ncls; ++i)
-            for (int j = 0; j <= i; ++j) {
-                const size_t b = (size_t)fr * sd.ncls + by[i], k = (size_t)fr * sd.ncls + by[j];
-                if (start[b + 1] > start[b] && start[k + 1] > start[k]) {
-                    units.emplace_back();
-                    units.back().fr = fr;
-                    units.back().cb = by[i];
-                    units.back().ck = by[j];
-                }
-            }
     // cost of a primitive quartet, a bra primitive pair and a quartet
     auto costs = [&](const Unit& u, double* prim, double* row, double* quartet) {
         *prim = team_r_cost(cL[u.cb] + cL[u.ck]) + sd.cls_nnz[u.ck] * team_nherm(cL[u.cb]);
         *row = sd.cls_nnz[u.cb] * cab[u.ck];
         *quartet = 8.0 * cab[u.cb] * cab[u.ck];
     };
+    for (int fr = 0; fr < F; ++fr)
+        for (int i = 0; i < sd.ncls; ++i)
+            for (int j = 0; j <= i; ++j) {
+                const size_t b = (size_t)fr * sd.ncls + i, k = (size_t)fr * sd.ncls + j;
+                if (start[b + 1] == start[b] || start[k + 1] == start[k]) continue;
+                // the ket transform costs (ket coefficients) x (bra Hermite
+                // functions) per primitive quartet, the bra transform (bra
+                // coefficients) x (ket component pairs) per bra primitive
+                // pair: the sides that cost less for the longest pairs
+                Unit u, v;
+                u.fr = v.fr = fr;
+                u.cb = v.ck = i;
+                u.ck = v.cb = j;
+                auto whole = [&](const Unit& x) {
+                    double cp, cr, cq;
+                    costs(x, &cp, &cr, &cq);
+                    return (double)sd.cls_npp[x.cb] * (sd.cls_npp[x.ck] * cp + cr);
+                };
+                units.push_back(whole(v) < whole(u) ? v : u);
+            }
     host_parallel_for((int)units.size(), [&](int i) {
         Unit& u = units[i];
         double cp, cr, cq;
@@ -628,6 +648,7 @@ TeamPlanHost build_team_plan(const SuperData& sd, const std::vector<double>& q, 
         double cp, cr, cq;
         costs(u, &cp, &cr, &cq);
         const int L1 = cL[u.cb], L2 = cL[u.ck], nab = cab[u.cb], ncd = cab[u.ck], nout = nab * ncd;
+        const SuperPair &bra = sd.pairs[sample[u.cb]], &ket = sd.pairs[sample[u.ck]];
         const int HS = team_nherm(L1 + L2) | 1, H1 = team_nherm(L1);
         const long long maxR = L1 + L2 > kTeamMaxRegL ? 3072 : 6144;
         // primitive quartets of a task of several bra pairs, and of the bra
@@ -643,9 +664,9 @@ TeamPlanHost build_team_plan(const SuperData& sd, const std::vector<double>& q, 
             auto it = known.find(key);
             if (it == known.end()) {
                 const int cap32 = std::max(2800, 34 * HS + ncd * H1 + nout + 200);
-                std::pair<Geometry, int> v(geometry(L1, L2, nab, ncd, rows, npk, nb, maxrows, 32, cap32, sc), 32);
+                std::pair<Geometry, int> v(geometry(L1, L2, bra, ket, rows, npk, nb, maxrows, 32, cap32, sc), 32);
                 if (v.first.slice > 4096 || few || large)
-                    v = {geometry(L1, L2, nab, ncd, rows, npk, nb, maxrows, 128, 9000, sc), 128};
+                    v = {geometry(L1, L2, bra, ket, rows, npk, nb, maxrows, 128, 9000, sc), 128};
                 it = known.emplace(key, v).first;
             }
             *team = it->second.second;
@@ -750,11 +771,11 @@ TeamPlanHost build_team_diagonal(const SuperData& sd, int nsm)
         const int c = sd.cls[p];
         const StepCosts sc{team_r_cost(2 * d.L), &sd.cls_work[c], &sd.cls_work[c], sd.cls_npp[c], sd.cls_npp[c]};
         int team = 32;
-        Geometry g = geometry(d.L, d.L, nab, nab, per, d.npp, 1, per, 32,
+        Geometry g = geometry(d.L, d.L, d, d, per, d.npp, 1, per, 32,
                               std::max(2800, 34 * HS + nab * team_nherm(d.L) + nab * nab + 200), sc);
         if (g.slice > 4096 || one[p] > target) {
             team = 128;
-            g = geometry(d.L, d.L, nab, nab, per, d.npp, 1, per, 128, 9000, sc);
+            g = geometry(d.L, d.L, d, d, per, d.npp, 1, per, 128, 9000, sc);
         }
         per = std::min(d.npp, (per + g.nr - 1) / g.nr * g.nr);
         TeamTask t{};

@@ -18,10 +18,11 @@
 //   4. digestion: each J / K element that the quartet touches is summed over
 //      the block and added with one atomic
 // Fock builds against the FP64 shell-quartet kernels before it (ms): benzene /
-// cc-pVDZ 17.9 -> 8.0, n-decane / 6-31G* 16.7 -> 14.1, NaCl / cc-pVTZ 19.8 ->
-// 4.4, water / cc-pVTZ UHF 8.1 -> 1.14 (there one warp evaluated a whole
-// contracted f quartet); 120 M FP64 warp instructions for benzene, 20 of 32
-// lanes active.  Schwarz pass of NaCl / cc-pVTZ 35 -> 0.9 ms.
+// cc-pVDZ 17.9 -> 7.7, n-decane / 6-31G* 16.7 -> 14.0, NaCl / cc-pVTZ 19.7 ->
+// 3.3, water / cc-pVTZ UHF 8.1 -> 0.89 (there one warp evaluated a whole
+// contracted f quartet); 114 M FP64 warp instructions for benzene, 21 of 32
+// lanes active (R 34 M at 23 lanes, step 2 47 M at 22, step 3 21 M at 18, the
+// digestion 12 M at 15).  Schwarz pass of NaCl / cc-pVTZ 35 -> 0.9 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,8 +37,8 @@ namespace hfx {
 namespace {
 
 constexpr int kNb = 456;          // recursion neighbours (ints; general form only)
-constexpr int kTeamHeaderBytes = 4 * kNb + 64;
-static_assert(kTeamHeaderBytes % 16 == 0, "team slices are 16-byte aligned");
+// shared-memory header: the work-queue box, in the general form the neighbours
+__host__ __device__ constexpr int team_header(int LC) { return LC < 0 ? 4 * kNb + 64 : 16; }
 
 template <int TEAM>
 __device__ __forceinline__ void team_sync()
@@ -230,14 +231,13 @@ __device__ __forceinline__ int first_at_least(const int* __restrict__ list, int 
 
 // LC: compiled total angular momentum, or -1 for any L.
 template <int LC, int TEAM>
-__global__ void __launch_bounds__(128, 4) k_team(TeamArgs a)
+__global__ void __launch_bounds__(TEAM, TEAM == 32 ? 16 : 4) k_team(TeamArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    int* nbt = reinterpret_cast<int*>(smem);
-    int* box = reinterpret_cast<int*>(smem + 4 * kNb);
-    const int tid = TEAM == 32 ? threadIdx.x & 31 : threadIdx.x;
-    double* sl = reinterpret_cast<double*>(smem + kTeamHeaderBytes) +
-                 (TEAM == 32 ? (size_t)(threadIdx.x >> 5) * a.slice : 0);
+    int* box = reinterpret_cast<int*>(smem);
+    int* nbt = reinterpret_cast<int*>(smem + 64);
+    const int tid = threadIdx.x;
+    double* sl = reinterpret_cast<double*>(smem + team_header(LC));
     if constexpr (LC < 0) {
         // recursion neighbours: axis, the two lower entries, the second one's factor
         for (int e = threadIdx.x; e < 455; e += blockDim.x) {
@@ -282,17 +282,18 @@ __global__ void __launch_bounds__(128, 4) k_team(TeamArgs a)
         const int HL = team_nherm(L), HS = HL | 1, H1 = team_nherm(L1);
         const int nA = bra0.nA, nB = bra0.nB, nC = ket.nA, nD = ket.nB, nab = nA * nB, ncd = nC * nD, nout = nab * ncd;
         const int nmb = bra0.nmem, nmk = ket.nmem, npk = ket.npp, nfb = nA + nB;
-        const int As = nout | 1, Ws = (ncd * H1) | 1;   // odd strides of bra blocks and W rows: no bank conflicts
+        const int As = nout | 1;                        // odd strides of bra blocks and W rows: no bank conflicts
         double* acc = sl;
         double* W = acc + t.parts * t.slots * As;
-        double* R = W + t.nw * Ws;
+        double* R = W + team_w(H1, nA, nB, nC, nD, t.nw, t.slots);
         double* R2 = R + t.nr * t.nkb * HS;                                     // second buffer and seeds (general L)
         double* S = R2 + (LC < 0 && L > kTeamMaxRegL ? t.nr * t.nkb * HS : 0);
         int* rowd = reinterpret_cast<int*>(S + (LC < 0 && L > kTeamMaxRegL ? (L + 1) * t.nr * t.nkb : 0));
         int* rstart = rowd + t.nr;
         int* bid = rstart + t.nb + 1;              // pair of each bra
-        int* kmem = bid + t.nb;                    // ket members: list start, length, coefficients, class | count << 16
-        int* kfn = kmem + 4 * nmk;                 // ket function indices
+        int* kmem = bid + t.nb;                    // ket members: list start, length, coefficients, class | count << 16,
+                                                   // first and last list entry
+        int* kfn = kmem + 6 * nmk;                 // ket function indices
         int* border = kfn + nC + nD;               // component pairs by decreasing work
         int* korder = border + nab;
         int* bfn = korder + ncd;                   // function indices of the round's bra pairs
@@ -301,16 +302,45 @@ __global__ void __launch_bounds__(128, 4) k_team(TeamArgs a)
             const int* tab = ket.tab;
             const int* ty = ket.type + ncd;
             for (int m = tid; m < nmk; m += TEAM) {
-                kmem[4 * m] = __ldg(tab + m);
-                kmem[4 * m + 1] = __ldg(tab + nmk + m);
-                kmem[4 * m + 2] = __ldg(tab + 2 * nmk + m);
-                kmem[4 * m + 3] = __ldg(ty + m) | __ldg(ty + nmk + m) << 16;
+                const int ls = __ldg(tab + m), lc = __ldg(tab + nmk + m);
+                kmem[6 * m] = ls;
+                kmem[6 * m + 1] = lc;
+                kmem[6 * m + 2] = __ldg(tab + 2 * nmk + m);
+                kmem[6 * m + 3] = __ldg(ty + m) | __ldg(ty + nmk + m) << 16;
+                kmem[6 * m + 4] = lc > 0 ? __ldg(tab + ls) : 0;
+                kmem[6 * m + 5] = lc > 0 ? __ldg(tab + ls + lc - 1) : -1;
             }
             for (int m = tid; m < nC + nD; m += TEAM) kfn[m] = __ldg(tab + 3 * nmk + m);
-            for (int m = tid; m < ncd; m += TEAM) korder[m] = __ldg(tab + 3 * nmk + nC + nD + m);
-            for (int m = tid; m < nab; m += TEAM) border[m] = __ldg(bra0.tab + 3 * nmb + nfb + m);
             for (int m = tid; m < t.nb; m += TEAM) bid[m] = a.order[t.b0 + m];
         }
+
+        // Component pairs in use, by decreasing work: those of the members
+        // that can reach the cut with the task's largest bra pair (the first)
+        // resp. with the ket pair (single bra pair).  The others' integrals
+        // stay zero: each is below the cut.
+        const double cut = a.mode == kTeamDiag ? -1.0 : a.mixed ? ket.cut32 : a.thr;
+        auto in_use = [&](const SuperPair& s, int nfn, int n, double other, double cut, int step, int* list) {
+            const int* seq = s.tab + 3 * s.nmem + nfn;
+            int got = 0;
+            for (int x0 = 0; x0 < n; x0 += 32) {
+                const int x = x0 + (tid & 31), v = x < n ? __ldg(seq + x) : 0;
+                const bool use = x < n && (cut <= 0.0 || __ldg(s.mq + (__ldg(s.type + v) & 255)) * other >= cut);
+                const unsigned m = __ballot_sync(0xffffffffu, use);
+                if (use) list[got + __popc(m & ((1u << (tid & 31)) - 1u))] = v;
+                got += __popc(m);
+            }
+            // up to a whole group of `step` component pairs, with ones not in use
+            for (int x = 0; x < n && got % step; ++x) {
+                const int v = __ldg(seq + x);
+                if (cut > 0.0 && __ldg(s.mq + (__ldg(s.type + v) & 255)) * other < cut) list[got++] = v;
+            }
+            return got;
+        };
+        const int nce = in_use(ket, nC + nD, ncd, bra0.qmax, cut, team_cd_group(ncd), korder);
+        const int nae = in_use(bra0, nfb, nab, ket.qmax, single ? cut : -1.0, 1, border);
+        const int Ws = (nce * H1) | 1;
+        if (nce < ncd || nae < nab)
+            for (int x = tid; x < t.parts * t.slots * As; x += TEAM) acc[x] = 0.0;
 
         // rows of the task: (bra slot, bra primitive pair); a bra pair whose
         // quartet the density screen drops gets no rows
@@ -440,16 +470,16 @@ __global__ void __launch_bounds__(128, 4) k_team(TeamArgs a)
         auto make_W_j = [&](auto jt, int w0, int nw, int k0, int nk, bool first) {
             constexpr int JT = decltype(jt)::value;
             const int ng = (H1 + JT - 1) / JT;             // groups per row
-            const int n = ncd * nw * ng;
+            const int n = nce * nw * ng;
             const float ing = 1.0f / ng, inw = 1.0f / nw;
             for (int o = tid; o < n; o += TEAM) {
                 const int q = fdiv(o, ng, ing), g = o - q * ng, cw = fdiv(q, nw, inw), row = q - cw * nw;
                 const int cd = korder[cw];
                 const unsigned fw = __ldg(ktype + cd);
                 const int m = fw & 255, ko = (fw >> 8) & 4095, nc = fw >> 20;
-                const int lc = kmem[4 * m + 1], cls = kmem[4 * m + 3] & 0xffff, nco = kmem[4 * m + 3] >> 16;
-                const double* cf = kcoef + kmem[4 * m + 2] + ko;
-                const int* list = ktab + kmem[4 * m];
+                const int lc = kmem[6 * m + 1], cls = kmem[6 * m + 3] & 0xffff, nco = kmem[6 * m + 3] >> 16;
+                const double* cf = kcoef + kmem[6 * m + 2] + ko;
+                const int* list = ktab + kmem[6 * m];
                 const short* codes = a.kcode + cls + ko;
                 const double* Rr = R + (size_t)(w0 + row) * nk * HS;
                 double s[JT];
@@ -458,12 +488,9 @@ __global__ void __launch_bounds__(128, 4) k_team(TeamArgs a)
                 const bool all = lc == npk;
                 int e0 = k0, e1 = k0 + nk;
                 if (!all) {
-                    e0 = 0;
-                    e1 = lc;
-                    if (nk < npk) {
-                        e0 = first_at_least(list, lc, k0);
-                        e1 = first_at_least(list, lc, k0 + nk);
-                    }
+                    const int lo = kmem[6 * m + 4], hi = kmem[6 * m + 5];
+                    e0 = lo >= k0 ? 0 : hi < k0 ? lc : first_at_least(list, lc, k0);
+                    e1 = hi < k0 + nk ? lc : lo >= k0 + nk ? 0 : first_at_least(list, lc, k0 + nk);
                 }
 #pragma unroll 2
                 for (int k = 0; k < nc; ++k) {
@@ -496,10 +523,10 @@ __global__ void __launch_bounds__(128, 4) k_team(TeamArgs a)
                         }
                     }
                 }
-                double* w = W + row * Ws + g * JT * ncd + cd;
+                double* w = W + row * Ws + g * JT * nce + cw;
 #pragma unroll
                 for (int j = 0; j < JT; ++j)
-                    if (g * JT + j < H1) w[j * ncd] = first ? s[j] : w[j * ncd] + s[j];
+                    if (g * JT + j < H1) w[j * nce] = first ? s[j] : w[j * nce] + s[j];
             }
         };
         auto make_W = [&](int w0, int nw, int k0, int nk, bool first) {
@@ -514,7 +541,7 @@ __global__ void __launch_bounds__(128, 4) k_team(TeamArgs a)
         // step 3: bra transform of one bra pair's `rows` rows from W row w0
         // on, its primitive pairs [ij0, ij0 + rows), into JC consecutive
         // component pairs cd of one ab; first: store, else add
-        auto bra_j = [&](auto jc, const SuperPair& bra, double* out, int ab, int cd, int w0, int ij0, int rows,
+        auto bra_j = [&](auto jc, const SuperPair& bra, double* out, int ab, int cw, int w0, int ij0, int rows,
                          bool first, int part, int parts) {
             constexpr int JC = decltype(jc)::value;
             const unsigned fw = __ldg(btype + ab);
@@ -536,25 +563,28 @@ __global__ void __launch_bounds__(128, 4) k_team(TeamArgs a)
             for (int j = 0; j < JC; ++j) s[j] = 0.0;
             for (int e = e0 + part; e < e1; e += parts) {
                 const int r = (all ? e : __ldg(list + e)) - ij0;
-                const double* w = W + (w0 + r) * Ws + cd;
+                const double* w = W + (w0 + r) * Ws + cw;
                 const double* c = cf + (size_t)e * nco;
 #pragma unroll 4
                 for (int k = 0; k < nc; ++k) {
                     const double cv = __ldg(c + k);
-                    const double* wk = w + (__ldg(codes + k) & 16383) * ncd;
+                    const double* wk = w + (__ldg(codes + k) & 16383) * nce;
 #pragma unroll
                     for (int j = 0; j < JC; ++j) s[j] = fma(cv, wk[j], s[j]);
                 }
             }
 #pragma unroll
-            for (int j = 0; j < JC; ++j) out[ab * ncd + cd + j] = first ? s[j] : out[ab * ncd + cd + j] + s[j];
+            for (int j = 0; j < JC; ++j) {
+                double* v = out + ab * ncd + korder[cw + j];
+                *v = first ? s[j] : *v + s[j];
+            }
         };
         // the bra transform of `ns` bra pairs (slots s0..) over the team
         auto make_acc = [&](int s0, int ns, int w0, bool first, int r0, int nr) {
             auto run = [&](auto jc) {
                 constexpr int JC = decltype(jc)::value;
                 // ab slowest: a warp's lanes share the bra coefficients' pattern
-                const int ng = ncd / JC, ngp = ng * t.parts, per = ns * ngp, n = nab * per;
+                const int ng = nce / JC, ngp = ng * t.parts, per = ns * ngp, n = nae * per;
                 const float iper = 1.0f / per, ingp = 1.0f / ngp, ing = 1.0f / ng;
                 for (int x = tid; x < n; x += TEAM) {
                     const int aw = fdiv(x, per, iper), y = x - aw * per, ab = border[aw];
@@ -567,10 +597,11 @@ __global__ void __launch_bounds__(128, 4) k_team(TeamArgs a)
                 }
             };
             // several component pairs per thread where that leaves no thread idle
-            const int n = ns * nout * t.parts;
-            if (ncd % 4 == 0 && n >= 4 * TEAM)
+            const int n = ns * nae * nce * t.parts;
+            const int step = team_cd_group(ncd);
+            if (step == 4 && n >= 4 * TEAM)
                 run(CInt<4>{});
-            else if (ncd % 3 == 0 && n >= 3 * TEAM)
+            else if (step == 3 && n >= 3 * TEAM)
                 run(CInt<3>{});
             else
                 run(CInt<1>{});
@@ -590,98 +621,138 @@ __global__ void __launch_bounds__(128, 4) k_team(TeamArgs a)
                 bfn[x] = __ldg(a.pairs[bid[s0 + s]].tab + 3 * nmb + x - s * nfb);
             }
             team_sync<TEAM>();
+            // per function pair of the round (bra pairs by slot, then the ket
+            // pair): member bound, Schwarz bound (negative: not a unique
+            // pair), pair index | (i != j) << 31
+            double* pm = W;     // W is not needed any more
+            float* pq = reinterpret_cast<float*>(pm + ns * nab + ncd);
+            unsigned* pp = reinterpret_cast<unsigned*>(pq + ns * nab + ncd);
+            const float inab = 1.0f / nab;
+            for (int x = tid; x < ns * nab + ncd; x += TEAM) {
+                const bool isket = x >= ns * nab;
+                const int s = isket ? 0 : fdiv(x, nab, inab), e = isket ? x - ns * nab : x - s * nab;
+                const int b = isket ? ketid : bid[s0 + s], n = isket ? nD : nB, u = e / n;
+                const int* f = isket ? kfn : bfn + s * nfb;
+                const int i = f[u], j = f[(isket ? nC : nA) + e - u * n];
+                const unsigned q = (unsigned)tri(i, j);
+                const float v = __ldg(Qf + q);
+                pq[x] = i < j && a.pairs[b].same ? -1.0f : v;
+                pp[x] = q | (i != j ? 0x80000000u : 0u);
+                if (a.mixed) pm[x] = __ldg(a.pairs[b].mq + (__ldg((isket ? ktype : btype) + e) & 255));
+            }
+            team_sync<TEAM>();
             for (int x = tid; x < ns * nout; x += TEAM) {
                 const int s = fdiv(x, nout, inout), o = x - s * nout, ab = fdiv(o, ncd, incd), cd = o - ab * ncd;
-                const int ia = ab / nB, ic = cd / nD;
-                const int* fb = bfn + s * nfb;
-                const int i = fb[ia], j = fb[nA + ab - ia * nB];
-                const int k = kfn[ic], l = kfn[nC + cd - ic * nD];
-                const long long pij = tri(i, j), pkl = tri(k, l);
-                const int b = bid[s0 + s];
-                bool skip = (i < j && a.pairs[b].same) || (k < l && ketsame) || (b == ketid && pij < pkl);
-                if (a.mixed && !skip)
-                    skip = __ldg(a.pairs[b].mq + (__ldg(btype + ab) & 255)) * __ldg(ket.mq + (__ldg(ktype + cd) & 255)) <
-                           ket.cut32;
+                const int xb = s * nab + ab, xk = ns * nab + cd;
+                const float qb = pq[xb], qk = pq[xk];
+                const unsigned eb = pp[xb], ek = pp[xk], pij = eb & 0x7fffffffu, pkl = ek & 0x7fffffffu;
+                bool skip = qb < 0.0f || qk < 0.0f || (pij < pkl && bid[s0 + s] == ketid);
+                if (a.mixed) skip = skip || pm[xb] * pm[xk] < ket.cut32;
                 if (a.screen) {
                     // decided in float away from the threshold, in double near it
-                    const float f = __ldg(Qf + pij) * __ldg(Qf + pkl);
+                    const float f = qb * qk;
                     if (f < a.thr_hi) skip = skip || f < a.thr_lo || __ldg(Qb + pij) * __ldg(Qb + pkl) < a.thr;
                 }
                 double* v = acc + s * As + o;
                 for (int part = 1; part < t.parts; ++part) *v += v[part * t.slots * As];
-                *v = skip ? 0.0 : times_pow2(*v, (i != j) + (k != l) + (pij != pkl));
+                *v = skip ? 0.0 : times_pow2(*v, (int)(eb >> 31) + (int)(ek >> 31) + (pij != pkl));
             }
             team_sync<TEAM>();
-            // every J and K element of the blocks: the sum over the block of
-            // density x integral, one thread each
+            // The six blocks of function pairs that a quartet touches, per bra
+            // pair: AB, CD, then per exchange matrix AC, BD, AD, BC.  Their
+            // densities go to shared memory in one pass (one load latency;
+            // with the loads inside the sums the digestion took 5.8 of the
+            // 17.1 ms of n-decane/6-31G*'s launches); then one thread sums
+            // each element of J and K over the opposite block.
             const int nac = nA * nC, nbd = nB * nD, nad = nA * nD, nbc = nB * nC, nx = nac + nbd + nad + nbc;
-            const int per = nab + ncd + a.nk * nx;
+            const int per = nab + ncd + a.nk * nx, Ds = per | 1;
             const float ins = 1.0f / ns;
+            double* Dl = W;
+            // row and column of element o of bra pair s, and its matrix (0: J, 1, 2: exchange)
+            auto element = [&](int o, int s, int& r, int& c) {
+                const int* fb = bfn + s * nfb;
+                if (o < nab) {
+                    const int ia = o / nB;
+                    r = fb[ia]; c = fb[nA + o - ia * nB];
+                    return 0;
+                }
+                if ((o -= nab) < ncd) {
+                    const int ic = o / nD;
+                    r = kfn[ic]; c = kfn[nC + o - ic * nD];
+                    return 0;
+                }
+                o -= ncd;
+                const int sp = o >= nx;
+                o -= sp ? nx : 0;
+                const bool b = o >= nac && (o < nac + nbd || o >= nac + nbd + nad);     // row from B
+                const bool dd = o >= nac && o < nac + nbd + nad;                         // column from D
+                o -= o < nac ? 0 : o < nac + nbd ? nac : o < nac + nbd + nad ? nac + nbd : nac + nbd + nad;
+                const int n = dd ? nD : nC, x = o / n;
+                r = fb[b ? nA + x : x]; c = kfn[dd ? nC + o - x * n : o - x * n];
+                return 1 + sp;
+            };
             // bra pair fastest: a warp's lanes sum blocks of one shape
+            for (int x = tid; x < ns * per; x += TEAM) {
+                const int o = fdiv(x, ns, ins), s = x - o * ns;
+                int r, c;
+                const int m = element(o, s, r, c);
+                const double* D = m == 0 ? Dj : (m == 1 ? a.Dk : a.Dk2) + moff;
+                Dl[s * Ds + o] = __ldg(D + (long long)r * K + c);
+            }
+            team_sync<TEAM>();
             for (int x = tid; x < ns * per; x += TEAM) {
                 int o = fdiv(x, ns, ins);
                 const int s = x - o * ns;
-                const int* fb = bfn + s * nfb;
+                int r, c;
+                const int m = element(o, s, r, c);
                 const double* v = acc + s * As;
-                const double* __restrict__ D = Dj;
-                double* M = a.J + moff;
-                // element (r, c); the summed block: n1 x n2 entries with
-                // strides s1, s2, their functions f1, f2
-                int r, c, n1, n2, s1, s2;
-                const int *f1, *f2;
+                const double* D = Dl + s * Ds;
+                int n1, n2, s1, s2;                   // the opposite block and its strides in the quartet's
                 if (o < nab) {                        // J_ij += D_kl
                     v += o * ncd;
-                    n1 = nC; n2 = nD; s1 = nD; s2 = 1;
-                    f1 = kfn; f2 = kfn + nC;
-                    const int ia = o / nB;
-                    r = fb[ia]; c = fb[nA + o - ia * nB];
+                    D += nab;
+                    n1 = 1; n2 = ncd; s1 = 0; s2 = 1;
                 } else if ((o -= nab) < ncd) {        // J_kl += D_ij
                     v += o;
-                    n1 = nA; n2 = nB; s1 = nB * ncd; s2 = ncd;
-                    f1 = fb; f2 = fb + nA;
-                    const int ic = o / nD;
-                    r = kfn[ic]; c = kfn[nC + o - ic * nD];
+                    n1 = 1; n2 = nab; s1 = 0; s2 = ncd;
                 } else {
                     o -= ncd;
-                    const bool sp = o >= nx;
-                    o -= sp ? nx : 0;
-                    D = (sp ? a.Dk2 : a.Dk) + moff;
-                    M = (sp ? a.Kx2 : a.Kx) + moff;
+                    D += nab + ncd;
+                    if (o >= nx) {
+                        o -= nx;
+                        D += nx;
+                    }
                     if (o < nac) {                    // K_ik += D_jl
-                        r = o / nC; c = o - r * nC;
-                        v += r * nB * ncd + c * nD;
+                        const int x1 = o / nC;
+                        v += x1 * nB * ncd + (o - x1 * nC) * nD;
+                        D += nac;
                         n1 = nB; n2 = nD; s1 = ncd; s2 = 1;
-                        f1 = fb + nA; f2 = kfn + nC;
-                        r = fb[r]; c = kfn[c];
                     } else if ((o -= nac) < nbd) {    // K_jl += D_ik
-                        r = o / nD; c = o - r * nD;
-                        v += r * ncd + c;
+                        const int x1 = o / nD;
+                        v += x1 * ncd + o - x1 * nD;
                         n1 = nA; n2 = nC; s1 = nB * ncd; s2 = nD;
-                        f1 = fb; f2 = kfn;
-                        r = fb[nA + r]; c = kfn[nC + c];
                     } else if ((o -= nbd) < nad) {    // K_il += D_jk
-                        r = o / nD; c = o - r * nD;
-                        v += r * nB * ncd + c;
+                        const int x1 = o / nD;
+                        v += x1 * nB * ncd + o - x1 * nD;
+                        D += nac + nbd + nad;
                         n1 = nB; n2 = nC; s1 = ncd; s2 = nD;
-                        f1 = fb + nA; f2 = kfn;
-                        r = fb[r]; c = kfn[nC + c];
                     } else {                          // K_jk += D_il
                         o -= nad;
-                        r = o / nC; c = o - r * nC;
-                        v += r * ncd + c * nD;
+                        const int x1 = o / nC;
+                        v += x1 * ncd + (o - x1 * nC) * nD;
+                        D += nac + nbd;
                         n1 = nA; n2 = nD; s1 = nB * ncd; s2 = 1;
-                        f1 = fb; f2 = kfn + nC;
-                        r = fb[nA + r]; c = kfn[c];
                     }
                 }
                 double sum = 0.0;
-                for (int x1 = 0; x1 < n1; ++x1) {
-                    const double* Dr = D + (long long)f1[x1] * K;
-                    const double* vr = v + x1 * s1;
+                for (int x1 = 0; x1 < n1; ++x1, v += s1, D += n2) {
 #pragma unroll 4
-                    for (int x2 = 0; x2 < n2; ++x2) sum = fma(__ldg(Dr + f2[x2]), vr[x2 * s2], sum);
+                    for (int x2 = 0; x2 < n2; ++x2) sum = fma(D[x2], v[x2 * s2], sum);
                 }
-                if (__double_as_longlong(sum) << 1) atomicAdd(M + (long long)r * K + c, sum);
+                if (__double_as_longlong(sum) << 1) {
+                    double* M = m == 0 ? a.J : m == 1 ? a.Kx : a.Kx2;
+                    atomicAdd(M + moff + (long long)r * K + c, sum);
+                }
             }
         };
 
@@ -720,8 +791,8 @@ __global__ void __launch_bounds__(128, 4) k_team(TeamArgs a)
                     team_sync<TEAM>();
                 }
                 if (a.mode == kTeamDiag) {
-                    for (int ab = tid; ab < nab; ab += TEAM)
-                        bra_j(CInt<1>{}, bra0, acc, ab, ab, 0, t.i0 + r0, nr, r0 == 0, 0, 1);
+                    for (int x = tid; x < nab; x += TEAM)
+                        bra_j(CInt<1>{}, bra0, acc, korder[x], x, 0, t.i0 + r0, nr, r0 == 0, 0, 1);
                 } else {
                     make_acc(0, 1, 0, r0 == 0, r0, nr);
                 }
@@ -875,16 +946,14 @@ KernelSpec team_density_spec(int npairs)
 cudaError_t team_spec(const TeamGroup& g, int nsm, KernelSpec* s)
 {
     s->func = g.team == 32 ? team_kernel<32>(g.L) : team_kernel<128>(g.L);
-    s->block = dim3(128);
-    const int teams = 128 / g.team;
-    s->smem = kTeamHeaderBytes + sizeof(double) * (size_t)g.slice * teams;
+    s->block = dim3((unsigned)g.team);
+    s->smem = team_header(g.L) + sizeof(double) * (size_t)g.slice;
     cudaError_t e = allow_smem(s->func);
     if (e != cudaSuccess) return e;
     int per = 1;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, s->func, 128, s->smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, s->func, g.team, s->smem);
     if (e != cudaSuccess) return e;
-    const long long need = ((long long)g.n + teams - 1) / teams;
-    s->grid = dim3((unsigned)std::min<long long>(need, (long long)nsm * std::max(1, per)));
+    s->grid = dim3((unsigned)std::min<long long>((long long)g.n, (long long)nsm * std::max(1, per)));
     return cudaSuccess;
 }
 

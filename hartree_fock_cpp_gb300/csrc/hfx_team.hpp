@@ -25,7 +25,6 @@ namespace hfx {
 // up to ten, f): bounds the Cartesian block of a quartet to 36 x 36, 10 KB of
 // shared memory.
 constexpr int kSuperMaxFn = 6;
-constexpr int kTeamMaxMembers = kSuperMaxFn * kSuperMaxFn;
 
 // Primitive-pair header: p, Px, Py, Pz, sqrt(2 pi^{5/2}) / p, unused.
 constexpr int kTeamHdr = 6;
@@ -119,20 +118,31 @@ __host__ __device__ constexpr int team_nherm(int L) { return (L + 1) * (L + 2) *
 // largest total angular momentum whose R table a thread keeps in registers
 constexpr int kTeamMaxRegL = 6;
 
+// W's part of a slice (doubles): nw rows, or the function pairs and the density
+// blocks of a round of the digestion, which take its place.
+__host__ __device__ inline int team_w(int H1, int nA, int nB, int nC, int nD, int nw, int slots)
+{
+    const int w = nw * ((nC * nD * H1) | 1), d = slots * ((nA * nB + nC * nD + 2 * (nA + nB) * (nC + nD)) | 1);
+    const int p = 2 * (slots * nA * nB + nC * nD);
+    return w > d ? (w > p ? w : p) : (d > p ? d : p);
+}
 // Shared-memory slice of a task (doubles): Cartesian blocks, ket-transformed
 // Hermite integrals, R tables (two and the seeds beyond kTeamMaxRegL), row
 // descriptors.
-__host__ __device__ inline int team_slice(int L1, int L2, int nab, int ncd, int nr, int nkb, int nw, int slots, int nb,
-                                          int parts)
+__host__ __device__ inline int team_slice(int L1, int L2, int nA, int nB, int nC, int nD, int nr, int nkb, int nw, int slots, int nb,
+                                          int parts, int nmk)
 {
     const int L = L1 + L2, HS = team_nherm(L) | 1;
-    int n = parts * slots * (nab * ncd | 1) + nw * (ncd * team_nherm(L1) | 1) + nr * nkb * HS;
+    const int nab = nA * nB, ncd = nC * nD;
+    int n = parts * slots * (nab * ncd | 1) + team_w(team_nherm(L1), nA, nB, nC, nD, nw, slots) + nr * nkb * HS;
     if (L > kTeamMaxRegL) n += nr * nkb * HS + (L + 1) * nr * nkb;
     // ints: rows, row starts, bra pairs, ket members and functions, bra
     // functions, the two orders of component pairs
-    n += (nr + 2 * nb + 1 + 4 * kTeamMaxMembers + 20 + 20 * slots + nab + ncd + 1) / 2;
+    n += (nr + 2 * nb + 1 + 6 * nmk + 20 + 20 * slots + nab + ncd + 1) / 2;
     return (n + 3) & ~1;
 }
+// Component pairs cd that one thread of step 3 computes where they are many.
+__host__ __device__ constexpr int team_cd_group(int ncd) { return ncd % 4 == 0 ? 4 : ncd % 3 == 0 ? 3 : 1; }
 // Consecutive tuv that one thread of step 2 computes (H1 > 1).
 __host__ __device__ constexpr int team_tuv_group(int H1) { return H1 == 10 || H1 == 20 || H1 == 35 ? 5 : 4; }
 
@@ -140,7 +150,7 @@ __host__ __device__ constexpr int team_tuv_group(int H1) { return H1 == 10 || H1
 // form), team size and slice tier.
 struct TeamGroup {
     int L;               // compiled total angular momentum, -1: general
-    int team;            // threads per team (32: four teams per CTA, 128: one)
+    int team;            // threads per team, one team per CTA
     int slice;           // doubles per team
     size_t off, n;
     double cost;
