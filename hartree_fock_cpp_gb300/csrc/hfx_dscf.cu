@@ -53,13 +53,15 @@ __global__ void k_axpby(int n, double a, const double* A, double b, const double
 {
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) C[e] = a * A[e] + b * B[e];
 }
-// E = T - T^T (column-major K x K)
-__global__ void k_antisym(int K, const double* T, double* E)
+// E = T - T^T (column-major K x K), and a copy of it where C is given
+__global__ void k_antisym(int K, const double* T, double* E, double* C)
 {
     int n = K * K;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         int i = e % K, j = e / K;
-        E[e] = T[e] - T[j + i * K];
+        const double v = T[e] - T[j + i * K];
+        E[e] = v;
+        if (C) C[e] = v;
     }
 }
 struct Coef8 {
@@ -74,6 +76,40 @@ __global__ void k_lincomb(int n, Coef8 cf, double* C)
         double s = 0.0;
         for (int i = 0; i < cf.n; ++i) s += cf.c[i] * cf.m[i][e];
         C[e] = s;
+    }
+}
+
+// Sums over the n elements of matrices, one CTA each: a.b, a.(b + c) or
+// |a - b|^2.  An iteration's inner products (DIIS row, energy, norms) are one
+// launch; as one cuBLAS call each they were 22 of them for two spins.
+enum DotMode { kDot = 0, kDotSum = 1, kDiff2 = 2 };
+constexpr int kMaxDots = 24;
+struct DotList {
+    const double *a[kMaxDots], *b[kMaxDots], *c[kMaxDots];
+    int mode[kMaxDots], slot[kMaxDots];
+    int count = 0;
+};
+__global__ void __launch_bounds__(1024) k_dots(int n, DotList d, double* out)
+{
+    __shared__ double part[32];
+    const int q = blockIdx.x, mode = d.mode[q];
+    const double *a = d.a[q], *b = d.b[q], *c = d.c[q];
+    double s = 0.0;
+    for (int e = threadIdx.x; e < n; e += blockDim.x) {
+        if (mode == kDiff2) {
+            const double v = a[e] - b[e];
+            s = fma(v, v, s);
+        } else {
+            s = fma(a[e], mode == kDotSum ? b[e] + c[e] : b[e], s);
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        s = threadIdx.x < (blockDim.x >> 5) ? part[threadIdx.x] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (threadIdx.x == 0) out[d.slot[q]] = s;
     }
 }
 
@@ -125,6 +161,7 @@ void release_handles(HandlePair h)
 DeviceScf::DeviceScf(FockSource& job, const ScfSetup& setup, int nspin) : job_(job), K_(job.K()), nspin_(nspin)
 {
     st_ = job.stream();
+    dots_.reset(new DotList());
     HandlePair h = acquire_handles();
     blas_ = h.blas;
     solver_ = h.solver;
@@ -182,16 +219,28 @@ void DeviceScf::gemm(bool ta, const double* A, bool tb, const double* B, double*
                  "dgemm");
 }
 
-// dot products of device vectors into the device scalar slot `slot`
-void DeviceScf::dot(const double* a, const double* b, int n, int slot)
+void DeviceScf::add_dot(int mode, const double* a, const double* b, const double* c, int slot)
 {
-    cublas_check(cublasSetPointerMode(blas_, CUBLAS_POINTER_MODE_DEVICE), "pointer mode");
-    cublas_check(cublasDdot(blas_, n, a, 1, b, 1, scal_.p + slot), "ddot");
-    cublas_check(cublasSetPointerMode(blas_, CUBLAS_POINTER_MODE_HOST), "pointer mode");
+    DotList& d = *dots_;
+    d.a[d.count] = a;
+    d.b[d.count] = b;
+    d.c[d.count] = c;
+    d.mode[d.count] = mode;
+    d.slot[d.count] = slot;
+    if (++d.count == kMaxDots) run_dots();
+}
+
+void DeviceScf::run_dots()
+{
+    if (dots_->count == 0) return;
+    k_dots<<<dots_->count, 1024, 0, st_>>>(K_ * K_, *dots_, scal_.p);
+    dots_->count = 0;
+    cuda_check(cudaGetLastError(), "dots");
 }
 
 void DeviceScf::fetch(double* host, int count)
 {
+    run_dots();
     cuda_check(cudaMemcpyAsync(host, scal_.p, sizeof(double) * count, cudaMemcpyDeviceToHost, st_), "D2H scalars");
     cuda_check(cudaStreamSynchronize(st_), "scf sync");
 }
@@ -255,17 +304,16 @@ void DeviceScf::build(int mode, double dthr)
 
 // E_[s] = F P S - S P F for every spin; energy terms and norms into scal_
 // slots: [0] = sum_s 1/2 P.(H+F), [1] = sum_s ||E_s||^2
-void DeviceScf::error_and_energy()
+void DeviceScf::error_and_energy(double* const* Ecopy)
 {
     const int n = K_ * K_;
     for (int s = 0; s < nspin_; ++s) {
         gemm(false, F_[s].p, false, P_[s].p, T1_.p);
         gemm(false, T1_.p, false, S_.p, T2_.p);
-        k_antisym<<<grid_for(n), 256, 0, st_>>>(K_, T2_.p, E_[s].p);
+        k_antisym<<<grid_for(n), 256, 0, st_>>>(K_, T2_.p, E_[s].p, Ecopy ? Ecopy[s] : nullptr);
         cuda_check(cudaGetLastError(), "antisym");
-        axpby(1.0, H_.p, 1.0, F_[s].p, T1_.p);
-        dot(P_[s].p, T1_.p, n, 10 + s);
-        dot(E_[s].p, E_[s].p, n, 12 + s);
+        add_dot(kDotSum, P_[s].p, H_.p, F_[s].p, 10 + s);
+        add_dot(kDot, E_[s].p, E_[s].p, nullptr, 12 + s);
     }
 }
 
@@ -276,29 +324,39 @@ void DeviceScf::error_and_energy()
 // (column-major); F' stays in Fq_[s] for a later syevd.
 void DeviceScf::diagonalise(const double* const* Fs, const int* nocc, double occ_factor, bool use_proj)
 {
+    int spins[2], count = 0, steps = 0;
     for (int s = 0; s < nspin_; ++s) {
         gemm(false, Fs[s], false, X_.p, T1_.p);        // F X
         gemm(true, X_.p, false, T1_.p, Fq_[s].p);      // X^T F X
         proj_[s] = use_proj && nocc[s] > 0 && nocc[s] < K_;
         if (proj_[s]) {
             // the step count changes little between SCF iterations
-            project(s, nocc[s], occ_factor, proj_steps_[s] > 0 ? proj_steps_[s] + 5 : Sp2Projector::kMaxSteps);
+            spins[count++] = s;
+            steps = std::max(steps, proj_steps_[s] > 0 ? proj_steps_[s] + 5 : Sp2Projector::kMaxSteps);
         } else {
             eigensolve(s, nocc[s], occ_factor, true);
         }
     }
+    if (count > 0) project(spins, count, nocc, occ_factor, steps);
 }
 
-void DeviceScf::project(int s, int nocc, double occ_factor, int max_steps)
+// The spins' projectors in the same launches, then their densities.
+void DeviceScf::project(const int* spins, int count, const int* nocc, double occ_factor, int max_steps)
 {
-    if (!sp2_) {
-        sp2_.reset(new Sp2Projector(K_));
-        D_.alloc((size_t)K_ * K_);
+    if (!sp2_) sp2_.reset(new Sp2Projector(K_));
+    Sp2Projector::Task t[2];
+    for (int x = 0; x < count; ++x) {
+        const int s = spins[x];
+        D_[s].alloc((size_t)K_ * K_);
+        proj_cap_[s] = max_steps;
+        t[x] = Sp2Projector::Task{Fq_[s].p, nocc[s], D_[s].p, scal_.p + 2 + s};
     }
-    proj_cap_[s] = max_steps;
-    sp2_->run(Fq_[s].p, nocc, D_.p, scal_.p + 2 + s, st_, max_steps);
-    gemm(false, X_.p, false, D_.p, T1_.p);                  // X D
-    gemm(false, T1_.p, true, T1_.p, Pn_[s].p, occ_factor);  // f (X D)(X D)^T = f X D X^T
+    sp2_->run(t, count, st_, max_steps);
+    for (int x = 0; x < count; ++x) {
+        const int s = spins[x];
+        gemm(false, X_.p, false, D_[s].p, T1_.p);               // X D
+        gemm(false, T1_.p, true, T1_.p, Pn_[s].p, occ_factor);  // f (X D)(X D)^T = f X D X^T
+    }
 }
 
 void DeviceScf::eigensolve(int s, int nocc, double occ_factor, bool density)
@@ -403,7 +461,6 @@ ScfOutput DeviceScf::run(const Basis& b, const ScfSetup& setup, const hfx_scf_op
             if (ctl->fault_at_iteration == n_it) throw Error(HFX_ERR_NUMERIC, "injected fault at an SCF iteration");
         }
         do_build();
-        error_and_energy();
         // history slot
         // slots in use are always a permutation of 0..size-1: reuse the oldest when full
         int slot;
@@ -413,14 +470,15 @@ ScfOutput DeviceScf::run(const Basis& b, const ScfSetup& setup, const hfx_scf_op
         } else {
             slot = (int)ring.size();
         }
-        for (int s = 0; s < nspin_; ++s) {
+        double* hEs[2] = {hE[slot * nspin_].p, nspin_ == 2 ? hE[slot * nspin_ + 1].p : nullptr};
+        error_and_energy(hEs);
+        for (int s = 0; s < nspin_; ++s)
             cuda_check(cudaMemcpyAsync(hF[slot * nspin_ + s].p, F_[s].p, bytes, cudaMemcpyDeviceToDevice, st_), "copy");
-            cuda_check(cudaMemcpyAsync(hE[slot * nspin_ + s].p, E_[s].p, bytes, cudaMemcpyDeviceToDevice, st_), "copy");
-        }
         ring.push_back(slot);
         // new row of B: <E_slot, E_r> summed over spins
         for (size_t q = 0; q < ring.size(); ++q)
-            for (int s = 0; s < nspin_; ++s) dot(hE[slot * nspin_ + s].p, hE[ring[q] * nspin_ + s].p, n, 16 + 2 * (int)q + s);
+            for (int s = 0; s < nspin_; ++s)
+                add_dot(kDot, hEs[s], hE[ring[q] * nspin_ + s].p, nullptr, 16 + 2 * (int)q + s);
         fetch(sc, 32);
         const double E_cur = 0.5 * (sc[10] + (nspin_ == 2 ? sc[11] : 0.0));
         const double en = std::sqrt(sc[12] + (nspin_ == 2 ? sc[13] : 0.0));
@@ -457,10 +515,7 @@ ScfOutput DeviceScf::run(const Basis& b, const ScfSetup& setup, const hfx_scf_op
         }
         diagonalise(Fuse, nocc, occf, use_proj);
         // RMSD(P_new - P) per spin
-        for (int s = 0; s < nspin_; ++s) {
-            axpby(1.0, Pn_[s].p, -1.0, P_[s].p, T1_.p);
-            dot(T1_.p, T1_.p, n, s);
-        }
+        for (int s = 0; s < nspin_; ++s) add_dot(kDiff2, Pn_[s].p, P_[s].p, nullptr, s);
         fetch(sc, 4);
         // a projection that did not converge within the step cap is repeated
         // with the full cap; one that did not converge at all (no gap at the
@@ -479,15 +534,14 @@ ScfOutput DeviceScf::run(const Basis& b, const ScfSetup& setup, const hfx_scf_op
                     continue;
                 }
                 if (proj_cap_[s] < Sp2Projector::kMaxSteps) {
-                    project(s, nocc[s], occf, Sp2Projector::kMaxSteps);
+                    project(&s, 1, nocc, occf, Sp2Projector::kMaxSteps);
                 } else {
                     ++out.projection_fallbacks;
                     proj_[s] = false;
                     proj_steps_[s] = 0;
                     eigensolve(s, nocc[s], occf, true);
                 }
-                axpby(1.0, Pn_[s].p, -1.0, P_[s].p, T1_.p);
-                dot(T1_.p, T1_.p, n, s);
+                add_dot(kDiff2, Pn_[s].p, P_[s].p, nullptr, s);
                 refetch = true;
             }
             if (!refetch) break;

@@ -38,11 +38,14 @@ public:
 
 private:
     void gemm(bool ta, const double* A, bool tb, const double* B, double* C, double alpha = 1.0, int kdim = 0);
-    void dot(const double* a, const double* b, int n, int slot);
+    // sums over all elements into scalar slots, one launch (mode: DotMode)
+    void add_dot(int mode, const double* a, const double* b, const double* c, int slot);
+    void run_dots();
     void fetch(double* host, int count);
     void axpby(double a, const double* A, double b, const double* B, double* C);
     void build(int mode, double dthr);
-    void error_and_energy();
+    // E_[s] (copied to Ecopy[s] where given), energy terms and norms into the scalar slots
+    void error_and_energy(double* const* Ecopy = nullptr);
     // new densities Pn_ of the (DIIS) Fock matrices; proj_[s] says which
     // spins took the SP2 projector (status in scalar slot 2 + s)
     void diagonalise(const double* const* Fs, const int* nocc, double occ_factor, bool use_proj);
@@ -50,7 +53,7 @@ private:
     // (density) the density Pn_
     void eigensolve(int s, int nocc, double occ_factor, bool density);
     // Pn_[s] from the SP2 projector of Fq_[s] within max_steps (status in slot 2 + s)
-    void project(int s, int nocc, double occ_factor, int max_steps);
+    void project(const int* spins, int count, const int* nocc, double occ_factor, int max_steps);
 
     FockSource& job_;
     int K_, nspin_;
@@ -58,8 +61,9 @@ private:
     cublasHandle_t blas_ = nullptr;
     cusolverDnHandle_t solver_ = nullptr;
     DevBuf<double> H_, S_, X_, T1_, T2_, Fp_, W_, work_, scal_, G_, dG_, Kr_;
-    DevBuf<double> P_[2], Pn_[2], F_[2], E_[2], C_[2], Gr_[2], Pr_[2], dP_[2], e_[2], Kx_[2], dK_[2], Fq_[2], D_;
+    DevBuf<double> P_[2], Pn_[2], F_[2], E_[2], C_[2], Gr_[2], Pr_[2], dP_[2], e_[2], Kx_[2], dK_[2], Fq_[2], D_[2];
     std::unique_ptr<Sp2Projector> sp2_;
+    std::unique_ptr<struct DotList> dots_;
     bool proj_[2] = {false, false};
     int proj_steps_[2] = {0, 0};  // steps the last projection took (0: unknown)
     int proj_cap_[2] = {0, 0};    // step cap of the projection in flight

@@ -632,9 +632,16 @@ void team_thresholds(TeamArgs& a, double thr, double dthr)
     a.dscreen = dthr > 0.0;
 }
 
-void TeamPlanDev::upload(const TeamPlanHost& h, cudaStream_t st)
+void TeamPlanDev::make_specs(int nsm)
+{
+    specs.resize(groups.size());
+    for (size_t g = 0; g < groups.size(); ++g) cuda_check(team_spec(groups[g], nsm, &specs[g]), "team kernel");
+}
+
+void TeamPlanDev::upload(const TeamPlanHost& h, int nsm, cudaStream_t st)
 {
     groups = h.groups;
+    make_specs(nsm);
     tasks.upload(h.tasks, st);
     order.upload(h.order, st);
 }
@@ -652,10 +659,8 @@ void Job::run_team(const TeamPlanDev& plan, int mode, double thr, double* out)
         a.mode = mode;
         team_thresholds(a, thr, 0.0);
         a.out = out;
-        KernelSpec ks;
-        cuda_check(team_spec(plan.groups[gi], nsm_, &ks), "team kernel");
         void* prm[] = {&a};
-        sk.kernel((int)(gi % (aux_.size() + 1)), ks, prm);
+        sk.kernel((int)(gi % (aux_.size() + 1)), plan.specs[gi], prm);
     }
     sk.join();
     cuda_check(cudaStreamSynchronize(stream_), "team kernel");
@@ -671,7 +676,7 @@ void Job::compute_schwarz()
     cuda_check(cudaMemsetAsync(d_qbf32_.p, 0, npair_bf * sizeof(float), stream_), "memset");
     const TeamPlanHost h = build_team_diagonal(sup_, nsm_);
     TeamPlanDev plan;
-    plan.upload(h, stream_);
+    plan.upload(h, nsm_, stream_);
     DevBuf<double> part;
     DevBuf<int> first;
     DevBuf<long long> qoff;
@@ -846,13 +851,6 @@ void Job::count_quartets(GroupSet& gs) const
     gs.nquartets = (int)quartets;
 }
 
-int Job::team_grid(const TeamGroup& g) const
-{
-    KernelSpec ks;
-    cuda_check(team_spec(g, nsm_, &ks), "team kernel");
-    return (int)ks.grid.x;
-}
-
 // The plan of one precision mode: FP64 quartets as tasks of the team kernel
 // over super pairs, and in a mixed plan the FP32 quartets (those whose own
 // bound is below the FP32 cut) as shell-quartet launch groups; the team kernel
@@ -874,7 +872,7 @@ void Job::build_jk_groups(bool mixed, GroupSet& gs)
     }
     const double thr = opt_.screening_threshold, tau = opt_.fp32_threshold;
     TeamPlanHost tp = build_team_plan(sup_, qsup_, mixed ? std::max(thr, tau) : thr, nsm_);
-    gs.team.upload(tp, stream_);
+    gs.team.upload(tp, nsm_, stream_);
     cuda_check(cudaStreamSynchronize(stream_), "plan upload");
     if (std::getenv("HFX_TRACE_SETUP"))
         std::fprintf(stderr, "team plan (%s): %zu tasks, %zu launches, %.1f ms\n", mixed ? "mixed" : "fp64",
@@ -1314,8 +1312,6 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
     const int n64 = groups.empty() ? naux + 1 : kFp64Lanes;
     for (size_t gi = 0; gi < gs.team.groups.size(); ++gi) {
         const TeamGroup& g = gs.team.groups[gi];
-        KernelSpec ks;
-        cuda_check(team_spec(g, nsm_, &ks), "team kernel");
         TeamArgs a = team_args(gs.team, g, ctr + groups.size() + gi);
         a.mode = kTeamFock;
         a.mixed = mixed_plan && mixed();
@@ -1330,7 +1326,7 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
         a.active = active;
         a.nk = nk;
         void* prm[] = {&a};
-        sk.kernel((int)(gi % n64), ks, prm);
+        sk.kernel((int)(gi % n64), gs.team.specs[gi], prm);
     }
     // FP32: on the lanes left, warp groups on the last
     int next_aux = 0;
@@ -1696,7 +1692,7 @@ void Job::eri_unique(double thr, double* out)
     cuda_check(cudaMemsetAsync(d_out.p, 0, nq * sizeof(double), stream_), "memset");
     // every super quartet whose bound can pass the BF-level test
     TeamPlanDev plan;
-    plan.upload(build_team_plan(sup_, qsup_, thr, nsm_), stream_);
+    plan.upload(build_team_plan(sup_, qsup_, thr, nsm_), nsm_, stream_);
     run_team(plan, kTeamEri, thr, d_out.p);
     cuda_check(cudaMemcpyAsync(out, d_out.p, nq * sizeof(double), cudaMemcpyDeviceToHost, stream_), "D2H");
     cuda_check(cudaStreamSynchronize(stream_), "eri_unique");

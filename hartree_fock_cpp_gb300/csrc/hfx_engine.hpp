@@ -159,9 +159,11 @@ void team_thresholds(TeamArgs& a, double thr, double dthr);
 // A team-kernel plan on the device.
 struct TeamPlanDev {
     std::vector<TeamGroup> groups;
+    std::vector<KernelSpec> specs;    // per group, kept: an eager build would query the occupancy 40 times
     DevBuf<TeamTask> tasks;
     DevBuf<int> order;
-    void upload(const TeamPlanHost& h, cudaStream_t st);
+    void upload(const TeamPlanHost& h, int nsm, cudaStream_t st);
+    void make_specs(int nsm);
 };
 
 // The launch plan of one precision mode.
@@ -301,7 +303,7 @@ public:
     // launch groups of a plan (FP64 or, for a mixed job, mixed)
     const std::vector<LaunchGroup>& plan_groups(bool mixed_plan) const { return plan(mixed_plan).groups; }
     const std::vector<TeamGroup>& plan_team(bool mixed_plan) const { return plan(mixed_plan).team.groups; }
-    int team_grid(const TeamGroup& g) const;
+    int team_grid(bool mixed_plan, size_t g) const { return (int)plan(mixed_plan).team.specs[g].grid.x; }
     void fock_uhf_device(const double* dPa, const double* dPb, double* dJ, double* dKa, double* dKb);
     void fock_rhf(const double* P, double* G);
     void fock_uhf(const double* Pa, const double* Pb, double* J, double* Ka, double* Kb);

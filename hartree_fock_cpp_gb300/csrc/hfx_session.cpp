@@ -361,6 +361,7 @@ void FockSession::combine_team(bool mixed_plan, Combined& c)
         c.team.groups.push_back(cg);
     }
     std::stable_sort(c.team.groups.begin(), c.team.groups.end(), [](const TeamGroup& a, const TeamGroup& b) { return a.cost > b.cost; });
+    c.team.make_specs(nsm_);
 }
 
 // One build of the live members switched on in active_ (J/K into acc_,
@@ -437,8 +438,6 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
     const int naux = (int)aux_.size();
     for (size_t gi = 0; gi < c.team.groups.size(); ++gi) {
         const TeamGroup& g = c.team.groups[gi];
-        KernelSpec ks;
-        cuda_check(team_spec(g, nsm_, &ks), "session team kernel");
         TeamArgs a{};
         a.pairs = super_.p;
         a.order = c.team.order.p;
@@ -463,7 +462,7 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
         a.nk = nk;
         a.slice = g.slice;
         void* prm[] = {&a};
-        sk.kernel((int)(gi % (c.groups.empty() ? naux + 1 : kFp64Lanes)), ks, prm);
+        sk.kernel((int)(gi % (c.groups.empty() ? naux + 1 : kFp64Lanes)), c.team.specs[gi], prm);
     }
     int next_aux = 0;
     for (size_t gi = 0; gi < c.groups.size(); ++gi) {

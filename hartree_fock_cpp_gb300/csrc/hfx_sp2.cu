@@ -30,8 +30,22 @@ constexpr double kTraceTol = 1e-6;  // tr(D) = nocc: otherwise no gap (fractiona
 
 // Gershgorin bounds of sym(F) = (F + F^T) / 2, one warp per row:
 // bounds[0] = min_i (f_ii - r_i), bounds[1] = max_i (f_ii + r_i).
-__global__ void __launch_bounds__(1024) k_sp2_bounds(int n, const double* __restrict__ F, double* __restrict__ bounds)
+// The projections of one run (blockIdx.y).
+struct Sp2Set {
+    const double* F;
+    double *X[2], *X2[2];
+    double *bounds, *traces, *D, *status;
+    int* state;
+    int nocc;
+};
+struct Sp2Sets {
+    Sp2Set s[2];
+};
+
+__global__ void __launch_bounds__(1024) k_sp2_bounds(int n, Sp2Sets sets)
 {
+    const double* __restrict__ F = sets.s[blockIdx.y].F;
+    double* bounds = sets.s[blockIdx.y].bounds;
     __shared__ double lo_w[32], hi_w[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     double lo = INFINITY, hi = -INFINITY;
@@ -107,11 +121,21 @@ __device__ __forceinline__ double sp2_form(int branch, int n, int r, int c, cons
     return 2.0 * Xp[e] - X2p[e];
 }
 
-__global__ void __launch_bounds__(kThreads) k_sp2_step(int n, int nt, int nocc, int j, const double* __restrict__ F,
-                                                        const double* __restrict__ bounds, const double* Xp,
-                                                        const double* X2p, double* Xo, double* X2o,
-                                                        double* __restrict__ traces, int* __restrict__ state)
+__global__ void __launch_bounds__(kThreads) k_sp2_step(int n, int nt, int j, Sp2Sets sets)
 {
+    const Sp2Set& set = sets.s[blockIdx.y];
+    const double* __restrict__ F = set.F;
+    const double* bounds = set.bounds;
+    const double *Xp = set.X[(j & 1) ^ 1], *X2p = set.X2[(j & 1) ^ 1];
+    double *Xo = set.X[j & 1], *X2o = set.X2[j & 1];
+    double* traces = set.traces;
+    int* state = set.state;
+    const int nocc = set.nocc;
+    // Programmatic dependent launch: the next step's blocks may be scheduled
+    // from here on and wait at their own dependency point, so that the ~45
+    // dependent launches of a projection do not each pay a launch gap.
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     extern __shared__ double sm[];
     const int ld = n + 1;  // odd row stride: the 8 rows of a panel fall in distinct banks
     double* A = sm;
@@ -185,13 +209,15 @@ __global__ void __launch_bounds__(kThreads) k_sp2_step(int n, int nt, int nocc, 
     }
 }
 
-__global__ void __launch_bounds__(256) k_sp2_finish(int n, int nt, int nocc, int steps, const double* __restrict__ traces,
-                                                     const int* __restrict__ state, const double* X0,
-                                                     const double* X1, double* __restrict__ D, double* status)
+__global__ void __launch_bounds__(256) k_sp2_finish(int n, int nt, int steps, Sp2Sets sets)
 {
+    const Sp2Set& set = sets.s[blockIdx.y];
+    const double* traces = set.traces;
+    const int nocc = set.nocc;
+    double* D = set.D;
     __shared__ int s_answer;
     if (threadIdx.x < 32) {
-        const Sp2Decision d = sp2_decide(steps, nt, nocc, traces, state);
+        const Sp2Decision d = sp2_decide(steps, nt, nocc, traces, set.state);
         int ans = d.answer;
         if (ans >= 0) {
             const double tr = warp_sum_fixed(traces + (size_t)ans * 2 * nt, nt);
@@ -201,9 +227,9 @@ __global__ void __launch_bounds__(256) k_sp2_finish(int n, int nt, int nocc, int
     }
     __syncthreads();
     const int ans = s_answer;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *status = ans >= 0 ? (double)(ans + 1) : 0.0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *set.status = ans >= 0 ? (double)(ans + 1) : 0.0;
     if (ans < 0) return;
-    const double* X = (ans & 1) ? X1 : X0;
+    const double* X = set.X[ans & 1];
     const size_t total = (size_t)n * n;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x)
         D[e] = X[e];
@@ -214,14 +240,6 @@ __global__ void __launch_bounds__(256) k_sp2_finish(int n, int nt, int nocc, int
 Sp2Projector::Sp2Projector(int n) : n_(n), nt_((n + kTile - 1) / kTile)
 {
     if (n < 1 || n > kMaxN) throw Error(HFX_ERR_INVALID, "SP2 projector: matrix dimension out of range");
-    const size_t nn = (size_t)n * n;
-    for (int p = 0; p < 2; ++p) {
-        X_[p].alloc(nn);
-        X2_[p].alloc(nn);
-    }
-    bounds_.alloc(2);
-    traces_.alloc((size_t)kMaxSteps * 2 * nt_);
-    state_.alloc((size_t)kMaxSteps * 2);
     smem_ = sizeof(double) * ((size_t)2 * kTile * (n + 1) + kThreads);
     // The limit is a property of the kernel, shared by every projector in the
     // process: always raise it to what the largest n needs, never to this n's
@@ -231,19 +249,47 @@ Sp2Projector::Sp2Projector(int n) : n_(n), nt_((n + kTile - 1) / kTile)
                "SP2 shared memory");
 }
 
-void Sp2Projector::run(const double* F, int nocc, double* D, double* status, cudaStream_t st, int max_steps)
+void Sp2Projector::run(const Task* tasks, int count, cudaStream_t st, int max_steps)
 {
-    if (nocc <= 0 || nocc >= n_) throw Error(HFX_ERR_INVALID, "SP2 projector: occupation out of range");
-    const int steps = std::max(1, std::min(max_steps, kMaxSteps));
-    k_sp2_bounds<<<1, 1024, 0, st>>>(n_, F, bounds_.p);
-    const int blocks = nt_ * (nt_ + 1) / 2;
-    for (int j = 0; j < steps; ++j) {
-        const int cur = j & 1, prev = cur ^ 1;
-        k_sp2_step<<<blocks, kThreads, smem_, st>>>(n_, nt_, nocc, j, F, bounds_.p, X_[prev].p, X2_[prev].p,
-                                                     X_[cur].p, X2_[cur].p, traces_.p, state_.p);
+    if (count < 1 || count > 2) throw Error(HFX_ERR_INVALID, "SP2 projector: one or two projections");
+    const size_t nn = (size_t)n_ * n_;
+    Sp2Sets sets{};
+    for (int t = 0; t < count; ++t) {
+        if (tasks[t].nocc <= 0 || tasks[t].nocc >= n_) throw Error(HFX_ERR_INVALID, "SP2 projector: occupation out of range");
+        Sp2Set& s = sets.s[t];
+        for (int p = 0; p < 2; ++p) {
+            X_[t][p].alloc(nn);
+            X2_[t][p].alloc(nn);
+            s.X[p] = X_[t][p].p;
+            s.X2[p] = X2_[t][p].p;
+        }
+        bounds_[t].alloc(2);
+        traces_[t].alloc((size_t)kMaxSteps * 2 * nt_);
+        state_[t].alloc((size_t)kMaxSteps * 2);
+        s.F = tasks[t].F;
+        s.nocc = tasks[t].nocc;
+        s.D = tasks[t].D;
+        s.status = tasks[t].status;
+        s.bounds = bounds_[t].p;
+        s.traces = traces_[t].p;
+        s.state = state_[t].p;
     }
-    const int grid = (int)std::min<size_t>(1024, ((size_t)n_ * n_ + 255) / 256);
-    k_sp2_finish<<<grid, 256, 0, st>>>(n_, nt_, nocc, steps, traces_.p, state_.p, X_[0].p, X_[1].p, D, status);
+    const int steps = std::max(1, std::min(max_steps, kMaxSteps));
+    k_sp2_bounds<<<dim3(1, count), 1024, 0, st>>>(n_, sets);
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(nt_ * (nt_ + 1) / 2), (unsigned)count);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem_;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    for (int j = 0; j < steps; ++j)
+        cuda_check(cudaLaunchKernelEx(&cfg, k_sp2_step, n_, nt_, j, sets), "SP2 step");
+    const int grid = (int)std::min<size_t>(1024, (nn + 255) / 256);
+    k_sp2_finish<<<dim3(grid, count), 256, 0, st>>>(n_, nt_, steps, sets);
     cuda_check(cudaGetLastError(), "SP2 projector");
 }
 

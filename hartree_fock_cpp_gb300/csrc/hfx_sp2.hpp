@@ -31,19 +31,33 @@ public:
     // 600, 35 vs 26 ms at 800; about 44 steps each).
     static constexpr int kScfMaxN = 640;
 
+    // One projection: D <- projector (n x n); *status (device double) <- number
+    // of steps when converged with tr(D) = nocc within the step limit, else 0
+    // (no gap, or too few steps: the caller falls back to an eigensolve).  F
+    // is not modified.  Requires 0 < nocc < n.
+    struct Task {
+        const double* F;
+        int nocc;
+        double* D;
+        double* status;
+    };
+
     explicit Sp2Projector(int n);
-    // D <- projector (n x n); *status (device double) <- number of steps when
-    // converged with tr(D) = nocc within max_steps (<= kMaxSteps), else 0 (no
-    // gap, or too few steps: the caller falls back to an eigensolve).  F is not
-    // modified.  Requires 0 < nocc < n.  Steps after convergence cost one
-    // launch each; callers that iterate pass the last count plus a margin.
-    void run(const double* F, int nocc, double* D, double* status, cudaStream_t st, int max_steps = kMaxSteps);
+    // `count` (1 or 2: the spins of an iteration) projections in the same
+    // launches, within max_steps (<= kMaxSteps).  Steps after convergence cost
+    // one launch each; callers that iterate pass the last count plus a margin.
+    void run(const Task* tasks, int count, cudaStream_t st, int max_steps = kMaxSteps);
+    void run(const double* F, int nocc, double* D, double* status, cudaStream_t st, int max_steps = kMaxSteps)
+    {
+        const Task t{F, nocc, D, status};
+        run(&t, 1, st, max_steps);
+    }
 
 private:
     int n_, nt_;
     size_t smem_;
-    DevBuf<double> X_[2], X2_[2], bounds_, traces_;
-    DevBuf<int> state_;
+    DevBuf<double> X_[2][2], X2_[2][2], bounds_[2], traces_[2];   // [projection][step parity]
+    DevBuf<int> state_[2];
 };
 
 }  // namespace hfx
