@@ -395,10 +395,10 @@ const ClassTables& class_tables()
 
 // Indices handed out one at a time; the first exception is rethrown after
 // every thread has joined.
-void host_parallel_for(int n, const std::function<void(int)>& f)
+void host_parallel_for(int n, const std::function<void(int)>& f, int most)
 {
     const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
-    const int nt = std::min(std::min(n, hw), 16);
+    const int nt = std::min(std::min(n, hw), std::min(most, 16));
     if (nt <= 1) {
         for (int i = 0; i < n; ++i) f(i);
         return;

@@ -146,8 +146,8 @@ PairData build_pair_data(const Basis& b, const Fragments& fr);
 // coefficient are left out (build_pair_data, build_super_data).
 constexpr double kPrimPairCut = 1e-18;
 
-// f(i) for i in [0, n) on up to 16 host threads.
-void host_parallel_for(int n, const std::function<void(int)>& f);
+// f(i) for i in [0, n) on up to `most` (and 16) host threads.
+void host_parallel_for(int n, const std::function<void(int)>& f, int most = 16);
 // Indices by decreasing cost (counting sort on 1/16-octave bins, stable); with
 // `shape`, equal bins are ordered by shape.
 std::vector<size_t> order_by_cost_desc(const std::vector<double>& cost,

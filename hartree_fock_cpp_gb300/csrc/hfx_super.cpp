@@ -627,6 +627,8 @@ TeamPlanHost build_team_plan(const SuperData& sd, const std::vector<double>& q, 
                 };
                 units.push_back(whole(v) < whole(u) ? v : u);
             }
+    // starting a thread costs 20-30 us: small molecules are planned on this one
+    const int threads = np < 128 ? 1 : np < 256 ? 4 : 16;
     host_parallel_for((int)units.size(), [&](int i) {
         Unit& u = units[i];
         double cp, cr, cq;
@@ -636,7 +638,7 @@ TeamPlanHost build_team_plan(const SuperData& sd, const std::vector<double>& q, 
             for (int s = 0; s < m; ++s) rows += sd.pairs[plan.order[b0 + s]].npp;
             u.total += rows * sd.pairs[ket].npp * cp + rows * cr + m * cq;
         });
-    });
+    }, threads);
     double total = 0.0;
     for (const Unit& u : units) total += u.total;
     // about 24 tasks for each of eight warps per SM, none below 40000
@@ -733,7 +735,7 @@ TeamPlanHost build_team_plan(const SuperData& sd, const std::vector<double>& q, 
                 s += n;
             }
         });
-    });
+    }, threads);
     group_tasks(plan, units, [&](const Unit& u) { return cL[u.cb] + cL[u.ck]; });
     return plan;
 }
