@@ -582,6 +582,10 @@ __global__ void __launch_bounds__(128) k_small(SmallArgs<T> a)
     constexpr int NCB = small_ncb<T, LA, LB, LC, LD>();
     const int task = blockIdx.x * blockDim.x + threadIdx.x;
     if (task >= a.ntasks) return;
+    const long long copy = (long long)(blockIdx.x & (a.ncopy - 1)) * a.cstride;
+    a.J += copy;
+    a.Kx += copy;
+    if constexpr (NK == 2) a.Kx2 += copy;
     const Task tk = a.tasks[task];
     const DPair bra = a.pairs[tk.bra];
     const DPair ket = a.pairs[tk.ket];

@@ -169,6 +169,10 @@ struct SmallArgs {
     // FP32 kernels: float copy of the BF-pair Schwarz bounds (the digestion's
     // screen then needs no FP64 arithmetic); addressed with bra.qoff
     const float* Qbf32;
+    // copies of the accumulators: a CTA adds to copy blockIdx.x % ncopy, copy
+    // c at c * cstride elements
+    int ncopy;
+    long long cstride;
 };
 
 // Arguments of the warp-per-shell-quartet kernel.
@@ -207,6 +211,10 @@ struct WarpArgs {
     // FP32 kernels: float copy of the BF-pair Schwarz bounds (the digestion's
     // screen then needs no FP64 arithmetic); addressed with bra.qoff
     const float* Qbf32;
+    // copies of the accumulators: a CTA adds to copy blockIdx.x % ncopy, copy
+    // c at c * cstride elements
+    int ncopy;
+    long long cstride;
 };
 
 #ifdef __CUDACC__

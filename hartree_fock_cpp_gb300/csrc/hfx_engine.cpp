@@ -1250,8 +1250,17 @@ cudaGraphExec_t GraphSink::instantiate()
     return exec;
 }
 
+int Job::acc_copies(bool mixed_plan) const
+{
+    return plan(mixed_plan).groups.empty() ? 1 : kAccCopies;
+}
+long long Job::acc_stride(bool mixed_plan) const
+{
+    return acc_copies(mixed_plan) > 1 ? (nmat() + 31) & ~31LL : nmat();
+}
+
 void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, const double* Dk2, double* J, double* Kx,
-                    double* Kx2, int* counters, bool mixed_plan, double dthr)
+                    double* Kx2, int* counters, bool mixed_plan, double dthr, int ncopy, long long cstride)
 {
     const GroupSet& gs = plan(mixed_plan);
     const std::vector<LaunchGroup>& groups = gs.groups;
@@ -1338,7 +1347,7 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
             const int lane = naux - next_aux;
             next_aux = (next_aux + 1) % (naux + 1 - kFp64Lanes);
             SmallArgs<float> a{d_pairs_.p, d_rec32_.p, tasks + g.off, (int)g.n, d_boys32_.p, opt_.screening_threshold,
-                               d_qbf_.p, K, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, d_qbf32_.p};
+                               d_qbf_.p, K, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, d_qbf32_.p, ncopy, cstride};
             cuda_check(small_spec_f32(g.pcb, g.pck, nk, (int)g.n, &ks), "small-class kernel");
             void* prm[] = {&a};
             sk.kernel(lane, ks, prm);
@@ -1347,7 +1356,7 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
             WarpArgs<float> a{d_pairs_.p, d_rec32_.p, d_pct_.p, d_abs_.p, d_kh_.p, d_kl_.p, tasks + g.off, (int)g.n,
                               ctr + gi, d_boys32_.p, opt_.screening_threshold, d_qbf_.p, K, Dj, Dk, Dk2, J, Kx, Kx2,
                               g.slice, g.lane_min_npp, Dsh, dthr, nullptr, nullptr, active, Dj32, Dk32, Dk232,
-                              d_qbf32_.p};
+                              d_qbf32_.p, ncopy, cstride};
             void* prm[] = {&a};
             sk.kernel(naux, ks, prm);
         }
@@ -1416,51 +1425,65 @@ int Job::max_fragment_K() const
     return m;
 }
 
-void Job::enqueue_finish_rhf(OpSink& sk, const double* Jacc, const double* Kacc, double* dG)
+void Job::enqueue_finish_rhf(OpSink& sk, const double* Jacc, const double* Kacc, double* dG, int ncopy, long long cstride)
 {
     const int* fk = d_fk_.p;
     const long long* fm = d_fmoff_.p;
     const unsigned char* act = d_active_.p;
-    void* prm[] = {&Jacc, &Kacc, &dG, &fk, &fm, &act};
+    void* prm[] = {&Jacc, &Kacc, &dG, &fk, &fm, &act, &ncopy, &cstride};
     sk.kernel(0, finish_rhf_spec(max_fragment_K(), frags_.count()), prm);
 }
 
 void Job::enqueue_rhf(OpSink& sk, const double* dP, double* dG, bool mixed_plan, double dthr)
 {
-    const size_t n = (size_t)nmat();
-    sk.zero(0, d_J_.p, n * sizeof(double));
-    sk.zero(0, d_K_.p, n * sizeof(double));
-    launch_jk(sk, 1, dP, dP, nullptr, d_J_.p, d_K_.p, nullptr, nullptr, mixed_plan, dthr);
-    enqueue_finish_rhf(sk, d_J_.p, d_K_.p, dG);
+    const int ncopy = acc_copies(mixed_plan);
+    const long long cstride = acc_stride(mixed_plan);
+    sk.zero(0, d_J_.p, (size_t)(ncopy * cstride) * sizeof(double));
+    sk.zero(0, d_K_.p, (size_t)(ncopy * cstride) * sizeof(double));
+    launch_jk(sk, 1, dP, dP, nullptr, d_J_.p, d_K_.p, nullptr, nullptr, mixed_plan, dthr, ncopy, cstride);
+    enqueue_finish_rhf(sk, d_J_.p, d_K_.p, dG, ncopy, cstride);
 }
 
 void Job::enqueue_uhf(OpSink& sk, const double* dPa, const double* dPb, double* dJ, double* dKa, double* dKb,
                       bool mixed_plan, double dthr)
 {
     long long n = nmat();
-    sk.zero(0, d_J_.p, (size_t)n * sizeof(double));
-    sk.zero(0, d_K_.p, (size_t)n * sizeof(double));
-    sk.zero(0, d_K2_.p, (size_t)n * sizeof(double));
+    int ncopy = acc_copies(mixed_plan);
+    long long cstride = acc_stride(mixed_plan);
+    for (double* p : {d_J_.p, d_K_.p, d_K2_.p}) sk.zero(0, p, (size_t)(ncopy * cstride) * sizeof(double));
     double* dj = d_Dj_.p;
     void* pa[] = {&dPa, &dPb, &dj, &n};
     sk.kernel(0, add_spec(n), pa);
-    launch_jk(sk, 2, d_Dj_.p, dPa, dPb, d_J_.p, d_K_.p, d_K2_.p, nullptr, mixed_plan, dthr);
+    launch_jk(sk, 2, d_Dj_.p, dPa, dPb, d_J_.p, d_K_.p, d_K2_.p, nullptr, mixed_plan, dthr, ncopy,
+              cstride);
     const double* jp = d_J_.p;
     const double* kp = d_K_.p;
     const double* k2 = d_K2_.p;
     const int* fk = d_fk_.p;
     const long long* fm = d_fmoff_.p;
     const unsigned char* act = d_active_.p;
-    void* prm[] = {&jp, &kp, &k2, &dJ, &dKa, &dKb, &fk, &fm, &act};
+    void* prm[] = {&jp, &kp, &k2, &dJ, &dKa, &dKb, &fk, &fm, &act, &ncopy, &cstride};
     sk.kernel(0, finish_uhf_spec(max_fragment_K(), frags_.count()), prm);
+}
+
+// Accumulators for a build with nk exchange matrices: grown, never shrunk
+// (the graphs of other variants hold their addresses; growing drops them).
+void Job::alloc_acc(int nk, bool mixed_plan)
+{
+    const size_t n = (size_t)(acc_copies(mixed_plan) * acc_stride(mixed_plan));
+    DevBuf<double>* b[3] = {&d_J_, &d_K_, &d_K2_};
+    for (int s = 0; s < nk + 1; ++s)
+        if (b[s]->n < n) {
+            clear_graphs();
+            b[s]->alloc(n);
+        }
 }
 
 void Job::fock_rhf_device_ex(const double* dP, double* dG, bool mixed_plan, double dthr)
 {
     cuda_check(cudaSetDevice(device_), "cudaSetDevice");
     const size_t n = (size_t)nmat();
-    d_J_.alloc(n);
-    d_K_.alloc(n);
+    alloc_acc(1, mixed_plan);
     cudaGraphExec_t ge = graph_for(1, mixed_plan, dthr);
     cuda_check(cudaEventRecord(ev0_, stream_), "event");
     if (ge) {
@@ -1615,9 +1638,7 @@ void Job::fock_uhf_device_ex(const double* dPa, const double* dPb, double* dJ, d
 {
     cuda_check(cudaSetDevice(device_), "cudaSetDevice");
     const size_t n = (size_t)nmat();
-    d_J_.alloc(n);
-    d_K_.alloc(n);
-    d_K2_.alloc(n);
+    alloc_acc(2, mixed_plan);
     d_Dj_.alloc(n);
     cudaGraphExec_t ge = graph_for(2, mixed_plan, dthr);
     cuda_check(cudaEventRecord(ev0_, stream_), "event");

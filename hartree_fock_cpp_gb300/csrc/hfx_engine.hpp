@@ -183,6 +183,14 @@ struct GroupSet {
 // against 11 + 8, ms: water/cc-pVTZ 1.14 / 0.92, NaCl/cc-pVTZ 3.73 / 3.4,
 // benzene/cc-pVDZ 8.10 / 7.84, n-decane/6-31G* mixed 3.20 / 3.02.
 constexpr int kAuxLanes = 11, kFp64Lanes = 8;
+// Copies of the J/K accumulators of a build with FP32 launches (a power of
+// two; CTAs spread over them, the symmetrisation adds them up): the FP32
+// kernels send 600 M FP64 reductions to the L2 for a K = 292 molecule, its
+// busiest slices 50-70% occupied and the average one 30%. 1 / 2 / 4 / 8
+// copies, ms: n-decane/6-31G* mixed 3.07 / 2.94 / 2.89 / 2.89, K = 292 tree
+// 18.0 / 17.6 / 17.5 / 17.4. FP64 builds reduce in the kernel first (1-4%) and
+// keep one.
+constexpr int kAccCopies = 4;
 
 // Destination of a Fock build's device work.  Lane 0 is the job's main
 // stream, lanes 1..n its auxiliary streams; fork() makes every auxiliary lane
@@ -332,12 +340,16 @@ private:
     void count_quartets(GroupSet& gs) const;
     void build_fp32_groups(GroupSet& gs);
     void launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, const double* Dk2, double* J, double* Kx,
-                   double* Kx2, int* counters = nullptr, bool mixed_plan = false, double dthr = 0.0);
+                   double* Kx2, int* counters = nullptr, bool mixed_plan = false, double dthr = 0.0, int ncopy = 1,
+                   long long cstride = 0);
+    int acc_copies(bool mixed_plan) const;
+    long long acc_stride(bool mixed_plan) const;
+    void alloc_acc(int nk, bool mixed_plan);
     const GroupSet& plan(bool mixed_plan) const { return mixed_plan && mixed() ? gs_mixed_ : gs_fp64_; }
     void record_stats_plan(int launches, const GroupSet& gs);
     StreamSink stream_sink() { return StreamSink(stream_, aux_, fork_ev_, aux_ev_); }
     int max_fragment_K() const;
-    void enqueue_finish_rhf(OpSink& sk, const double* Jacc, const double* Kacc, double* dG);
+    void enqueue_finish_rhf(OpSink& sk, const double* Jacc, const double* Kacc, double* dG, int ncopy = 1, long long cstride = 0);
     void enqueue_rhf(OpSink& sk, const double* dP, double* dG, bool mixed_plan, double dthr);
     void enqueue_uhf(OpSink& sk, const double* dPa, const double* dPb, double* dJ, double* dKa, double* dKb, bool mixed_plan,
                      double dthr);

@@ -9,11 +9,19 @@
 
 namespace hfx {
 
+// sum of an accumulator element over its copies
+__device__ __forceinline__ double copies(const double* A, long long e, int ncopy, long long cstride)
+{
+    double v = A[e];
+    for (int c = 1; c < ncopy; ++c) v += A[c * cstride + e];
+    return v;
+}
+
 // G = (Jacc + Jacc^T)/4 - 1/2 (Kacc + Kacc^T)/8   (RHF, linalg.hpp:100-129),
 // per molecule block of the packed buffers (blockIdx.y = molecule); blocks of
 // molecules switched off for this build (active[f] == 0) are left untouched
 __global__ void k_finish_rhf(const double* Jacc, const double* Kacc, double* G, const int* fk, const long long* fmoff,
-                             const unsigned char* active)
+                             const unsigned char* active, int ncopy, long long cstride)
 {
     if (active && !active[blockIdx.y]) return;
     const int K = fk[blockIdx.y];
@@ -21,15 +29,16 @@ __global__ void k_finish_rhf(const double* Jacc, const double* Kacc, double* G, 
     const int n = K * K;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         int i = e / K, j = e - i * K;
-        double J = 0.25 * (Jacc[o + e] + Jacc[o + j * K + i]);
-        double X = 0.125 * (Kacc[o + e] + Kacc[o + j * K + i]);
+        double J = 0.25 * (copies(Jacc, o + e, ncopy, cstride) + copies(Jacc, o + j * K + i, ncopy, cstride));
+        double X = 0.125 * (copies(Kacc, o + e, ncopy, cstride) + copies(Kacc, o + j * K + i, ncopy, cstride));
         G[o + e] = J - 0.5 * X;
     }
 }
 
 // J = (Jacc + Jacc^T)/4, K = (Kacc + Kacc^T)/8  (UHF, linalg.hpp:215-296)
 __global__ void k_finish_uhf(const double* Jacc, const double* Ka, const double* Kb, double* J, double* Kao,
-                             double* Kbo, const int* fk, const long long* fmoff, const unsigned char* active)
+                             double* Kbo, const int* fk, const long long* fmoff, const unsigned char* active, int ncopy,
+                             long long cstride)
 {
     if (active && !active[blockIdx.y]) return;
     const int K = fk[blockIdx.y];
@@ -37,9 +46,9 @@ __global__ void k_finish_uhf(const double* Jacc, const double* Ka, const double*
     const int n = K * K;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         int i = e / K, j = e - i * K;
-        J[o + e] = 0.25 * (Jacc[o + e] + Jacc[o + j * K + i]);
-        Kao[o + e] = 0.125 * (Ka[o + e] + Ka[o + j * K + i]);
-        Kbo[o + e] = 0.125 * (Kb[o + e] + Kb[o + j * K + i]);
+        J[o + e] = 0.25 * (copies(Jacc, o + e, ncopy, cstride) + copies(Jacc, o + j * K + i, ncopy, cstride));
+        Kao[o + e] = 0.125 * (copies(Ka, o + e, ncopy, cstride) + copies(Ka, o + j * K + i, ncopy, cstride));
+        Kbo[o + e] = 0.125 * (copies(Kb, o + e, ncopy, cstride) + copies(Kb, o + j * K + i, ncopy, cstride));
     }
 }
 

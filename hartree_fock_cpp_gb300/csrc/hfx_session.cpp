@@ -472,7 +472,7 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
             const int lane = naux - next_aux;
             next_aux = (next_aux + 1) % (naux + 1 - kFp64Lanes);
             SmallArgs<float> a{pairs32_.p, anchor32_.p, tasks + g.off, (int)g.n, boys32_.p, thr_, nullptr,
-                               0, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p};
+                               0, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p, 1, 0};
             cuda_check(small_spec_f32(g.pcb, g.pck, nk, (int)g.n, &ks), "session small-class kernel");
             void* prm[] = {&a};
             sk.kernel(lane, ks, prm);
@@ -480,7 +480,7 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
             cuda_check(warp_spec(true, nk, g.grid, g.warps_per_cta, g.slice, &ks), "session warp kernel");
             WarpArgs<float> a{pairs32_.p, anchor32_.p, pct_.p, abs_.p, kh_.p, kl_.p, tasks + g.off, (int)g.n,
                               ctr + gi, boys32_.p, thr_, nullptr, 0, Dj, Dk, Dk2, J, Kx, Kx2, g.slice,
-                              g.lane_min_npp, Dsh, dthr, nullptr, nullptr, active, Dj32, Dk32, Dk232, anchor32_.p};
+                              g.lane_min_npp, Dsh, dthr, nullptr, nullptr, active, Dj32, Dk32, Dk232, anchor32_.p, 1, 0};
             void* prm[] = {&a};
             sk.kernel(naux, ks, prm);
         }
@@ -491,11 +491,13 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
     const int* fk = fk_.p;
     const long long* fm = fmoff_.p;
     const int nf = (int)live_.size();
+    int ncopy = 1;
+    long long cstride = 0;
     if (nk == 1) {
         const double* jp = acc_[0].p;
         const double* kp = acc_[1].p;
         double* G = out_[0].p;
-        void* prm[] = {&jp, &kp, &G, &fk, &fm, &active};
+        void* prm[] = {&jp, &kp, &G, &fk, &fm, &active, &ncopy, &cstride};
         sk.kernel(0, finish_rhf_spec(kmax, nf), prm);
     } else {
         const double* jp = acc_[0].p;
@@ -504,7 +506,7 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
         double* o0 = out_[0].p;
         double* o1 = out_[1].p;
         double* o2 = out_[2].p;
-        void* prm[] = {&jp, &kp, &k2, &o0, &o1, &o2, &fk, &fm, &active};
+        void* prm[] = {&jp, &kp, &k2, &o0, &o1, &o2, &fk, &fm, &active, &ncopy, &cstride};
         sk.kernel(0, finish_uhf_spec(kmax, nf), prm);
     }
 }

@@ -240,6 +240,12 @@ __global__ void __launch_bounds__(256) k_warp_quartet(WarpArgs<T> a)
     }
     __syncthreads();
 
+    if (a.ncopy > 1) {
+        const long long copy = (long long)(blockIdx.x & (a.ncopy - 1)) * a.cstride;
+        a.J += copy;
+        a.Kx += copy;
+        if constexpr (NK == 2) a.Kx2 += copy;
+    }
     const T* __restrict__ rec = a.rec;
     while (true) {
         int tk = 0;
