@@ -1,16 +1,13 @@
-// hfx_class.cuh -- thread-per-shell-quartet kernels for the small
-// angular-momentum classes (at most 36 Cartesian integrals per shell quartet
-// and total L <= 4: (ss|ss) (ps|ss) (ps|ps) (pp|ss) (pp|ps) (ds|ss) (ds|ps)
-// (ds|ds) (dp|ss)), instantiated for T = double and T = float.
+// hfx_class.cuh -- thread-per-task kernels for the FP32 quartets of the 19
+// classes up to (dd|ds) with at most d functions, and the register-resident
+// Hermite recursion that the team kernel uses too.
 //
-// These classes carry most of the primitive quartets of contracted basis sets
-// (cc-pVDZ carbon s shells have 9 primitives, so one (ss|ss) shell quartet is
-// up to 6561 primitive quartets).  One thread owns one shell quartet and loops
-// over all of its primitive quartets with every index, loop bound and
-// sparsity pattern fixed at compile time: the Boys seeds, the R_{tuv} table,
-// the ket-transformed W and the Cartesian accumulators stay in registers; no
-// shared memory, no barriers.  The quartet list of a class is sorted by
-// primitive count, so a warp's 32 lanes run loops of equal length.
+// One thread owns a tile of one shell quartet's primitive quartets with every
+// index, loop bound and sparsity pattern fixed at compile time: the Boys
+// seeds, the R_{tuv} table, the ket-transformed W and the Cartesian
+// accumulators stay in registers; no shared memory, no barriers.  The tasks
+// of a class are sorted by cost and shape, so a warp's 32 lanes run loops of
+// equal length.
 //
 // Per primitive quartet (the reference's primitive_repulsion,
 // integrals.hpp:624-699, evaluated once per shell quartet here):
@@ -130,78 +127,39 @@ __host__ __device__ constexpr int rec_stride(int la, int lb) { return (5 + n_coe
 template <typename T, int L>
 __device__ __forceinline__ void boys_all(T Tv, const T* __restrict__ tab, T (&F)[L + 1])
 {
-    if constexpr (sizeof(T) == 4) {
-        // FP32: both forms, then a select per order (no divergence inside a
-        // warp whose lanes straddle T = 36): the table row of (L, k) as two
-        // 16-byte loads, Taylor + downward recursion; and the asymptotic
-        // F_0 = sqrt(pi/T)/2 with upward recursion (exp(-T) < 3e-16 there)
-        const bool in_table = Tv < (T)kBoysTMax;
-        int k;
-        const T nd = boys_grid_offset(in_table ? Tv : (T)0, k);
-        const float4* row = reinterpret_cast<const float4*>(tab + ((size_t)L * kBoysN + k) * kBoys32Row);
-        const float4 c0 = __ldg(row), c1 = __ldg(row + 1);
-        T Ft[L + 1];
-        T r = c1.x;                       // F_{L+4}/24
-        r = fma(r, nd, c0.w);             // F_{L+3}/6
-        r = fma(r, nd, c0.z);             // F_{L+2}/2
-        r = fma(r, nd, c0.y);             // F_{L+1}
-        Ft[L] = fma(r, nd, c0.x);
-        if constexpr (L > 0) {
-            T x = (T)(1.0 / 24.0);
-            x = fma(x, nd, (T)(1.0 / 6.0));
-            x = fma(x, nd, (T)0.5);
-            x = fma(x, nd, (T)1);
-            x = fma(x, nd, (T)1);
-            const T e = c1.y * x;
-            const T t2 = Tv + Tv;
+    // FP32: both forms, then a select per order (no divergence inside a
+    // warp whose lanes straddle T = 36): the table row of (L, k) as two
+    // 16-byte loads, Taylor + downward recursion; and the asymptotic
+    // F_0 = sqrt(pi/T)/2 with upward recursion (exp(-T) < 3e-16 there)
+    const bool in_table = Tv < (T)kBoysTMax;
+    int k;
+    const T nd = boys_grid_offset(in_table ? Tv : (T)0, k);
+    const float4* row = reinterpret_cast<const float4*>(tab + ((size_t)L * kBoysN + k) * kBoys32Row);
+    const float4 c0 = __ldg(row), c1 = __ldg(row + 1);
+    T Ft[L + 1];
+    T r = c1.x;                       // F_{L+4}/24
+    r = fma(r, nd, c0.w);             // F_{L+3}/6
+    r = fma(r, nd, c0.z);             // F_{L+2}/2
+    r = fma(r, nd, c0.y);             // F_{L+1}
+    Ft[L] = fma(r, nd, c0.x);
+    if constexpr (L > 0) {
+        T x = (T)(1.0 / 24.0);
+        x = fma(x, nd, (T)(1.0 / 6.0));
+        x = fma(x, nd, (T)0.5);
+        x = fma(x, nd, (T)1);
+        x = fma(x, nd, (T)1);
+        const T e = c1.y * x;
+        const T t2 = Tv + Tv;
 #pragma unroll
-            for (int m = L - 1; m >= 0; --m) Ft[m] = fma(t2, Ft[m + 1], e) * ((T)1 / (T)(2 * m + 1));
-        }
-        const T rs = rsqrt(fmax(Tv, (T)1e-30));
-        T Fa = (T)0.88622692545275801365 * rs;
-        const T inv2T = (T)0.5 * rs * rs;
+        for (int m = L - 1; m >= 0; --m) Ft[m] = fma(t2, Ft[m + 1], e) * ((T)1 / (T)(2 * m + 1));
+    }
+    const T rs = rsqrt(fmax(Tv, (T)1e-30));
+    T Fa = (T)0.88622692545275801365 * rs;
+    const T inv2T = (T)0.5 * rs * rs;
 #pragma unroll
-        for (int m = 0; m <= L; ++m) {
-            F[m] = in_table ? Ft[m] : Fa;
-            Fa = (T)(2 * m + 1) * Fa * inv2T;
-        }
-    } else {
-        if (Tv < (T)kBoysTMax) {
-            // the (L, k) row: F_{L+j}(T_k) / j!, j = 0..6, then exp(-T_k)
-            const int k = (int)(Tv * (T)kBoysInvStep + (T)0.5);
-            const T nd = (T)k * ((T)1 / (T)kBoysInvStep) - Tv;
-            const double2* row = reinterpret_cast<const double2*>(tab + ((size_t)L * kBoysN + k) * kBoys64Row);
-            const double2 c0 = __ldg(row), c1 = __ldg(row + 1), c2 = __ldg(row + 2), c3 = __ldg(row + 3);
-            T r = c3.x;
-            r = fma(r, nd, c2.y);
-            r = fma(r, nd, c2.x);
-            r = fma(r, nd, c1.y);
-            r = fma(r, nd, c1.x);
-            r = fma(r, nd, c0.y);
-            F[L] = fma(r, nd, c0.x);
-            if constexpr (L > 0) {
-                T x = (T)(1.0 / 5040.0);
-                x = fma(x, nd, (T)(1.0 / 720.0));
-                x = fma(x, nd, (T)(1.0 / 120.0));
-                x = fma(x, nd, (T)(1.0 / 24.0));
-                x = fma(x, nd, (T)(1.0 / 6.0));
-                x = fma(x, nd, (T)0.5);
-                x = fma(x, nd, (T)1);
-                x = fma(x, nd, (T)1);
-                const T e = c3.y * x;
-                const T t2 = Tv + Tv;
-    #pragma unroll
-                for (int m = L - 1; m >= 0; --m) F[m] = fma(t2, F[m + 1], e) * ((T)1 / (T)(2 * m + 1));
-            }
-        } else {
-            const T rs = rsqrt(Tv);
-            F[0] = (T)0.88622692545275801365 * rs;
-            if constexpr (L > 0) {
-                const T inv2T = (T)0.5 * rs * rs;
-    #pragma unroll
-                for (int m = 0; m < L; ++m) F[m + 1] = (T)(2 * m + 1) * F[m] * inv2T;
-            }
-        }
+    for (int m = 0; m <= L; ++m) {
+        F[m] = in_table ? Ft[m] : Fa;
+        Fa = (T)(2 * m + 1) * Fa * inv2T;
     }
 }
 
@@ -243,18 +201,11 @@ __device__ __forceinline__ void hermite_R(T X, T Y, T Z, const T (&s)[L + 1], T 
 template <typename T>
 __device__ __forceinline__ void load_header(const T* r, T& p, T& x, T& y, T& z)
 {
-    if constexpr (sizeof(T) == 4) {
-        const float4 h = __ldg(reinterpret_cast<const float4*>(r));
-        p = h.x;
-        x = h.y;
-        y = h.z;
-        z = h.w;
-    } else {
-        p = __ldg(r);
-        x = __ldg(r + 1);
-        y = __ldg(r + 2);
-        z = __ldg(r + 3);
-    }
+    const float4 h = __ldg(reinterpret_cast<const float4*>(r));
+    p = h.x;
+    x = h.y;
+    y = h.z;
+    z = h.w;
 }
 
 __device__ __forceinline__ long long spidx(int a, int b)
@@ -421,141 +372,107 @@ __device__ __forceinline__ void small_quartet(const SmallArgs<T>& a, const Task&
     double* Kx = a.Kx + bra.moff;
     double* Kx2 = a.Kx2 + (NK == 2 ? bra.moff : 0);
     const bool same_pair = (tk.bra == tk.ket);
-    if constexpr (sizeof(T) == 8 && !kBlockDigestFP64) {
+    // Block digestion: the degeneracy weight is applied in place (0 for
+    // the non-canonical and BF-screened elements); then every J / K
+    // element the quartet touches is summed over the quartet in registers
+    // (FP32 quartets: float products with the float density copies) and
+    // added to the FP64 accumulators once -- nab + ncd + na nc + na nd +
+    // nb nc + nb nd atomics per quartet instead of 6 per integral.
+    constexpr int NA = c_nc(LA), NC = c_nc(LC);
+    const T* __restrict__ QbT = a.Qbf32 + bra.qoff;
+    const bool screen = a.thr >= 0.0;
+    const T thrT = (T)a.thr;
 #pragma unroll
-        for (int ab = 0; ab < NAB; ++ab) {
-            const int ia = ab / NB, ib = ab % NB;
-            const int i = bra.bf0 + ia, j = bra.bf1 + ib;
-            const long long pij = spidx(i, j);
-            const double qb = __ldg(Qbf + pij);
-            if (bra.same && ia < ib) continue;
-#pragma unroll
-            for (int cd = 0; cd < NCD; ++cd) {
-                const int ic = (C0 + cd) / ND, id = (C0 + cd) % ND;
-                const int k = ket.bf0 + ic, l = ket.bf1 + id;
-                if (ket.same && ic < id) continue;
-                const long long pkl = spidx(k, l);
-                if (same_pair && pij < pkl) continue;
-                if (a.thr >= 0.0 && qb * __ldg(Qbf + pkl) < a.thr) continue;
-                const double v =
-                    (double)acc[ab][cd] * ((i == j ? 1.0 : 2.0) * (k == l ? 1.0 : 2.0) * (pij == pkl ? 1.0 : 2.0));
-                atomicAdd(J + (long long)i * K + j, __ldg(Dj + (long long)k * K + l) * v);
-                atomicAdd(J + (long long)k * K + l, __ldg(Dj + (long long)i * K + j) * v);
-                atomicAdd(Kx + (long long)i * K + k, __ldg(Dk + (long long)j * K + l) * v);
-                atomicAdd(Kx + (long long)j * K + l, __ldg(Dk + (long long)i * K + k) * v);
-                atomicAdd(Kx + (long long)i * K + l, __ldg(Dk + (long long)j * K + k) * v);
-                atomicAdd(Kx + (long long)j * K + k, __ldg(Dk + (long long)i * K + l) * v);
-                if constexpr (NK == 2) {
-                    atomicAdd(Kx2 + (long long)i * K + k, __ldg(Dk2 + (long long)j * K + l) * v);
-                    atomicAdd(Kx2 + (long long)j * K + l, __ldg(Dk2 + (long long)i * K + k) * v);
-                    atomicAdd(Kx2 + (long long)i * K + l, __ldg(Dk2 + (long long)j * K + k) * v);
-                    atomicAdd(Kx2 + (long long)j * K + k, __ldg(Dk2 + (long long)i * K + l) * v);
-                }
-            }
-        }
-    } else {
-        // Block digestion: the degeneracy weight is applied in place (0 for
-        // the non-canonical and BF-screened elements); then every J / K
-        // element the quartet touches is summed over the quartet in registers
-        // (FP32 quartets: float products with the float density copies) and
-        // added to the FP64 accumulators once -- nab + ncd + na nc + na nd +
-        // nb nc + nb nd atomics per quartet instead of 6 per integral.
-        constexpr int NA = c_nc(LA), NC = c_nc(LC);
-        const T* __restrict__ QbT = schwarz_of<T>(a) + bra.qoff;
-        const bool screen = a.thr >= 0.0;
-        const T thrT = (T)a.thr;
-#pragma unroll
-        for (int ab = 0; ab < NAB; ++ab) {
-            const int ia = ab / NB, ib = ab % NB;
-            const int i = bra.bf0 + ia, j = bra.bf1 + ib;
-            const long long pij = spidx(i, j);
-            const T qb = __ldg(QbT + pij);
-#pragma unroll
-            for (int cd = 0; cd < NCD; ++cd) {
-                const int ic = (C0 + cd) / ND, id = (C0 + cd) % ND;
-                const int k = ket.bf0 + ic, l = ket.bf1 + id;
-                const long long pkl = spidx(k, l);
-                const bool skip = (bra.same && ia < ib) || (ket.same && ic < id) || (same_pair && pij < pkl) ||
-                                  (screen && qb * __ldg(QbT + pkl) < thrT);
-                const T f = (i == j ? (T)1 : (T)2) * (k == l ? (T)1 : (T)2) * (pij == pkl ? (T)1 : (T)2);
-                acc[ab][cd] = skip ? (T)0 : acc[ab][cd] * f;
-            }
-        }
-        const T* __restrict__ Dj32 = density_of<T>(a.Dj, a.Dj32) + bra.moff;
-        const int i0 = bra.bf0, j0 = bra.bf1, k0 = ket.bf0, l0 = ket.bf1;
-        auto d32 = [&](const T* D, int r, int c) { return __ldg(D + (long long)r * K + c); };
-        auto put = [&](double* M, int r, int c, T v) {
-            if (v != (T)0) add_to_fp64<T>(M + (long long)r * K + c, v);
-        };
-#pragma unroll
-        for (int ab = 0; ab < NAB; ++ab) {
-            T sj = 0;
-#pragma unroll
-            for (int cd = 0; cd < NCD; ++cd) sj += d32(Dj32, k0 + (C0 + cd) / ND, l0 + (C0 + cd) % ND) * acc[ab][cd];
-            put(J, i0 + ab / NB, j0 + ab % NB, sj);
-        }
+    for (int ab = 0; ab < NAB; ++ab) {
+        const int ia = ab / NB, ib = ab % NB;
+        const int i = bra.bf0 + ia, j = bra.bf1 + ib;
+        const long long pij = spidx(i, j);
+        const T qb = __ldg(QbT + pij);
 #pragma unroll
         for (int cd = 0; cd < NCD; ++cd) {
-            T sj = 0;
-#pragma unroll
-            for (int ab = 0; ab < NAB; ++ab) sj += d32(Dj32, i0 + ab / NB, j0 + ab % NB) * acc[ab][cd];
-            put(J, k0 + (C0 + cd) / ND, l0 + (C0 + cd) % ND, sj);
+            const int ic = (C0 + cd) / ND, id = (C0 + cd) % ND;
+            const int k = ket.bf0 + ic, l = ket.bf1 + id;
+            const long long pkl = spidx(k, l);
+            const bool skip = (bra.same && ia < ib) || (ket.same && ic < id) || (same_pair && pij < pkl) ||
+                              (screen && qb * __ldg(QbT + pkl) < thrT);
+            const T f = (i == j ? (T)1 : (T)2) * (k == l ? (T)1 : (T)2) * (pij == pkl ? (T)1 : (T)2);
+            acc[ab][cd] = skip ? (T)0 : acc[ab][cd] * f;
         }
+    }
+    const T* __restrict__ Dj32 = a.Dj32 + bra.moff;
+    const int i0 = bra.bf0, j0 = bra.bf1, k0 = ket.bf0, l0 = ket.bf1;
+    auto d32 = [&](const T* D, int r, int c) { return __ldg(D + (long long)r * K + c); };
+    auto put = [&](double* M, int r, int c, T v) {
+        if (v != (T)0) add_to_fp64<T>(M + (long long)r * K + c, v);
+    };
 #pragma unroll
-        for (int sp = 0; sp < NK; ++sp) {
-            const T* __restrict__ Dk32 =
-                (sp == 0 ? density_of<T>(a.Dk, a.Dk32) : density_of<T>(a.Dk2, a.Dk232)) + bra.moff;
-            double* KK = sp == 0 ? Kx : Kx2;
-            // K_ik += D_jl v, K_jl += D_ik v, K_il += D_jk v, K_jk += D_il v
+    for (int ab = 0; ab < NAB; ++ab) {
+        T sj = 0;
 #pragma unroll
-            for (int ia = 0; ia < NA; ++ia)
+        for (int cd = 0; cd < NCD; ++cd) sj += d32(Dj32, k0 + (C0 + cd) / ND, l0 + (C0 + cd) % ND) * acc[ab][cd];
+        put(J, i0 + ab / NB, j0 + ab % NB, sj);
+    }
 #pragma unroll
-                for (int ic = 0; ic < NC; ++ic) {
-                    T s = 0;
+    for (int cd = 0; cd < NCD; ++cd) {
+        T sj = 0;
 #pragma unroll
-                    for (int ib = 0; ib < NB; ++ib)
+        for (int ab = 0; ab < NAB; ++ab) sj += d32(Dj32, i0 + ab / NB, j0 + ab % NB) * acc[ab][cd];
+        put(J, k0 + (C0 + cd) / ND, l0 + (C0 + cd) % ND, sj);
+    }
 #pragma unroll
-                        for (int id = 0; id < ND; ++id)
-                            if (ic * ND + id >= C0 && ic * ND + id < C1) s += d32(Dk32, j0 + ib, l0 + id) * acc[ia * NB + ib][ic * ND + id - C0];
-                    put(KK, i0 + ia, k0 + ic, s);
-                }
+    for (int sp = 0; sp < NK; ++sp) {
+        const T* __restrict__ Dk32 =
+            (sp == 0 ? a.Dk32 : a.Dk232) + bra.moff;
+        double* KK = sp == 0 ? Kx : Kx2;
+        // K_ik += D_jl v, K_jl += D_ik v, K_il += D_jk v, K_jk += D_il v
 #pragma unroll
-            for (int ib = 0; ib < NB; ++ib)
+        for (int ia = 0; ia < NA; ++ia)
 #pragma unroll
-                for (int id = 0; id < ND; ++id) {
-                    T s = 0;
+            for (int ic = 0; ic < NC; ++ic) {
+                T s = 0;
 #pragma unroll
-                    for (int ia = 0; ia < NA; ++ia)
+                for (int ib = 0; ib < NB; ++ib)
 #pragma unroll
-                        for (int ic = 0; ic < NC; ++ic)
-                            if (ic * ND + id >= C0 && ic * ND + id < C1) s += d32(Dk32, i0 + ia, k0 + ic) * acc[ia * NB + ib][ic * ND + id - C0];
-                    put(KK, j0 + ib, l0 + id, s);
-                }
+                    for (int id = 0; id < ND; ++id)
+                        if (ic * ND + id >= C0 && ic * ND + id < C1) s += d32(Dk32, j0 + ib, l0 + id) * acc[ia * NB + ib][ic * ND + id - C0];
+                put(KK, i0 + ia, k0 + ic, s);
+            }
 #pragma unroll
-            for (int ia = 0; ia < NA; ++ia)
+        for (int ib = 0; ib < NB; ++ib)
 #pragma unroll
-                for (int id = 0; id < ND; ++id) {
-                    T s = 0;
+            for (int id = 0; id < ND; ++id) {
+                T s = 0;
 #pragma unroll
-                    for (int ib = 0; ib < NB; ++ib)
+                for (int ia = 0; ia < NA; ++ia)
 #pragma unroll
-                        for (int ic = 0; ic < NC; ++ic)
-                            if (ic * ND + id >= C0 && ic * ND + id < C1) s += d32(Dk32, j0 + ib, k0 + ic) * acc[ia * NB + ib][ic * ND + id - C0];
-                    put(KK, i0 + ia, l0 + id, s);
-                }
+                    for (int ic = 0; ic < NC; ++ic)
+                        if (ic * ND + id >= C0 && ic * ND + id < C1) s += d32(Dk32, i0 + ia, k0 + ic) * acc[ia * NB + ib][ic * ND + id - C0];
+                put(KK, j0 + ib, l0 + id, s);
+            }
 #pragma unroll
-            for (int ib = 0; ib < NB; ++ib)
+        for (int ia = 0; ia < NA; ++ia)
 #pragma unroll
-                for (int ic = 0; ic < NC; ++ic) {
-                    T s = 0;
+            for (int id = 0; id < ND; ++id) {
+                T s = 0;
 #pragma unroll
-                    for (int ia = 0; ia < NA; ++ia)
+                for (int ib = 0; ib < NB; ++ib)
 #pragma unroll
-                        for (int id = 0; id < ND; ++id)
-                            if (ic * ND + id >= C0 && ic * ND + id < C1) s += d32(Dk32, i0 + ia, l0 + id) * acc[ia * NB + ib][ic * ND + id - C0];
-                    put(KK, j0 + ib, k0 + ic, s);
-                }
-        }
+                    for (int ic = 0; ic < NC; ++ic)
+                        if (ic * ND + id >= C0 && ic * ND + id < C1) s += d32(Dk32, j0 + ib, k0 + ic) * acc[ia * NB + ib][ic * ND + id - C0];
+                put(KK, i0 + ia, l0 + id, s);
+            }
+#pragma unroll
+        for (int ib = 0; ib < NB; ++ib)
+#pragma unroll
+            for (int ic = 0; ic < NC; ++ic) {
+                T s = 0;
+#pragma unroll
+                for (int ia = 0; ia < NA; ++ia)
+#pragma unroll
+                    for (int id = 0; id < ND; ++id)
+                        if (ic * ND + id >= C0 && ic * ND + id < C1) s += d32(Dk32, i0 + ia, l0 + id) * acc[ia * NB + ib][ic * ND + id - C0];
+                put(KK, j0 + ib, k0 + ic, s);
+            }
     }
 }
 
@@ -563,13 +480,13 @@ __device__ __forceinline__ void small_quartet(const SmallArgs<T>& a, const Task&
 // would not fit the register file split their ket component pairs over
 // small_ncb(...) threads per task (each computes R, its block's ket sums,
 // its block's integrals and their digestion; J and K are linear in the
-// integrals), at most 36 (FP64) / 40 (FP32) accumulators per thread.
+// integrals), at most 40 accumulators per thread.
 template <typename T, int LA, int LB, int LC, int LD>
 __host__ __device__ constexpr int small_ncb()
 {
     constexpr int ncd = c_nc(LC) * c_nc(LD);
     constexpr int nab = c_nc(LA) * c_nc(LB);
-    constexpr int budget = sizeof(T) == 8 ? 36 : 40;   // accumulators per thread
+    constexpr int budget = 40;   // accumulators per thread
     int nb = 1;
     while (nb < ncd && nab * ((ncd + nb - 1) / nb) > budget) ++nb;
     return nb;

@@ -1,17 +1,16 @@
 // hfx_device.cuh -- device-side data layout and helpers shared by the
 // shell-quartet kernels.
 //
-// HBM layout of one job (all arrays device-resident for the job's lifetime):
+// Layout of the FP32 launches of a mixed-precision job (device-resident for the
+// job's lifetime; the FP64 tables are those of hfx_team.hpp):
 //   DPair[npairs]    one record per shell pair (A >= B in shell order), the
 //                    shell with the higher L stored first ("0" side)
-//   pp_geo[npp]      PairGeo per primitive pair: (p, Px, Py, Pz)
-//   E pool           per primitive pair, the dense Hermite->Cartesian matrix
-//                    E[ab][tuv] (n0*n1 x H(l0+l1)), with the primitive weights
-//                    w_i(a) w_j(b) (coefficient x cart_norm) and
-//                    exp(-mu |AB|^2) folded in; tuv in the reference's packed
-//                    order (integrals.hpp:343-358)
+//   records          per primitive pair, see PairClassTab
 //   Qbf[K(K+1)/2]    BF-level Schwarz bounds, pair_index order
-//   boys table       F_m(T_k), T_k = k/16, m = 0..kBoysM-1
+// The host image of the pair data also holds the geometry (PairGeo) and the
+// dense Hermite->Cartesian matrices E[ab][tuv] of every primitive pair
+// (hfx_debug_pair_data), tuv in the reference's packed order
+// (integrals.hpp:343-358).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -37,13 +36,6 @@ constexpr int kBoysN = kBoysTMax * kBoysInvStep + 1;
 // so that one evaluation is two 16-byte loads.
 constexpr int kBoys32MaxL = 12;
 constexpr int kBoys32Row = 8;
-// The FP64 Fock kernels' table, one 8-double row per (L, k): {F_L, F_{L+1},
-// F_{L+2}/2!, ..., F_{L+6}/6!, exp(-T_k)} at T_k = k/16, L <= kBoys64MaxL:
-// the 7-term Taylor expansion of F_L about T_k with its coefficients
-// pre-scaled (four 16-byte loads and six FMAs, no multiplies).
-constexpr int kBoys64MaxL = 12;
-constexpr int kBoys64Row = 8;
-
 // Primitive-pair geometry: p = alpha + beta and the product centre P.
 struct __align__(32) PairGeo {
     double p, x, y, z;
@@ -187,7 +179,7 @@ struct WarpArgs {
     const Task* tasks;
     int ntasks;
     int* counter;
-    const T* boys;             // per-L rows: kBoys64Row doubles (FP64) / kBoys32Row floats (FP32)
+    const T* boys;             // per-L rows of kBoys32Row floats
     double thr;
     const double* Qbf;
     int K;
@@ -201,8 +193,6 @@ struct WarpArgs {
     int lane_min_npp;          // lane-parallel R for L <= 6 and ket npp >= this (0: never)
     const double* Dsh;         // per shell pair max |D| (density screening), or null
     double dthr;               // skip a quartet when Q_AB Q_CD max|D| < dthr (0: never)
-    double* Qout_bf;           // Schwarz pass (NK = 0): BF-pair bounds out
-    unsigned long long* Qout_sh;   // Schwarz pass: per shell pair max bound (double bits)
     const unsigned char* active;   // packed jobs: per molecule, 0 = skip its quartets (null: all)
     // FP32 kernels: float copies of Dj / Dk / Dk2 for the block digestion
     const float* Dj32;
@@ -268,34 +258,6 @@ __device__ __forceinline__ bool density_negligible(const DPair& b, const DPair& 
     d = fmax(d, D[shell_pair_id(b.sh1, k.sh0)]);
     d = fmax(d, D[shell_pair_id(b.sh1, k.sh1)]);
     return b.qmax * k.qmax * d < dthr;
-}
-
-// Digestion form of the FP64 kernels: false = 6 atomics per integral,
-// true = per-quartet block sums (the FP32 kernels always use block sums).
-// Block sums measured 0-4% slower for FP64 builds (benzene/cc-pVDZ,
-// n-decane/6-31G*), which are bound by the FP64 pipe, not by atomics.
-constexpr bool kBlockDigestFP64 = false;
-
-// The density the block digestion multiplies with: FP64 kernels the FP64
-// matrix, FP32 kernels its float copy.
-template <typename T>
-__device__ __forceinline__ const T* density_of(const double* d64, const float* d32)
-{
-    if constexpr (sizeof(T) == 8)
-        return d64;
-    else
-        return d32;
-}
-
-// The BF-pair Schwarz bounds a kernel of precision T screens with: FP64
-// kernels the double table, FP32 kernels its float copy.
-template <typename T, typename A>
-__device__ __forceinline__ const T* schwarz_of(const A& a)
-{
-    if constexpr (sizeof(T) == 8)
-        return a.Qbf;
-    else
-        return a.Qbf32;
 }
 
 // Quartet of a molecule that takes no part in this build of a packed job.

@@ -3,15 +3,15 @@
 // Job creation replaces what the reference does per SCF inside ERI_GPU
 // (cuda/src/eri.cu:20-89): instead of an AoS of basis functions plus a
 // CPU-side Schwarz table, the job keeps in HBM
-//   * one record per shell pair with its primitive-pair geometry and the
-//     dense Hermite->Cartesian E matrices (weights and exp(-mu AB^2) folded),
-//   * a Boys-function table (FP64, Taylor grid),
+//   * the super pairs of the FP64 kernel (hfx_team.hpp) and, for mixed
+//     precision, one float record per shell pair and primitive pair,
+//   * Boys-function tables,
 //   * the BF-level Schwarz table, computed on the device from the diagonal
-//     shell quartets (the reference's schwarz_bounds, integrals.hpp:732-752,
-//     runs on the CPU even on its GPU path, eri.cu:32),
-//   * the screened list of unique shell quartets (the reference screens per
-//     basis-function quartet, integrals.hpp:771),
-// so that every Fock build is: upload density -> one work-queue launch ->
+//     quartets (the reference's schwarz_bounds, integrals.hpp:732-752, runs on
+//     the CPU even on its GPU path, eri.cu:32),
+//   * the plans: the tasks of the surviving quartets (the reference screens
+//     per basis-function quartet, integrals.hpp:771),
+// so that every Fock build is: upload density -> one graph launch ->
 // symmetrise -> download, with no ERI storage.
 #include "hfx_engine.hpp"
 
@@ -1352,10 +1352,10 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
             void* prm[] = {&a};
             sk.kernel(lane, ks, prm);
         } else {
-            cuda_check(warp_spec(true, nk, g.grid, g.warps_per_cta, g.slice, &ks), "warp kernel");
+            cuda_check(warp_spec(nk, g.grid, g.warps_per_cta, g.slice, &ks), "warp kernel");
             WarpArgs<float> a{d_pairs_.p, d_rec32_.p, d_pct_.p, d_abs_.p, d_kh_.p, d_kl_.p, tasks + g.off, (int)g.n,
                               ctr + gi, d_boys32_.p, opt_.screening_threshold, d_qbf_.p, K, Dj, Dk, Dk2, J, Kx, Kx2,
-                              g.slice, g.lane_min_npp, Dsh, dthr, nullptr, nullptr, active, Dj32, Dk32, Dk232,
+                              g.slice, g.lane_min_npp, Dsh, dthr, active, Dj32, Dk32, Dk232,
                               d_qbf32_.p, ncopy, cstride};
             void* prm[] = {&a};
             sk.kernel(naux, ks, prm);

@@ -26,8 +26,7 @@ KernelSpec to_float_spec(long long n);   // k_to_float(A, B, n)
 KernelSpec density_blocks_spec(int npairs);   // k_density_blocks(pairs, npairs, D1, D2, Dsh)
 KernelSpec rebase_tasks_spec(long long n);    // k_rebase_tasks(tasks, n, delta): bra, ket += delta
 cudaError_t small_spec_f32(int pcb, int pck, int nk, int ntasks, KernelSpec* s);   // k_small(SmallArgs<float>)
-cudaError_t warp_spec(bool fp32, int nk, int grid, int warps_per_cta, int slice, KernelSpec* s);
-cudaError_t launch_warp(bool fp32, const void* args, int nk, int grid, int warps_per_cta, cudaStream_t st);
+cudaError_t warp_spec(int nk, int grid, int warps_per_cta, int slice, KernelSpec* s);   // k_warp_quartet(WarpArgs<float>)
 // shared-memory slice (elements) of a warp task; the lane-parallel R mode (L <= 6,
 // ket npp >= lane_min_npp, 0: never) needs 32 R vectors, the level-parallel one a round
 int warp_slice_elems(int l0b, int l1b, int l0k, int l1k, int npp_ket, int lane_min_npp);

@@ -477,10 +477,10 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
             void* prm[] = {&a};
             sk.kernel(lane, ks, prm);
         } else {
-            cuda_check(warp_spec(true, nk, g.grid, g.warps_per_cta, g.slice, &ks), "session warp kernel");
+            cuda_check(warp_spec(nk, g.grid, g.warps_per_cta, g.slice, &ks), "session warp kernel");
             WarpArgs<float> a{pairs32_.p, anchor32_.p, pct_.p, abs_.p, kh_.p, kl_.p, tasks + g.off, (int)g.n,
                               ctr + gi, boys32_.p, thr_, nullptr, 0, Dj, Dk, Dk2, J, Kx, Kx2, g.slice,
-                              g.lane_min_npp, Dsh, dthr, nullptr, nullptr, active, Dj32, Dk32, Dk232, anchor32_.p, 1, 0};
+                              g.lane_min_npp, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p, 1, 0};
             void* prm[] = {&a};
             sk.kernel(naux, ks, prm);
         }

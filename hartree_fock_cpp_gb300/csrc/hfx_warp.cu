@@ -1,5 +1,5 @@
 // hfx_warp.cu -- warp-per-shell-quartet McMurchie-Davidson kernel with direct
-// J/K digestion, for any angular-momentum class (runtime L), FP64 or FP32.
+// J/K digestion, for any angular-momentum class (runtime L), in FP32.
 //
 // Each warp takes shell quartets from a global work queue and works on its own
 // slice of shared memory; there are no CTA-wide barriers.  Per bra primitive
@@ -39,75 +39,37 @@ __device__ __forceinline__ T w_fma(T a, T b, T c)
 template <typename T>
 __device__ __forceinline__ void boys_top(T Tv, int L, const T* __restrict__ tab, T& FL, T& e, bool& table)
 {
-    if constexpr (sizeof(T) == 4) {
-        // FP32 table: one 8-float row per (L, k), Taylor terms pre-scaled
-        if (Tv < (T)kBoysTMax) {
-            table = true;
-            int k;
-            const T nd = boys_grid_offset(Tv, k);
-            const float4* row = reinterpret_cast<const float4*>(tab + ((size_t)L * kBoysN + k) * kBoys32Row);
-            const float4 c0 = __ldg(row), c1 = __ldg(row + 1);
-            T r = c1.x;
-            r = w_fma(r, nd, c0.w);
-            r = w_fma(r, nd, c0.z);
-            r = w_fma(r, nd, c0.y);
-            FL = w_fma(r, nd, c0.x);
-            T x = (T)(1.0 / 24.0);
-            x = w_fma(x, nd, (T)(1.0 / 6.0));
-            x = w_fma(x, nd, (T)0.5);
-            x = w_fma(x, nd, (T)1);
-            x = w_fma(x, nd, (T)1);
-            e = c1.y * x;
-        } else {
-            table = false;
-            FL = (T)0;
-            e = (T)0;
-        }
-    } else if (Tv < (T)kBoysTMax) {
-        // FP64 table: one 8-double row per (L, k), Taylor terms pre-scaled
+    // FP32 table: one 8-float row per (L, k), Taylor terms pre-scaled
+    if (Tv < (T)kBoysTMax) {
         table = true;
-        int k = (int)(Tv * (T)kBoysInvStep + (T)0.5);
-        T nd = (T)k * ((T)1 / (T)kBoysInvStep) - Tv;
-        const double2* row = reinterpret_cast<const double2*>(tab + ((size_t)L * kBoysN + k) * kBoys64Row);
-        const double2 c0 = __ldg(row), c1 = __ldg(row + 1), c2 = __ldg(row + 2), c3 = __ldg(row + 3);
-        T r = c3.x;
-        r = w_fma(r, nd, c2.y);
-        r = w_fma(r, nd, c2.x);
-        r = w_fma(r, nd, c1.y);
-        r = w_fma(r, nd, c1.x);
+        int k;
+        const T nd = boys_grid_offset(Tv, k);
+        const float4* row = reinterpret_cast<const float4*>(tab + ((size_t)L * kBoysN + k) * kBoys32Row);
+        const float4 c0 = __ldg(row), c1 = __ldg(row + 1);
+        T r = c1.x;
+        r = w_fma(r, nd, c0.w);
+        r = w_fma(r, nd, c0.z);
         r = w_fma(r, nd, c0.y);
         FL = w_fma(r, nd, c0.x);
-        // exp(-T) = exp(-T_k) exp(nd), |nd| <= 1/32
-        T x = (T)(1.0 / 5040.0);
-        x = w_fma(x, nd, (T)(1.0 / 720.0));
-        x = w_fma(x, nd, (T)(1.0 / 120.0));
-        x = w_fma(x, nd, (T)(1.0 / 24.0));
+        T x = (T)(1.0 / 24.0);
         x = w_fma(x, nd, (T)(1.0 / 6.0));
         x = w_fma(x, nd, (T)0.5);
         x = w_fma(x, nd, (T)1);
         x = w_fma(x, nd, (T)1);
-        e = c3.y * x;
+        e = c1.y * x;
     } else {
         table = false;
         FL = (T)0;
-        e = L >= 5 ? (T)exp(-(double)Tv) : (T)0;
+        e = (T)0;
     }
 }
 
 // 1/(2m+1), m = 0..15, for the downward Boys recursion
-__constant__ double c_inv_odd64[16] = {1.0,       1.0 / 3,  1.0 / 5,  1.0 / 7,  1.0 / 9,  1.0 / 11,
-                                       1.0 / 13,  1.0 / 15, 1.0 / 17, 1.0 / 19, 1.0 / 21, 1.0 / 23,
-                                       1.0 / 25,  1.0 / 27, 1.0 / 29, 1.0 / 31};
 __constant__ float c_inv_odd32[16] = {1.0f,       1.0f / 3,  1.0f / 5,  1.0f / 7,  1.0f / 9,  1.0f / 11,
                                       1.0f / 13,  1.0f / 15, 1.0f / 17, 1.0f / 19, 1.0f / 21, 1.0f / 23,
                                       1.0f / 25,  1.0f / 27, 1.0f / 29, 1.0f / 31};
 template <typename T>
 __device__ __forceinline__ T inv_odd(int m);
-template <>
-__device__ __forceinline__ double inv_odd<double>(int m)
-{
-    return c_inv_odd64[m];
-}
 template <>
 __device__ __forceinline__ float inv_odd<float>(int m)
 {
@@ -405,22 +367,6 @@ __global__ void __launch_bounds__(256) k_warp_quartet(WarpArgs<T> a)
             __syncwarp();
         }
 
-        // Schwarz pass: diagonal (ab|ab) of the diagonal shell quartet (AB|AB)
-        if constexpr (NK == 0) {
-            for (int e = lane; e < nout; e += 32) {
-                const int ab = e / ncd, cd = e - ab * ncd;
-                if (ab != cd) continue;
-                const int ia = ab / n1, ib = ab - ia * n1;
-                if (bra.same && ia < ib) continue;
-                const double v = (double)acc[e];
-                const double qv = sqrt(v > 0.0 ? v : 0.0);
-                a.Qout_bf[bra.qoff + wpidx(bra.bf0 + ia, bra.bf1 + ib)] = qv;
-                atomicMax(a.Qout_sh + task.bra, (unsigned long long)__double_as_longlong(qv));
-            }
-            __syncwarp();
-            continue;
-        }
-
         // digestion (FP64), into the bra pair's molecule's matrices
         const int K = bra.kdim;
         const double* __restrict__ Qbf = a.Qbf + bra.qoff;
@@ -430,109 +376,83 @@ __global__ void __launch_bounds__(256) k_warp_quartet(WarpArgs<T> a)
         double* J = a.J + bra.moff;
         double* Kx = a.Kx + bra.moff;
         double* Kx2 = a.Kx2 + (NK == 2 ? bra.moff : 0);
-        if constexpr (sizeof(T) == 8 && !kBlockDigestFP64) {
-            for (int e = lane; e < nout; e += 32) {
-                const int ab = e / ncd, cd = e - ab * ncd;
-                const int ia = ab / n1, ib = ab - ia * n1, ic = cd / n3, id = cd - ic * n3;
-                const int i = bra.bf0 + ia, j = bra.bf1 + ib, k = ket.bf0 + ic, l = ket.bf1 + id;
-                if (bra.same && ia < ib) continue;
-                if (ket.same && ic < id) continue;
-                const long long pij = wpidx(i, j), pkl = wpidx(k, l);
-                if (task.bra == task.ket && pij < pkl) continue;
-                if (a.thr >= 0.0 && __ldg(Qbf + pij) * __ldg(Qbf + pkl) < a.thr) continue;
-                double v = (double)acc[e] * ((i == j ? 1.0 : 2.0) * (k == l ? 1.0 : 2.0) * (pij == pkl ? 1.0 : 2.0));
-                atomicAdd(J + (long long)i * K + j, __ldg(Dj + (long long)k * K + l) * v);
-                atomicAdd(J + (long long)k * K + l, __ldg(Dj + (long long)i * K + j) * v);
-                atomicAdd(Kx + (long long)i * K + k, __ldg(Dk + (long long)j * K + l) * v);
-                atomicAdd(Kx + (long long)j * K + l, __ldg(Dk + (long long)i * K + k) * v);
-                atomicAdd(Kx + (long long)i * K + l, __ldg(Dk + (long long)j * K + k) * v);
-                atomicAdd(Kx + (long long)j * K + k, __ldg(Dk + (long long)i * K + l) * v);
-                if (NK == 2) {
-                    atomicAdd(Kx2 + (long long)i * K + k, __ldg(Dk2 + (long long)j * K + l) * v);
-                    atomicAdd(Kx2 + (long long)j * K + l, __ldg(Dk2 + (long long)i * K + k) * v);
-                    atomicAdd(Kx2 + (long long)i * K + l, __ldg(Dk2 + (long long)j * K + k) * v);
-                    atomicAdd(Kx2 + (long long)j * K + k, __ldg(Dk2 + (long long)i * K + l) * v);
-                }
+        // Block digestion: weights in place (0 for non-canonical and
+        // BF-screened elements), then one lane per J / K element the
+        // quartet touches sums its contributions (FP32 quartets: float
+        // products with the float density copies) and adds the sum to the
+        // FP64 accumulator: nab + ncd + na nc + na nd + nb nc + nb nd
+        // atomics per quartet instead of 6 per integral.
+        const T* __restrict__ QbT = a.Qbf32 + bra.qoff;
+        const bool screen = a.thr >= 0.0;
+        const T thrT = (T)a.thr;
+        for (int e = lane; e < nout; e += 32) {
+            const int ab = e / ncd, cd = e - ab * ncd;
+            const int ia = ab / n1, ib = ab - ia * n1, ic = cd / n3, id = cd - ic * n3;
+            const int i = bra.bf0 + ia, j = bra.bf1 + ib, k = ket.bf0 + ic, l = ket.bf1 + id;
+            const long long pij = wpidx(i, j), pkl = wpidx(k, l);
+            const bool skip = (bra.same && ia < ib) || (ket.same && ic < id) ||
+                              (task.bra == task.ket && pij < pkl) ||
+                              (screen && __ldg(QbT + pij) * __ldg(QbT + pkl) < thrT);
+            const T f = (i == j ? (T)1 : (T)2) * (k == l ? (T)1 : (T)2) * (pij == pkl ? (T)1 : (T)2);
+            acc[e] = skip ? (T)0 : acc[e] * f;
+        }
+        __syncwarp();
+        const int n0 = w_nc(bra.l0), n2 = w_nc(ket.l0);
+        const int i0 = bra.bf0, j0 = bra.bf1, k0 = ket.bf0, l0 = ket.bf1;
+        const T* __restrict__ Dj32 = a.Dj32 + bra.moff;
+        auto d32 = [&](const T* D, int r, int c) { return __ldg(D + (long long)r * K + c); };
+        auto put = [&](double* M, int r, int c, T v) {
+            if (v != (T)0) add_to_fp64<T>(M + (long long)r * K + c, v);
+        };
+        for (int ab = lane; ab < nab; ab += 32) {
+            T sj = 0;
+            for (int cd = 0; cd < ncd; ++cd) sj += d32(Dj32, k0 + cd / n3, l0 + cd % n3) * acc[ab * ncd + cd];
+            put(J, i0 + ab / n1, j0 + ab % n1, sj);
+        }
+        for (int cd = lane; cd < ncd; cd += 32) {
+            T sj = 0;
+            for (int ab = 0; ab < nab; ++ab) sj += d32(Dj32, i0 + ab / n1, j0 + ab % n1) * acc[ab * ncd + cd];
+            put(J, k0 + cd / n3, l0 + cd % n3, sj);
+        }
+        for (int sp = 0; sp < NK; ++sp) {
+            const T* __restrict__ Dk32 =
+                (sp == 0 ? a.Dk32 : a.Dk232) + bra.moff;
+            double* KK = sp == 0 ? Kx : Kx2;
+            // K_ik += D_jl v over (b, d)
+            for (int q = lane; q < n0 * n2; q += 32) {
+                const int ia = q / n2, ic = q - ia * n2;
+                T s = 0;
+                for (int ib = 0; ib < n1; ++ib)
+                    for (int id = 0; id < n3; ++id)
+                        s += d32(Dk32, j0 + ib, l0 + id) * acc[(ia * n1 + ib) * ncd + ic * n3 + id];
+                put(KK, i0 + ia, k0 + ic, s);
             }
-        } else {
-            // Block digestion: weights in place (0 for non-canonical and
-            // BF-screened elements), then one lane per J / K element the
-            // quartet touches sums its contributions (FP32 quartets: float
-            // products with the float density copies) and adds the sum to the
-            // FP64 accumulator: nab + ncd + na nc + na nd + nb nc + nb nd
-            // atomics per quartet instead of 6 per integral.
-            const T* __restrict__ QbT = schwarz_of<T>(a) + bra.qoff;
-            const bool screen = a.thr >= 0.0;
-            const T thrT = (T)a.thr;
-            for (int e = lane; e < nout; e += 32) {
-                const int ab = e / ncd, cd = e - ab * ncd;
-                const int ia = ab / n1, ib = ab - ia * n1, ic = cd / n3, id = cd - ic * n3;
-                const int i = bra.bf0 + ia, j = bra.bf1 + ib, k = ket.bf0 + ic, l = ket.bf1 + id;
-                const long long pij = wpidx(i, j), pkl = wpidx(k, l);
-                const bool skip = (bra.same && ia < ib) || (ket.same && ic < id) ||
-                                  (task.bra == task.ket && pij < pkl) ||
-                                  (screen && __ldg(QbT + pij) * __ldg(QbT + pkl) < thrT);
-                const T f = (i == j ? (T)1 : (T)2) * (k == l ? (T)1 : (T)2) * (pij == pkl ? (T)1 : (T)2);
-                acc[e] = skip ? (T)0 : acc[e] * f;
+            // K_jl += D_ik v over (a, c)
+            for (int q = lane; q < n1 * n3; q += 32) {
+                const int ib = q / n3, id = q - ib * n3;
+                T s = 0;
+                for (int ia = 0; ia < n0; ++ia)
+                    for (int ic = 0; ic < n2; ++ic)
+                        s += d32(Dk32, i0 + ia, k0 + ic) * acc[(ia * n1 + ib) * ncd + ic * n3 + id];
+                put(KK, j0 + ib, l0 + id, s);
             }
-            __syncwarp();
-            const int n0 = w_nc(bra.l0), n2 = w_nc(ket.l0);
-            const int i0 = bra.bf0, j0 = bra.bf1, k0 = ket.bf0, l0 = ket.bf1;
-            const T* __restrict__ Dj32 = density_of<T>(a.Dj, a.Dj32) + bra.moff;
-            auto d32 = [&](const T* D, int r, int c) { return __ldg(D + (long long)r * K + c); };
-            auto put = [&](double* M, int r, int c, T v) {
-                if (v != (T)0) add_to_fp64<T>(M + (long long)r * K + c, v);
-            };
-            for (int ab = lane; ab < nab; ab += 32) {
-                T sj = 0;
-                for (int cd = 0; cd < ncd; ++cd) sj += d32(Dj32, k0 + cd / n3, l0 + cd % n3) * acc[ab * ncd + cd];
-                put(J, i0 + ab / n1, j0 + ab % n1, sj);
+            // K_il += D_jk v over (b, c)
+            for (int q = lane; q < n0 * n3; q += 32) {
+                const int ia = q / n3, id = q - ia * n3;
+                T s = 0;
+                for (int ib = 0; ib < n1; ++ib)
+                    for (int ic = 0; ic < n2; ++ic)
+                        s += d32(Dk32, j0 + ib, k0 + ic) * acc[(ia * n1 + ib) * ncd + ic * n3 + id];
+                put(KK, i0 + ia, l0 + id, s);
             }
-            for (int cd = lane; cd < ncd; cd += 32) {
-                T sj = 0;
-                for (int ab = 0; ab < nab; ++ab) sj += d32(Dj32, i0 + ab / n1, j0 + ab % n1) * acc[ab * ncd + cd];
-                put(J, k0 + cd / n3, l0 + cd % n3, sj);
-            }
-            for (int sp = 0; sp < NK; ++sp) {
-                const T* __restrict__ Dk32 =
-                    (sp == 0 ? density_of<T>(a.Dk, a.Dk32) : density_of<T>(a.Dk2, a.Dk232)) + bra.moff;
-                double* KK = sp == 0 ? Kx : Kx2;
-                // K_ik += D_jl v over (b, d)
-                for (int q = lane; q < n0 * n2; q += 32) {
-                    const int ia = q / n2, ic = q - ia * n2;
-                    T s = 0;
-                    for (int ib = 0; ib < n1; ++ib)
-                        for (int id = 0; id < n3; ++id)
-                            s += d32(Dk32, j0 + ib, l0 + id) * acc[(ia * n1 + ib) * ncd + ic * n3 + id];
-                    put(KK, i0 + ia, k0 + ic, s);
-                }
-                // K_jl += D_ik v over (a, c)
-                for (int q = lane; q < n1 * n3; q += 32) {
-                    const int ib = q / n3, id = q - ib * n3;
-                    T s = 0;
-                    for (int ia = 0; ia < n0; ++ia)
-                        for (int ic = 0; ic < n2; ++ic)
-                            s += d32(Dk32, i0 + ia, k0 + ic) * acc[(ia * n1 + ib) * ncd + ic * n3 + id];
-                    put(KK, j0 + ib, l0 + id, s);
-                }
-                // K_il += D_jk v over (b, c)
-                for (int q = lane; q < n0 * n3; q += 32) {
-                    const int ia = q / n3, id = q - ia * n3;
-                    T s = 0;
-                    for (int ib = 0; ib < n1; ++ib)
-                        for (int ic = 0; ic < n2; ++ic)
-                            s += d32(Dk32, j0 + ib, k0 + ic) * acc[(ia * n1 + ib) * ncd + ic * n3 + id];
-                    put(KK, i0 + ia, l0 + id, s);
-                }
-                // K_jk += D_il v over (a, d)
-                for (int q = lane; q < n1 * n2; q += 32) {
-                    const int ib = q / n2, ic = q - ib * n2;
-                    T s = 0;
-                    for (int ia = 0; ia < n0; ++ia)
-                        for (int id = 0; id < n3; ++id)
-                            s += d32(Dk32, i0 + ia, l0 + id) * acc[(ia * n1 + ib) * ncd + ic * n3 + id];
-                    put(KK, j0 + ib, k0 + ic, s);
-                }
+            // K_jk += D_il v over (a, d)
+            for (int q = lane; q < n1 * n2; q += 32) {
+                const int ib = q / n2, ic = q - ib * n2;
+                T s = 0;
+                for (int ia = 0; ia < n0; ++ia)
+                    for (int id = 0; id < n3; ++id)
+                        s += d32(Dk32, i0 + ia, l0 + id) * acc[(ia * n1 + ib) * ncd + ic * n3 + id];
+                put(KK, j0 + ib, k0 + ic, s);
             }
         }
         __syncwarp();
@@ -577,29 +497,18 @@ static cudaError_t warp_spec_t(int nk, int grid, int warps_per_cta, int slice, K
         s->func = (const void*)kern;
         return allow_max_smem(kern);
     };
-    cudaError_t e = nk == 2 ? pick(k_warp_quartet<T, 2>) : nk == 0 ? pick(k_warp_quartet<T, 0>) : pick(k_warp_quartet<T, 1>);
+    cudaError_t e = nk == 2 ? pick(k_warp_quartet<T, 2>)  : pick(k_warp_quartet<T, 1>);
     s->grid = dim3((unsigned)grid);
     s->block = dim3((unsigned)(32 * warps_per_cta));
     s->smem = kWarpSmemHeader + sizeof(T) * (size_t)slice * warps_per_cta;
     return e;
 }
 
-// Launch configuration of k_warp_quartet<T, nk> (T = float when fp32); also
-// raises the kernel's shared-memory limit the first time it is asked for.
-cudaError_t warp_spec(bool fp32, int nk, int grid, int warps_per_cta, int slice, KernelSpec* s)
+// Launch configuration of k_warp_quartet<float, nk>; also raises the kernel's
+// shared-memory limit the first time it is asked for.
+cudaError_t warp_spec(int nk, int grid, int warps_per_cta, int slice, KernelSpec* s)
 {
-    return fp32 ? warp_spec_t<float>(nk, grid, warps_per_cta, slice, s)
-                : warp_spec_t<double>(nk, grid, warps_per_cta, slice, s);
-}
-
-cudaError_t launch_warp(bool fp32, const void* args, int nk, int grid, int warps_per_cta, cudaStream_t st)
-{
-    const int slice = fp32 ? ((const WarpArgs<float>*)args)->slice : ((const WarpArgs<double>*)args)->slice;
-    KernelSpec s;
-    cudaError_t e = warp_spec(fp32, nk, grid, warps_per_cta, slice, &s);
-    if (e != cudaSuccess) return e;
-    void* prm[] = {const_cast<void*>(args)};
-    return cudaLaunchKernel(s.func, s.grid, s.block, prm, s.smem, st);
+    return warp_spec_t<float>(nk, grid, warps_per_cta, slice, s);
 }
 
 }  // namespace hfx
