@@ -14,7 +14,7 @@
 //
 // Limits: K <= kNoAllocMaxK basis functions and at most kNoAllocMaxGroups
 // kernel launch groups per build; larger jobs are rejected with
-// HFX_ERR_UNSUPPORTED.  The array (2 * 512 * 512 doubles + 64 ints, about
+// HFX_ERR_UNSUPPORTED.  The array (2 * 512 * 512 doubles + 256 ints, about
 // 4 MB) is reserved on a device when the first job is created there (module
 // loading is lazy by default; job creation resolves the array's address) and
 // stays reserved until the process exits.  All calls share it: two builds that overlap on the GPU (two
@@ -30,7 +30,8 @@
 namespace hfx {
 
 constexpr int kNoAllocMaxK = 512;
-constexpr int kNoAllocMaxGroups = 64;
+// a mixed build of cc-pVTZ molecules with d and f functions has up to about 75
+constexpr int kNoAllocMaxGroups = 256;
 
 struct NoAllocScratch {
     double jacc[kNoAllocMaxK * kNoAllocMaxK];

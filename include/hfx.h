@@ -170,7 +170,8 @@ typedef struct {
 
 hfx_status hfx_last_build_stats(const hfx_job *job, hfx_build_stats *stats);
 
-/* Launch shape of a job's Fock-build plans: primitive quartets per task of
+/* Launch shape of the FP32 part of a job's mixed-precision plan (the FP64
+ * tasks are sized by their cost): primitive quartets per task of
  * the thread-per-quartet kernels (small_chunk) and of the warp kernel
  * (warp_chunk; heavily contracted quartets are split into chunks of bra
  * primitive pairs), the warp kernel's maximum warps per CTA (1..8), and the
@@ -296,9 +297,12 @@ hfx_status hfx_debug_packed_pairs(const hfx_molecule *mols, int n, int *npairs, 
 
 /* Test hook (no device work): the launch groups of a job's Fock-build plan
  * (mixed != 0: the mixed-precision plan of a mixed job), 10 doubles per
- * group: kind (0 thread-per-quartet class kernel, 1 warp kernel), bra and
- * ket pair class (class kernels), fp32, tasks, algorithmic flops, primitive
- * quartets, grid, shared-memory slice and warps per CTA (warp kernel).
+ * group: kind (0 FP32 thread-per-quartet class kernel, 1 FP32 warp kernel, 2
+ * FP64 team kernel), bra and ket pair class (class kernels) or compiled total
+ * angular momentum (-1: general) and threads per team (team kernel), fp32,
+ * tasks, algorithmic flops (team kernel: estimated instructions), primitive
+ * quartets (team kernel: 0), grid, shared-memory slice, warps per CTA (warp
+ * kernel).
  * Pass rows = NULL to get ngroups.  No counterpart in the reference. */
 hfx_status hfx_debug_plan(const hfx_job *job, int mixed, int *ngroups, double *rows);
 

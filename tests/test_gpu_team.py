@@ -7,11 +7,14 @@ accurate-Boys restatement of the reference's tensor and contractions.
 Tolerance: G, J and K are sums of at most K^2 products |D| |(ij|kl)| with
 |D| <= 1 and |(ij|kl)| <= 5 here, each integral within 1e-14 of its size:
 1e-11 on a matrix element, 1e-12 on an integral."""
+import ctypes
+
 import numpy as np
 import pytest
 
 import oracle as O
 import hartree_fock_cpp_gb300 as H
+from hartree_fock_cpp_gb300 import _lib
 from hartree_fock_cpp_gb300 import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -53,6 +56,22 @@ def test_super_shell_kernel_matches_oracle(name, thr):
     assert np.abs(J - O.coulomb_matrix(Pa, Pb, eri)).max() < 1e-11
     assert np.abs(Ka - O.exchange_matrix(Pa, eri)).max() < 1e-11
     assert np.abs(Kb - O.exchange_matrix(Pb, eri)).max() < 1e-11
+
+
+def test_allocation_free_build_takes_a_mixed_plan_of_many_launches():
+    """NaCl/cc-pVTZ mixed: FP64 launches of every angular momentum beside the
+    FP32 classes, more than 64 in all."""
+    torch = pytest.importorskip("torch")
+    with H.FockBuilder(config=W.nacl_scan(8)[3], basis_set="cc-pVTZ", precision=H.HFX_PREC_MIXED,
+                       fp32_threshold=1e-2) as fb:
+        P = torch.from_numpy(_densities(fb.K, 7)[0]).cuda()
+        want, got = torch.empty_like(P), torch.full_like(P, float("nan"))
+        torch.cuda.synchronize()
+        fb.repulsion_matrix_device(P.data_ptr(), want.data_ptr())
+        _lib.check(_lib.lib.hfx_fock_rhf_device_noalloc(fb._job, ctypes.c_void_p(P.data_ptr()),
+                                                        ctypes.c_void_p(got.data_ptr())))
+        torch.cuda.synchronize()
+    assert float((want - got).abs().max()) < 1e-11
 
 
 def test_shells_given_as_functions_share_exponents_in_any_order():
