@@ -591,6 +591,11 @@ PairData build_pair_data(const Basis& basis, const Fragments& fr)
 void Job::build_pairs()
 {
     PairData pd = build_pair_data(basis_, frags_);
+    // The FP32 tasks are tiles of the records, which their kernels index
+    // without a check: the list of shell pairs takes the records' counts.  The
+    // super pairs fold both orders of two shells' common exponents and keep
+    // other primitive pairs.
+    take_record_counts(hpairs_, pd);
     dpairs_host_ = std::move(pd.dpairs);
     for (size_t p = 0; p < dpairs_host_.size(); ++p) dpairs_host_[p].qmax = qsh_[p];
     d_pairs_.upload(dpairs_host_, stream_);
@@ -604,6 +609,16 @@ void Job::build_pairs()
     d_kh_.upload(ct.k_herm, stream_);
     d_kl_.upload(ct.k_lin, stream_);
     cuda_check(cudaStreamSynchronize(stream_), "pair upload");
+}
+
+void take_record_counts(std::vector<HostPair>& pairs, const PairData& pd)
+{
+    if (pairs.size() != pd.hpairs.size()) throw Error(HFX_ERR_INVALID, "shell pairs and their records disagree");
+    for (size_t p = 0; p < pairs.size(); ++p) {
+        if (pairs[p].s0 != pd.hpairs[p].s0 || pairs[p].s1 != pd.hpairs[p].s1 || pairs[p].frag != pd.hpairs[p].frag)
+            throw Error(HFX_ERR_INVALID, "shell pairs and their records disagree");
+        pairs[p].npp = pd.hpairs[p].npp;
+    }
 }
 
 TeamArgs Job::team_args(const TeamPlanDev& plan, const TeamGroup& g, int* counter) const

@@ -140,6 +140,8 @@ Basis concat_basis(const std::vector<Basis>& mols, Fragments& fr);
 Fragments single_fragment(const Basis& b);
 
 PairData build_pair_data(const Basis& b, const Fragments& fr);
+// Primitive-pair counts of `pd`'s records into a list of the same shell pairs.
+void take_record_counts(std::vector<HostPair>& pairs, const PairData& pd);
 
 // Primitive pairs below this fraction of their shell pair's largest
 // coefficient are left out (build_pair_data, build_super_data).

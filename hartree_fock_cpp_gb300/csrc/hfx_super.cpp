@@ -265,11 +265,13 @@ SuperData build_super_data(const Basis& b, const Fragments& fr)
             const int nt = A.L + B.L + 1;
             std::vector<std::vector<double>> cf(nm);    // per member: all primitive pairs' coefficients
             std::vector<std::vector<double>> big(nm);   // and each one's largest
+            std::vector<std::vector<double>> own(nm);   // the same, (i, j) and (j, i) of one super shell apart
             std::vector<std::vector<char>> has(nm);
             for (int m = 0; m < nm; ++m) {
                 const int la = b.shells[A.shells[m / nb]].L, lb = b.shells[B.shells[m % nb]].L;
                 cf[m].assign((size_t)nq * tc.c[la][lb].ncoef, 0.0);
                 big[m].assign(nq, 0.0);
+                own[m].assign(nq, -1.0);
                 has[m].assign(nq, 0);
             }
             const double ox[3] = {cA.x, cA.y, cA.z}, px[3] = {cB.x, cB.y, cB.z};
@@ -287,9 +289,11 @@ SuperData build_super_data(const Basis& b, const Fragments& fr)
                         const int ia = A.at[m / nb][i], jb = B.at[m % nb][j];
                         const Shell &sa = b.shells[A.shells[m / nb]], &sb = b.shells[B.shells[m % nb]];
                         if (ia < 0 || jb < 0 || (same && A.shells[m / nb] < B.shells[m % nb])) continue;
-                        ++has[m][q];
+                        const bool folded = has[m][q] != 0;   // the second order of one Gaussian
+                        has[m][q] = 1;
                         const TeamClass& k = tc.c[sa.L][sb.L];
                         double* c = cf[m].data() + (size_t)q * k.ncoef;
+                        double mx = 0.0;
                         for (int a = 0; a < ncart(sa.L); ++a)
                             for (int g = 0; g < ncart(sb.L); ++g) {
                                 int ax, ay, az, bx, by, bz;
@@ -298,12 +302,18 @@ SuperData build_super_data(const Basis& b, const Fragments& fr)
                                 const double w = sa.w[(size_t)a * sa.nprim() + ia] * sb.w[(size_t)g * sb.nprim() + jb];
                                 for (int t = 0; t <= ax + bx; ++t)
                                     for (int u = 0; u <= ay + by; ++u)
-                                        for (int v = 0; v <= az + bz; ++v, ++c)
-                                            *c += w * e(0, ax, bx, t) * e(1, ay, by, u) * e(2, az, bz, v);
+                                        for (int v = 0; v <= az + bz; ++v, ++c) {
+                                            const double x = w * e(0, ax, bx, t) * e(1, ay, by, u) * e(2, az, bz, v);
+                                            mx = std::max(mx, std::fabs(x));
+                                            *c += x;
+                                        }
                             }
-                        c -= k.ncoef;
-                        double mx = 0.0;
-                        for (int x = 0; x < k.ncoef; ++x) mx = std::max(mx, std::fabs(c[x]));
+                        own[m][i * (int)B.exps.size() + j] = mx;
+                        if (folded) {
+                            c -= k.ncoef;
+                            mx = 0.0;
+                            for (int x = 0; x < k.ncoef; ++x) mx = std::max(mx, std::fabs(c[x]));
+                        }
                         big[m][q] = mx;
                     }
                 }
@@ -359,16 +369,21 @@ SuperData build_super_data(const Basis& b, const Fragments& fr)
                 const TeamClass& k = tc.c[b.shells[A.shells[m / nb]].L][b.shells[B.shells[m % nb]].L];
                 o.tab[m] = (int)o.tab.size();
                 o.tab[2 * nm + m] = (int)o.coef.size();
-                int n = 0;
                 for (int q : seq) {
                     if (!has[m][q]) continue;
-                    n += has[m][q];
                     o.tab.push_back(place[q]);
                     o.coef.insert(o.coef.end(), cf[m].begin() + (size_t)q * k.ncoef,
                                   cf[m].begin() + (size_t)(q + 1) * k.ncoef);
                     ++o.tab[nm + m];
                 }
-                if (!same || A.shells[m / nb] >= B.shells[m % nb]) o.npp.push_back(n);
+                if (!same || A.shells[m / nb] >= B.shells[m % nb]) {
+                    // primitive pairs of the shell pair by itself, as build_pair_data keeps them
+                    double mx = 0.0;
+                    for (double v : own[m]) mx = std::max(mx, v);
+                    int n = 0;
+                    for (double v : own[m]) n += v >= 0.0 && v >= kPrimPairCut * mx;
+                    o.npp.push_back(n);
+                }
             }
         }
     });

@@ -169,7 +169,7 @@ struct SuperData {
     int ncls = 0;
     std::vector<std::vector<int>> members;   // per pair: ids of its member shell pairs
     std::vector<std::vector<int>> member_at; // and their member numbers
-    std::vector<std::vector<int>> member_npp;   // and their primitive pairs, (i, j) and (j, i) of one shell counted apart
+    std::vector<std::vector<int>> member_npp;   // and the primitive pairs of each shell pair by itself (build statistics)
     std::vector<int> pbase;             // per molecule: first super pair
     int maxL = 0;
 };
