@@ -225,21 +225,18 @@ void Job::init(const hfx_options& opt)
     auto t1 = tnow();
     compute_schwarz();
     auto t2 = tnow();
-    {
-        const int F = frags_.count();
-        std::vector<int> fk(F);
-        std::vector<long long> fm(F);
-        for (int f = 0; f < F; ++f) {
-            fk[f] = frags_.K(f);
-            fm[f] = frags_.moff[f];
-        }
-        d_fk_.upload(fk, stream_);
-        d_fmoff_.upload(fm, stream_);
-        if (packed_) {
-            std::vector<unsigned char> on(F, 1);
-            d_active_.upload(on, stream_);
-        }
+    // read by the uploads until the plan's synchronisation
+    const int F = frags_.count();
+    std::vector<int> fk(F);
+    std::vector<long long> fm(F);
+    const std::vector<unsigned char> on(F, 1);
+    for (int f = 0; f < F; ++f) {
+        fk[f] = frags_.K(f);
+        fm[f] = frags_.moff[f];
     }
+    d_fk_.upload(fk, stream_);
+    d_fmoff_.upload(fm, stream_);
+    if (packed_) d_active_.upload(on, stream_);
     auto t3 = tnow();
     build_jk_groups(false, gs_fp64_);
     auto t4 = tnow();
@@ -1727,8 +1724,9 @@ void Job::eri_unique(double thr, double* out)
     d_out.alloc(nq);
     cuda_check(cudaMemsetAsync(d_out.p, 0, nq * sizeof(double), stream_), "memset");
     // every super quartet whose bound can pass the BF-level test
+    const TeamPlanHost host = build_team_plan(sup_, qsup_, thr, nsm_);
     TeamPlanDev plan;
-    plan.upload(build_team_plan(sup_, qsup_, thr, nsm_), nsm_, stream_);
+    plan.upload(host, nsm_, stream_);
     run_team(plan, kTeamEri, thr, d_out.p);
     cuda_check(cudaMemcpyAsync(out, d_out.p, nq * sizeof(double), cudaMemcpyDeviceToHost, stream_), "D2H");
     cuda_check(cudaStreamSynchronize(stream_), "eri_unique");

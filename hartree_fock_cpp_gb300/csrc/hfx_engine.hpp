@@ -72,6 +72,9 @@ struct DevBuf {
         p = static_cast<T*>(pool_alloc(count * sizeof(T)));
         n = count;
     }
+    // The copy may still read v when this returns (pageable memory that the
+    // GPU reaches directly is not staged): v lives until the stream is waited for.
+    void upload(std::vector<T>&&, cudaStream_t) = delete;
     void upload(const std::vector<T>& v, cudaStream_t st)
     {
         alloc(v.size());
@@ -163,6 +166,7 @@ struct TeamPlanDev {
     std::vector<KernelSpec> specs;    // per group, kept: an eager build would query the occupancy 40 times
     DevBuf<TeamTask> tasks;
     DevBuf<int> order;
+    void upload(TeamPlanHost&&, int, cudaStream_t) = delete;   // as DevBuf::upload
     void upload(const TeamPlanHost& h, int nsm, cudaStream_t st);
     void make_specs(int nsm);
 };

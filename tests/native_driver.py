@@ -8,14 +8,15 @@ LIB_DIR = os.path.join(REPO, "hartree_fock_cpp_gb300")
 INCLUDE = ["-I", os.path.join(LIB_DIR, "csrc"), "-I", os.path.join(REPO, "include"), "-I", "/usr/local/cuda/include"]
 
 
-def compile_driver(source, path):
-    """Build `source` to the executable `path`; returns the compiler's result."""
+def compile_driver(source, path, link=True):
+    """Build `source` to the executable `path` (link=False: to an object);
+    returns the compiler's result."""
     src = str(path) + ".cpp"
     with open(src, "w") as f:
         f.write(source)
-    return subprocess.run(["g++", "-std=c++17", "-O1", "-o", str(path), src] + INCLUDE +
-                          ["-L", LIB_DIR, "-lhfx", "-Wl,-rpath," + LIB_DIR, "-Wl,--allow-shlib-undefined", "-lpthread"],
-                          capture_output=True, text=True)
+    cmd = ["g++", "-std=c++17", "-O1", "-o", str(path), src] + INCLUDE
+    cmd += ["-L", LIB_DIR, "-lhfx", "-Wl,-rpath," + LIB_DIR, "-Wl,--allow-shlib-undefined", "-lpthread"] if link else ["-c"]
+    return subprocess.run(cmd, capture_output=True, text=True)
 
 
 def run_driver(source, path, *args):
