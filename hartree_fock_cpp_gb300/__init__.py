@@ -180,8 +180,9 @@ class FockBuilder:
         check(lib.hfx_set_launch_shape(self._job, ctypes.byref(s)))
 
     def autotune_launch_shape(self, P, builds=2):
-        """Coordinate search over the launch shape at density P; the job keeps
-        the fastest.  Returns (shape dict, best build ms)."""
+        """Coordinate search over the launch shape of a mixed-precision job's
+        FP32 launches at density P; the job keeps the fastest (an FP64 job its
+        own).  Returns (shape dict, best build ms)."""
         P = self._mat(P)
         s = _lib.LaunchShape()
         ms = ctypes.c_double()

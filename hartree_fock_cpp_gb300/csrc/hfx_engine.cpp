@@ -1540,15 +1540,16 @@ void Job::set_launch_shape(const hfx_launch_shape& s)
         s.warp_max_warps < 1 || s.warp_max_warps > 8 || s.lane_min_npp < 0)
         throw Error(HFX_ERR_INVALID, "launch shape out of range");
     shape_ = s;
-    build_jk_groups(false, gs_fp64_);
-    if (mixed()) build_jk_groups(true, gs_mixed_);
+    if (!mixed()) return;   // the shape is the FP32 launches'
+    build_jk_groups(true, gs_mixed_);
     d_counters_.alloc(std::max<size_t>(1, std::max(gs_fp64_.launches(), gs_mixed_.launches())));
 }
 
 // Coordinate search over the launch shape: for each parameter in turn (small
 // chunk, warp chunk, warps per CTA, lane-mode threshold), try its candidates with the others held,
-// keep the fastest; each trial times the job's own plan (mixed when the job
-// is mixed) at density P on the device, the best of `builds` builds.
+// keep the fastest; each trial times the job's mixed plan at density P on the
+// device, the best of `builds` builds.  An FP64 job has nothing to search: its
+// builds are timed once and its shape stays.
 double Job::autotune_launch_shape(const double* P, int builds, hfx_launch_shape* out)
 {
     const size_t n = (size_t)nmat();
@@ -1569,6 +1570,10 @@ double Job::autotune_launch_shape(const double* P, int builds, hfx_launch_shape*
     };
     hfx_launch_shape cur = shape_;
     double cur_ms = trial(cur);
+    if (!mixed()) {
+        if (out) *out = cur;
+        return cur_ms;
+    }
     static const int small_c[] = {64, 128, 256, 512, 1024};
     static const int warp_c[] = {1024, 2048, 4096, 8192, 16384};
     static const int wpc_c[] = {2, 4, 8};

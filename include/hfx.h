@@ -190,9 +190,10 @@ typedef struct {
 hfx_status hfx_get_launch_shape(const hfx_job *job, hfx_launch_shape *shape);
 hfx_status hfx_set_launch_shape(hfx_job *job, const hfx_launch_shape *shape);
 /* Autotuner: coordinate search over the four parameters, timing the job's
- * own plan (mixed when the job is mixed) at density P (host K x K) with the
- * best of `builds` device builds per trial; the job keeps the fastest shape.
- * best_ms: its kernel time. */
+ * mixed plan at density P (host K x K) with the best of `builds` device builds
+ * per trial; the job keeps the fastest shape.  An FP64 job keeps its shape,
+ * which none of its launches use, and times its builds with it.  best_ms: the
+ * kernel time. */
 hfx_status hfx_autotune_launch_shape(hfx_job *job, const double *P, int builds, hfx_launch_shape *shape,
                                      double *best_ms);
 
