@@ -20,10 +20,10 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <mutex>
 #include <vector>
 
 #include "hfx_engine.hpp"
+#include "hfx_smem.hpp"
 
 namespace hfx {
 
@@ -126,23 +126,6 @@ __global__ void __launch_bounds__(kGridThreads) k_grid_eval(GridArgs a)
     }
 }
 
-cudaError_t allow_grid_smem()
-{
-    static std::mutex mu;
-    static bool done = false;
-    std::lock_guard<std::mutex> lk(mu);
-    if (done) return cudaSuccess;
-    int dev = 0, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaFuncAttributes fa{};
-    cudaError_t e = cudaFuncGetAttributes(&fa, k_grid_eval);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_grid_eval, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
-    if (e == cudaSuccess) done = true;
-    return e;
-}
-
 size_t grid_smem_limit()
 {
     int dev = 0, optin = 0;
@@ -171,7 +154,7 @@ void grid_eval(const Basis& b, int device, const double* M, int column, const do
         exps.insert(exps.end(), s.exps.begin(), s.exps.end());
         w.insert(w.end(), s.w.begin(), s.w.end());
     }
-    cuda_check(allow_grid_smem(), "grid kernel attribute");
+    cuda_check(allow_max_smem((const void*)k_grid_eval), "grid kernel attribute");
     cudaStream_t st;
     cuda_check(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
     try {

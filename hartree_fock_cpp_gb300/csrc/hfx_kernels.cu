@@ -6,6 +6,7 @@
 #include <algorithm>
 
 #include "hfx_engine.hpp"
+#include "hfx_smem.hpp"
 
 namespace hfx {
 
@@ -124,5 +125,21 @@ __global__ void k_rebase_tasks(Task* t, long long n, int delta)
 KernelSpec rebase_tasks_spec(long long n) { return elementwise_spec((const void*)k_rebase_tasks, n, 1); }
 KernelSpec add_spec(long long n) { return elementwise_spec((const void*)k_add, n, 1); }
 KernelSpec to_float_spec(long long n) { return elementwise_spec((const void*)k_to_float, n, 1); }
+
+cudaError_t allow_max_smem(const void* kernel)
+{
+    static OncePerDevice raised;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return raised.run(dev, kernel, [&] {
+        int optin = 0;
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        cudaFuncAttributes fa{};
+        const cudaError_t g = cudaFuncGetAttributes(&fa, kernel);
+        if (g != cudaSuccess) return g;
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
+    });
+}
 
 }  // namespace hfx

@@ -26,10 +26,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <mutex>
-#include <set>
 
 #include "hfx_class.cuh"
+#include "hfx_smem.hpp"
 #include "hfx_team.hpp"
 
 namespace hfx {
@@ -878,24 +877,6 @@ __global__ void k_team_density(const SuperPair* pairs, int npairs, const double*
     Dsh[p] = m;
 }
 
-// Largest dynamic shared memory for a kernel, raised once per process.
-cudaError_t allow_smem(const void* f)
-{
-    static std::mutex mu;
-    static std::set<const void*> done;
-    std::lock_guard<std::mutex> lk(mu);
-    if (done.count(f)) return cudaSuccess;
-    int dev = 0, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaFuncAttributes fa{};
-    cudaError_t e = cudaFuncGetAttributes(&fa, f);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
-    if (e == cudaSuccess) done.insert(f);
-    return e;
-}
-
 template <int TEAM>
 const void* team_kernel(int L)
 {
@@ -948,7 +929,7 @@ cudaError_t team_spec(const TeamGroup& g, int nsm, KernelSpec* s)
     s->func = g.team == 32 ? team_kernel<32>(g.L) : team_kernel<128>(g.L);
     s->block = dim3((unsigned)g.team);
     s->smem = team_header(g.L) + sizeof(double) * (size_t)g.slice;
-    cudaError_t e = allow_smem(s->func);
+    cudaError_t e = allow_max_smem(s->func);
     if (e != cudaSuccess) return e;
     int per = 1;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, s->func, g.team, s->smem);

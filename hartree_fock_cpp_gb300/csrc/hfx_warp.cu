@@ -18,10 +18,8 @@
 // recursion over m of integrals.hpp:541-618, driven by a neighbour table.
 #include <cuda_runtime.h>
 
-#include <mutex>
-#include <set>
-
 #include "hfx_device.cuh"
+#include "hfx_smem.hpp"
 
 namespace hfx {
 
@@ -470,32 +468,12 @@ int warp_slice_elems(int l0b, int l1b, int l0k, int l1k, int npp_ket, int lane_m
     return nab * ncd + w_nh(L1) * ncd + r;
 }
 
-// Raise a kernel's dynamic shared-memory limit to the device maximum once
-// per process: launches from concurrent jobs then never race on the attribute.
-template <typename K>
-static cudaError_t allow_max_smem(K kern)
-{
-    static std::mutex mu;
-    static std::set<const void*> done;
-    std::lock_guard<std::mutex> lk(mu);
-    if (done.count((const void*)kern)) return cudaSuccess;
-    int dev = 0, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaFuncAttributes fa{};
-    cudaError_t err = cudaFuncGetAttributes(&fa, kern);
-    if (err != cudaSuccess) return err;
-    err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
-    if (err == cudaSuccess) done.insert((const void*)kern);
-    return err;
-}
-
 template <typename T>
 static cudaError_t warp_spec_t(int nk, int grid, int warps_per_cta, int slice, KernelSpec* s)
 {
     auto pick = [&](auto kern) -> cudaError_t {
         s->func = (const void*)kern;
-        return allow_max_smem(kern);
+        return allow_max_smem(s->func);
     };
     cudaError_t e = nk == 2 ? pick(k_warp_quartet<T, 2>)  : pick(k_warp_quartet<T, 1>);
     s->grid = dim3((unsigned)grid);

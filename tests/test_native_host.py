@@ -17,3 +17,23 @@ def test_upload_refuses_a_temporary(tmp_path, call, kept):
                                      tmp_path / "prog", link=False)
     assert (r.returncode == 0) == kept, r.stderr
     assert kept or "deleted" in r.stderr
+
+
+def test_shared_memory_limit_is_raised_once_per_device_and_kernel(tmp_path):
+    """A second device needs its own limit; a failed attempt is repeated."""
+    out = native_driver.run_driver(r"""
+#include <cstdio>
+#include "hfx_smem.hpp"
+int main()
+{
+    hfx::OncePerDevice once;
+    int a, b, calls = 0;
+    auto ok = [&] { ++calls; return cudaSuccess; };
+    auto bad = [&] { ++calls; return cudaErrorInvalidValue; };
+    std::printf("%d ", once.run(0, &a, bad) != cudaSuccess);
+    for (int dev : {0, 0, 1, 1, 0})
+        for (const void* k : {(const void*)&a, (const void*)&b}) once.run(dev, k, ok);
+    std::printf("%d\n", calls);
+}
+""", tmp_path / "prog")
+    assert out.split() == ["1", "5"]
