@@ -302,8 +302,8 @@ hfx_status hfx_debug_packed_pairs(const hfx_molecule *mols, int n, int *npairs, 
  * FP64 team kernel), bra and ket pair class (class kernels) or compiled total
  * angular momentum (-1: general) and threads per team (team kernel), fp32,
  * tasks, algorithmic flops (team kernel: estimated instructions), primitive
- * quartets (team kernel: 0), grid, shared-memory slice, warps per CTA (warp
- * kernel).
+ * quartets (team kernel: 0), grid, shared-memory slice and warps per CTA (warp
+ * and team kernels).
  * Pass rows = NULL to get ngroups.  No counterpart in the reference. */
 hfx_status hfx_debug_plan(const hfx_job *job, int mixed, int *ngroups, double *rows);
 

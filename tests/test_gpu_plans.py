@@ -36,3 +36,11 @@ def test_launch_shape_rebuilds_the_mixed_plan_only(precision, monkeypatch, capfd
             assert shape == dict(small_chunk=100, warp_chunk=2000, warp_max_warps=4, lane_min_npp=10)
         # 8 K^2 products at most, |D| <= 2 / K, FP32 within 1e-6 of an integral below 0.1
         assert np.abs(fb.repulsion_matrix(P) - G).max() < (1.6e-6 * fb.K if mixed else 1e-12)
+
+
+def test_plan_rows_report_the_launches_team_sizes():
+    """NaCl/cc-pVTZ has tasks for teams of one warp and of 128 threads."""
+    with H.FockBuilder(config=W.nacl_scan(8)[3], basis_set="cc-pVTZ") as fb:
+        rows = fb.plan()
+    assert {r["pck"] for r in rows} == {32, 128}
+    assert all(r["kind"] == 2 and r["warps_per_cta"] * 32 == r["pck"] for r in rows)
