@@ -369,10 +369,14 @@ def run_engine(args):
         "fock_builds_per_s": {"fp64": 1e3 / build_ms},
         "eri_rate": {"shell_quartets_per_s": s["quartets"] / (kernel_ms * 1e-3),
                      "primitive_quartets_per_s": s["prim_quartets"] / (kernel_ms * 1e-3),
-                     "shell_quartets_per_build": s["quartets"], "note": "surviving (Schwarz-screened) quartets of one FP64 build"},
+                     "shell_quartets_per_build": s["quartets"], "note": "surviving (Schwarz-screened) shell quartets of one FP64 build; the primitive "
+                             "quartets are those evaluated, each distinct one of shells with common exponents once"},
         "roofline": {"bound": "fp64_pipe", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak, "traffic": None,
                      "peak_source": "measured FP64 FMA-loop peak of this GPU (hfx_measure_peaks, same run)",
+                     "note": "achieved counts the algorithmic flops of every surviving shell quartet by itself; the kernel "
+                             "evaluates the primitive quartets that shells share once, so frac is no share of pipe "
+                             "time and passes 1",
                      "flops_per_launch": flops, "kernel_ms": kernel_ms, "fp32_peak_tflops": fp32_peak / 1e3,
                      "dmma_peak_tflops": dmma_peak / 1e3 if dmma_peak else None},
         "e2e": {"value": whole_job_rate(1, e2e_t, ws), "unit": UNIT, "h2d_bytes_per_step": h2d,
@@ -473,8 +477,8 @@ def mixed_section(H, W, torch, flush, args, local, scf_kw, peaks):
              "scf_iterations_fp64": r64["iterations"], "scf_iterations_mixed": rmx["iterations"],
              "scf_fock_ms_fp64": r64["fock_ms"], "scf_fock_ms_mixed": rmx["fock_ms"],
              "scf_builds_mixed_fp64_delta": [rmx["mixed_builds"], rmx["fp64_builds"], rmx["delta_builds"]],
-             # pipe-time fraction of the mixed build's quartet kernels:
-             # (F64 / peak64 + F32 / peak32) / elapsed
+             # algorithmic flops over the pipes' peaks, (F64 / peak64 + F32 / peak32) / elapsed:
+             # not a share of pipe time, the FP64 kernel executes fewer than F64
              "roofline": {"bound": "fp64+fp32 pipes", "flops_fp64": smx["flops_fp64"], "flops_fp32": smx["flops_fp32"],
                           "kernel_ms": kms_mx, "peak_fp64_tflops": peaks[0] / 1e3, "peak_fp32_tflops": peaks[1] / 1e3,
                           "frac": (smx["flops_fp64"] / (peaks[0] * 1e9) + smx["flops_fp32"] / (peaks[1] * 1e9))

@@ -528,7 +528,7 @@ hfx_status hfx_debug_plan(const hfx_job* job, int mixed, int* ngroups, double* r
             const TeamGroup& x = team[g];
             double* r = rows + 10 * (groups.size() + g);
             r[0] = 2; r[1] = x.L; r[2] = x.team; r[3] = 0; r[4] = (double)x.n;
-            r[5] = x.cost; r[6] = 0; r[7] = job->job->team_grid(mixed != 0, g); r[8] = x.slice; r[9] = x.team / 32;
+            r[5] = x.cost; r[6] = x.prims; r[7] = job->job->team_grid(mixed != 0, g); r[8] = x.slice; r[9] = x.team / 32;
         }
     });
 }

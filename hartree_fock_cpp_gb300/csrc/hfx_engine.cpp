@@ -808,15 +808,15 @@ std::shared_ptr<DevBuf<double>> team_boys_device(int device, cudaStream_t st)
     return t;
 }
 
-// Surviving shell quartets, their primitive quartets and algorithmic flops,
-// counted per class pair on bounds sorted in decreasing order (every quartet
+// Surviving shell quartets and their algorithmic flops (each shell quartet by
+// itself, whatever its kernel shares), counted per class pair on bounds sorted in decreasing order (every quartet
 // is one unordered pair of a molecule's shell pairs with Q_X Q_Y >= thr).
 void Job::count_quartets(GroupSet& gs) const
 {
     const double thr = opt_.screening_threshold;
     constexpr int kPC = (kMaxL + 1) * (kMaxL + 2) / 2;
     double quartets = 0.0;
-    gs.prims = gs.flops64 = 0.0;
+    gs.flops64 = 0.0;
     for (int fr = 0; fr < frags_.count(); ++fr) {
         struct Entry {
             double q, npp;
@@ -856,7 +856,6 @@ void Job::count_quartets(GroupSet& gs) const
                     pr *= 0.5;
                 }
                 quartets += n;
-                gs.prims += pr;
                 gs.flops64 += pr * flops_per_prim(l0[a], l1[a], l0[b], l1[b]);
             }
     }
@@ -885,6 +884,9 @@ void Job::build_jk_groups(bool mixed, GroupSet& gs)
     const double thr = opt_.screening_threshold, tau = opt_.fp32_threshold;
     TeamPlanHost tp = build_team_plan(sup_, qsup_, mixed ? std::max(thr, tau) : thr, nsm_);
     gs.team.upload(tp, nsm_, stream_);
+    gs.prims = 0.0;
+    for (const LaunchGroup& g : gs.groups) gs.prims += g.prims;
+    for (const TeamGroup& g : tp.groups) gs.prims += g.prims;
     cuda_check(cudaStreamSynchronize(stream_), "plan upload");
     if (std::getenv("HFX_TRACE_SETUP"))
         std::fprintf(stderr, "team plan (%s): %zu tasks, %zu launches, %.1f ms\n", mixed ? "mixed" : "fp64",

@@ -342,7 +342,7 @@ void FockSession::combine_team(bool mixed_plan, Combined& c)
         TeamGroup cg = *kv.second.front().g;
         cg.off = off;
         cg.n = 0;
-        cg.cost = 0.0;
+        cg.cost = cg.prims = 0.0;
         for (const Part& p : kv.second) {
             long long n = (long long)p.g->n;
             TeamTask* t = c.team.tasks.p + off;
@@ -356,6 +356,7 @@ void FockSession::combine_team(bool mixed_plan, Combined& c)
             off += (size_t)n;
             cg.n += p.g->n;
             cg.cost += p.g->cost;
+            cg.prims += p.g->prims;
             cg.slice = std::max(cg.slice, p.g->slice);
         }
         c.team.groups.push_back(cg);

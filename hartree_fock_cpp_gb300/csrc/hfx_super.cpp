@@ -522,7 +522,7 @@ Geometry geometry(int L1, int L2, const SuperPair& bra, const SuperPair& ket, in
 }
 
 template <typename U, typename F>
-void group_tasks(TeamPlanHost& plan, const std::vector<U>& units, F&& total_L)
+void group_tasks(TeamPlanHost& plan, const SuperData& sd, const std::vector<U>& units, F&& total_L)
 {
     // launch groups: (compiled L, team, slice tier); tasks by decreasing cost
     static const int tiers[] = {1024, 1536, 2048, 3072, 4096, 5120, 8192, 12800, 28000};
@@ -561,7 +561,11 @@ void group_tasks(TeamPlanHost& plan, const std::vector<U>& units, F&& total_L)
         g.cost = std::get<0>(e);
         std::vector<double> cost(refs.size());
         for (size_t x = 0; x < refs.size(); ++x) cost[x] = units[refs[x].unit].cost[refs[x].at];
-        for (size_t x : order_by_cost_desc(cost)) plan.tasks.push_back(units[refs[x].unit].t[refs[x].at]);
+        for (size_t x : order_by_cost_desc(cost)) {
+            const TeamTask& t = units[refs[x].unit].t[refs[x].at];
+            g.prims += (double)(t.i1 - t.i0) * sd.pairs[t.ket].npp;
+            plan.tasks.push_back(t);
+        }
         plan.groups.push_back(g);
     }
 }
@@ -751,7 +755,7 @@ TeamPlanHost build_team_plan(const SuperData& sd, const std::vector<double>& q, 
             }
         });
     }, threads);
-    group_tasks(plan, units, [&](const Unit& u) { return cL[u.cb] + cL[u.ck]; });
+    group_tasks(plan, sd, units, [&](const Unit& u) { return cL[u.cb] + cL[u.ck]; });
     return plan;
 }
 
@@ -813,7 +817,7 @@ TeamPlanHost build_team_diagonal(const SuperData& sd, int nsm)
         }
         plan.first.push_back(out);
     }
-    group_tasks(plan, units, [](const Unit& u) { return u.L; });
+    group_tasks(plan, sd, units, [](const Unit& u) { return u.L; });
     return plan;
 }
 

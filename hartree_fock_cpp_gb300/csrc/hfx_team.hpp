@@ -153,7 +153,8 @@ struct TeamGroup {
     int team;            // threads per team, one team per CTA
     int slice;           // doubles per team
     size_t off, n;
-    double cost;
+    double cost;         // estimated FP64 instructions
+    double prims;        // primitive quartets whose R the tasks compute
 };
 
 // Host image of a job's super pairs.

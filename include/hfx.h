@@ -161,9 +161,12 @@ typedef struct {
     double kernel_ms;         /* device time of the shell-quartet kernel launches alone */
     double quartets;          /* surviving shell quartets */
     double quartets_fp32;     /* of which computed in FP32 */
-    double prim_quartets;     /* primitive quartets evaluated */
-    double flops_fp64;        /* algorithmic flops (MD count) done in FP64 */
-    double flops_fp32;        /* algorithmic flops done in FP32 */
+    double prim_quartets;     /* primitive quartets that the plan's tasks evaluate: in FP64 each
+                                 distinct one of shells with common exponents once */
+    double flops_fp64;        /* algorithmic flops (MD count) of the shell quartets done in FP64,
+                                 each by itself: more than the kernel executes, which shares the
+                                 primitive quartets of shells with common exponents */
+    double flops_fp32;        /* the same count of the shell quartets done in FP32 */
     int launches;             /* kernel launches of the build */
     int reserved[7];
 } hfx_build_stats;
@@ -302,7 +305,7 @@ hfx_status hfx_debug_packed_pairs(const hfx_molecule *mols, int n, int *npairs, 
  * FP64 team kernel), bra and ket pair class (class kernels) or compiled total
  * angular momentum (-1: general) and threads per team (team kernel), fp32,
  * tasks, algorithmic flops (team kernel: estimated instructions), primitive
- * quartets (team kernel: 0), grid, shared-memory slice and warps per CTA (warp
+ * quartets evaluated, grid, shared-memory slice and warps per CTA (warp
  * and team kernels).
  * Pass rows = NULL to get ngroups.  No counterpart in the reference. */
 hfx_status hfx_debug_plan(const hfx_job *job, int mixed, int *ngroups, double *rows);

@@ -44,3 +44,23 @@ def test_plan_rows_report_the_launches_team_sizes():
         rows = fb.plan()
     assert {r["pck"] for r in rows} == {32, 128}
     assert all(r["kind"] == 2 and r["warps_per_cta"] * 32 == r["pck"] for r in rows)
+
+
+# Primitive pairs of the super pairs of a first-row atom in cc-pVDZ, whose s
+# shells share nine exponents, the p shells four, and the d shell has one: the
+# pair of a super shell with itself holds every unordered pair once.
+CCPVDZ_ATOM = [45, 36, 10, 9, 4, 1]
+
+
+@pytest.mark.parametrize("config,basis,pairs", [([("C", (0.1, 0.0, -0.2))], "cc-pVDZ", CCPVDZ_ATOM),
+                                                ([("H", (0.0, 0.0, 0.0)), ("H", (0.0, 0.0, 1.4))], "6-31G",
+                                                 [6, 1, 6, 1, 3, 3, 9, 3, 3, 1])], ids=["shared", "separate"])
+def test_primitive_quartets_are_those_evaluated(config, basis, pairs):
+    """Without a screen every unordered pair of super pairs is evaluated, each
+    on all its primitive quartets."""
+    with H.FockBuilder(config=config, basis_set=basis, screening_threshold=-1.0) as fb:
+        fb.repulsion_matrix(_density(fb.K, 2))
+        s, rows = fb.stats(), fb.plan()
+    n = np.array(pairs)
+    assert s["prim_quartets"] == (n.sum() ** 2 + (n * n).sum()) // 2
+    assert s["prim_quartets"] == sum(r["prims"] for r in rows)
