@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <cmath>
 #include <condition_variable>
 #include <cstring>
 #include <deque>
@@ -256,19 +257,51 @@ private:
         std::strncpy(o->message, j.message.c_str(), sizeof(o->message) - 1);
     }
 
-    // device bytes a job will hold: pair data and records, quartet lists,
-    // J/K and SCF work matrices
-    static size_t estimate_footprint(const Basis& b)
+    // Device bytes that a job will hold, its share of a Fock session included:
+    // pair tables, task lists and work matrices; the tables and matrices twice
+    // for the allocator's power-of-two blocks.  Surviving shell quartets are
+    // counted with exp(-mu R^2) of the outermost primitives for a shell pair's
+    // bound, e^-5 below the threshold: 1.05-1.9 times those of a plan (trees of
+    // 7-60 heavy atoms and alkanes, STO-3G to cc-pVTZ).  A FP32 list holds one
+    // 16-byte task each, an FP64 list one of 32 bytes per eight (5-13%
+    // measured); a session copies both.  Held and estimated: tree of 24, K = 520,
+    // mixed UHF 5.6 and 7.8 GB (4.8 GB its FP32 list); tree of 16, K = 292, 0.55
+    // and 0.9 GB.
+    static size_t estimate_footprint(const Basis& b, int nspin, bool mixed, const hfx_scf_options& scf, bool packed)
     {
-        size_t K = b.K, prims = 0, pairs = 0;
-        for (size_t x = 0; x < b.shells.size(); ++x)
+        const ClassTables& ct = class_tables();
+        const size_t K = b.K, ns = b.shells.size();
+        const double thr = scf.screening_threshold == 0.0 ? 1e-8 : scf.screening_threshold;
+        const double reach = thr > 0.0 ? 5.0 - std::log(thr) : INFINITY;
+        size_t tables = 0;
+        std::vector<double> decay;   // -log of the pairs' bounds, those within reach
+        for (size_t x = 0; x < ns; ++x)
             for (size_t y = 0; y <= x; ++y) {
-                ++pairs;
-                prims += (size_t)b.shells[x].nprim() * b.shells[y].nprim();
+                const Shell &s0 = b.shells[x], &s1 = b.shells[y];
+                const int l0 = std::max(s0.L, s1.L), l1 = std::min(s0.L, s1.L);
+                const PairClassTab& t = ct.tab[l0 * (l0 + 1) / 2 + l1];
+                const size_t per = 8 * (size_t)(kTeamHdr + t.ncoef) + 4 + (mixed ? 4 * (size_t)t.stride : 0);
+                tables += (size_t)s0.nprim() * s1.nprim() * per + sizeof(SuperPair) + sizeof(DPair);
+                const double a = *std::min_element(s0.exps.begin(), s0.exps.end());
+                const double c = *std::min_element(s1.exps.begin(), s1.exps.end());
+                const double R2 = (s0.x - s1.x) * (s0.x - s1.x) + (s0.y - s1.y) * (s0.y - s1.y) + (s0.z - s1.z) * (s0.z - s1.z);
+                const double d = a * c / (a + c) * R2;
+                if (d < reach) decay.push_back(d);
             }
-        const size_t per_prim_pair = 8 * (4 + 100) * 2 + 8 * 36 * 35;    // records (64+32 bit) + dense E bound
-        const size_t tasks = pairs * pairs / 2 * 12 / 4;                  // screened list, generous
-        return prims * per_prim_pair + tasks + 8 * K * K * 64 + (size_t(64) << 20);
+        std::sort(decay.begin(), decay.end());
+        double quartets = 0.0;       // pairs of pairs X <= Y with decay X + decay Y < reach
+        for (size_t x = 0, n = decay.size(); x < decay.size(); ++x) {
+            while (n > 0 && decay[x] + decay[n - 1] >= reach) --n;
+            if (n > x) quartets += (double)(n - x);
+        }
+        const double lists = quartets * (mixed ? 16.0 + 4.0 : 4.0) * (packed ? 2.0 : 1.0);
+        // K x K matrices: J/K accumulators (kAccCopies in a mixed build), the
+        // build's staging and float densities, the SCF step, its projector and
+        // eigensolver, the DIIS ring
+        const size_t build = (nspin + 1) * (mixed ? kAccCopies : 1) + 4 * nspin + 2, step = 15 + 14 * nspin;
+        const size_t history = scf.max_history > 0 ? scf.max_history : 8;
+        const size_t matrices = build + step + 2 * nspin * history;
+        return 2 * (tables + 8 * K * K * matrices) + (size_t)lists + (size_t(64) << 20);
     }
 
     void worker()
@@ -383,7 +416,8 @@ private:
                              j->basis_path.empty() ? nullptr : j->basis_path.c_str()};
             Basis b = build_basis(mol);
             j->K = b.K;
-            size_t fp = estimate_footprint(b);
+            const int nspin = j->method == 1 ? 2 : 1;
+            size_t fp = estimate_footprint(b, nspin, j->precision == HFX_PREC_MIXED, j->scf, opt_.pack_max > 1);
             if (j->inject_fault == HFX_FAULT_OOM) fp = budget_ + 1;
             reserve(*j, fp);
             if (j->inject_fault == HFX_FAULT_ALLOC) throw Error(HFX_ERR_OOM, "injected allocation failure");
@@ -394,7 +428,6 @@ private:
             o.device = opt_.device;
             Job job(b, o);
             ScfSetup setup = scf_setup(b, true);
-            const int nspin = j->method == 1 ? 2 : 1;
             const double deadline = j->timeout_s > 0 ? j->t_submit + j->timeout_s : 0.0;
             ScfControl ctl{&j->cancel, deadline, j->inject_fault == HFX_FAULT_ITERATION ? 3 : 0};
             ScfOutput out;
