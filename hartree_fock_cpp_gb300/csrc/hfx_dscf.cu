@@ -69,11 +69,11 @@ struct Coef8 {
     const double* m[8];
     int n;
 };
-// C = sum_i c_i M_i
-__global__ void k_lincomb(int n, Coef8 cf, double* C)
+// C = sum_i c_i M_i, added to C where `add` is set
+__global__ void k_lincomb(int n, Coef8 cf, int add, double* C)
 {
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        double s = 0.0;
+        double s = add ? C[e] : 0.0;
         for (int i = 0; i < cf.n; ++i) s += cf.c[i] * cf.m[i][e];
         C[e] = s;
     }
@@ -446,7 +446,11 @@ ScfOutput DeviceScf::run(const Basis& b, const ScfSetup& setup, const hfx_scf_op
             ++out.delta_builds;
         }
     };
-    double sc[32];
+    // scalars of an iteration: norms and energies, from 16 on the new row of B
+    const int nscal = 16 + 2 * std::max(8, maxh);
+    scal_.alloc(std::max(64, nscal));
+    std::vector<double> scalars(nscal);
+    double* sc = scalars.data();
     double E_prev = 0.0;
     int n_it = 0;
     std::vector<double> Pswap;
@@ -479,7 +483,7 @@ ScfOutput DeviceScf::run(const Basis& b, const ScfSetup& setup, const hfx_scf_op
         for (size_t q = 0; q < ring.size(); ++q)
             for (int s = 0; s < nspin_; ++s)
                 add_dot(kDot, hEs[s], hE[ring[q] * nspin_ + s].p, nullptr, 16 + 2 * (int)q + s);
-        fetch(sc, 32);
+        fetch(sc, 16 + 2 * std::max(8, (int)ring.size()));
         const double E_cur = 0.5 * (sc[10] + (nspin_ == 2 ? sc[11] : 0.0));
         const double en = std::sqrt(sc[12] + (nspin_ == 2 ? sc[13] : 0.0));
         for (size_t q = 0; q < ring.size(); ++q) {
@@ -500,14 +504,16 @@ ScfOutput DeviceScf::run(const Basis& b, const ScfSetup& setup, const hfx_scf_op
             rhs[hn] = 1.0;
             solve_full_piv(hn + 1, A.data(), rhs.data(), x.data());
             for (int s = 0; s < nspin_; ++s) {
-                Coef8 cf{};
-                cf.n = hn;
-                for (int i = 0; i < hn; ++i) {
-                    cf.c[i] = x[i];
-                    cf.m[i] = hF[ring[i] * nspin_ + s].p;
+                for (int i0 = 0; i0 < hn; i0 += 8) {
+                    Coef8 cf{};
+                    cf.n = std::min(8, hn - i0);
+                    for (int i = 0; i < cf.n; ++i) {
+                        cf.c[i] = x[i0 + i];
+                        cf.m[i] = hF[ring[i0 + i] * nspin_ + s].p;
+                    }
+                    k_lincomb<<<grid_for(n), 256, 0, st_>>>(n, cf, i0 > 0, T2_.p);
+                    cuda_check(cudaGetLastError(), "lincomb");
                 }
-                k_lincomb<<<grid_for(n), 256, 0, st_>>>(n, cf, T2_.p);
-                cuda_check(cudaGetLastError(), "lincomb");
                 // T2_ is reused by error_and_energy; keep the DIIS Fock in E_ (its history copy is saved)
                 cuda_check(cudaMemcpyAsync(E_[s].p, T2_.p, bytes, cudaMemcpyDeviceToDevice, st_), "copy");
                 Fuse[s] = E_[s].p;
