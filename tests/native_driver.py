@@ -19,10 +19,15 @@ def compile_driver(source, path, link=True):
     return subprocess.run(cmd, capture_output=True, text=True)
 
 
+def run_program(path, *args, stdin=None):
+    """The standard output of a built program."""
+    r = subprocess.run([str(path)] + [str(a) for a in args], capture_output=True, text=True, timeout=300, input=stdin)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return r.stdout
+
+
 def run_driver(source, path, *args):
     """Build and run; the program's standard output."""
     c = compile_driver(source, path)
     assert c.returncode == 0, c.stderr
-    r = subprocess.run([str(path)] + [str(a) for a in args], capture_output=True, text=True, timeout=300)
-    assert r.returncode == 0, r.stdout + r.stderr
-    return r.stdout
+    return run_program(path, *args)
