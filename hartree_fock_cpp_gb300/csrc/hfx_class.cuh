@@ -196,8 +196,8 @@ __device__ __forceinline__ void hermite_R(T X, T Y, T Z, const T (&s)[L + 1], T 
     });
 }
 
-// (p, Px, Py, Pz) of a primitive-pair record: one 16-byte load in FP32
-// (records are 16-byte aligned), four loads in FP64
+// (p, Px, Py, Pz) of a primitive-pair record: one 16-byte load (records are
+// 16-byte aligned)
 template <typename T>
 __device__ __forceinline__ void load_header(const T* r, T& p, T& x, T& y, T& z)
 {
@@ -362,12 +362,8 @@ __device__ __forceinline__ void small_quartet(const SmallArgs<T>& a, const Task&
         }
     }
 
-    // digestion (FP64), into the bra pair's molecule's matrices
+    // digestion into the FP64 matrices of the bra pair's molecule
     const int K = bra.kdim;
-    const double* __restrict__ Qbf = a.Qbf + bra.qoff;
-    const double* __restrict__ Dj = a.Dj + bra.moff;
-    const double* __restrict__ Dk = a.Dk + bra.moff;
-    const double* __restrict__ Dk2 = a.Dk2 + (NK == 2 ? bra.moff : 0);
     double* J = a.J + bra.moff;
     double* Kx = a.Kx + bra.moff;
     double* Kx2 = a.Kx2 + (NK == 2 ? bra.moff : 0);
@@ -375,8 +371,8 @@ __device__ __forceinline__ void small_quartet(const SmallArgs<T>& a, const Task&
     // Block digestion: the degeneracy weight is applied in place (0 for
     // the non-canonical and BF-screened elements); then every J / K
     // element the quartet touches is summed over the quartet in registers
-    // (FP32 quartets: float products with the float density copies) and
-    // added to the FP64 accumulators once -- nab + ncd + na nc + na nd +
+    // (float products with the float density copies) and added to the FP64
+    // accumulators once -- nab + ncd + na nc + na nd +
     // nb nc + nb nd atomics per quartet instead of 6 per integral.
     constexpr int NA = c_nc(LA), NC = c_nc(LC);
     const T* __restrict__ QbT = a.Qbf32 + bra.qoff;

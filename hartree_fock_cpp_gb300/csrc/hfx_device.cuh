@@ -53,8 +53,8 @@ __host__ __device__ inline PairGeo make_pairgeo(double p, double x, double y, do
 struct __align__(16) DPair {
     int bf0, bf1;      // first basis function of shell 0 / shell 1
     int l0, l1;        // l0 >= l1
-    int pp0, npp;      // primitive-pair range
-    long long e_off;   // offset of the first dense E block (elements)
+    int pp0, npp;      // primitive pairs: the first one's geometry (host image only), their number
+    long long e_off;   // offset of the first dense E block (elements; host image only)
     int same;          // shell 0 == shell 1
     int id;            // pair id (index in the pair array)
     double qmax;       // max_ab sqrt((ab|ab)) over the pair's BF pairs
@@ -143,23 +143,18 @@ struct SmallArgs {
     int ntasks;
     const T* boys;
     double thr;
-    const double* Qbf;
-    int K;
-    const double* Dj;
-    const double* Dk;
-    const double* Dk2;
     double* J;
     double* Kx;
     double* Kx2;
     const double* Dsh;         // per shell pair max |D| (density screening), or null
     double dthr;               // skip a quartet when Q_AB Q_CD max|D| < dthr (0: never)
     const unsigned char* active;   // packed jobs: per molecule, 0 = skip its quartets (null: all)
-    // FP32 kernels: float copies of Dj / Dk / Dk2 for the block digestion
+    // float copies of the densities for the block digestion
     const float* Dj32;
     const float* Dk32;
     const float* Dk232;
-    // FP32 kernels: float copy of the BF-pair Schwarz bounds (the digestion's
-    // screen then needs no FP64 arithmetic); addressed with bra.qoff
+    // float copy of the BF-pair Schwarz bounds (the digestion's screen then
+    // needs no FP64 arithmetic); addressed with bra.qoff
     const float* Qbf32;
     // copies of the accumulators: a CTA adds to copy blockIdx.x % ncopy, copy
     // c at c * cstride elements
@@ -181,11 +176,6 @@ struct WarpArgs {
     int* counter;
     const T* boys;             // per-L rows of kBoys32Row floats
     double thr;
-    const double* Qbf;
-    int K;
-    const double* Dj;
-    const double* Dk;
-    const double* Dk2;
     double* J;
     double* Kx;
     double* Kx2;
@@ -194,12 +184,12 @@ struct WarpArgs {
     const double* Dsh;         // per shell pair max |D| (density screening), or null
     double dthr;               // skip a quartet when Q_AB Q_CD max|D| < dthr (0: never)
     const unsigned char* active;   // packed jobs: per molecule, 0 = skip its quartets (null: all)
-    // FP32 kernels: float copies of Dj / Dk / Dk2 for the block digestion
+    // float copies of the densities for the block digestion
     const float* Dj32;
     const float* Dk32;
     const float* Dk232;
-    // FP32 kernels: float copy of the BF-pair Schwarz bounds (the digestion's
-    // screen then needs no FP64 arithmetic); addressed with bra.qoff
+    // float copy of the BF-pair Schwarz bounds (the digestion's screen then
+    // needs no FP64 arithmetic); addressed with bra.qoff
     const float* Qbf32;
     // copies of the accumulators: a CTA adds to copy blockIdx.x % ncopy, copy
     // c at c * cstride elements

@@ -423,7 +423,7 @@ void host_parallel_for(int n, const std::function<void(int)>& f, int most)
     if (err) std::rethrow_exception(err);
 }
 
-PairData build_pair_data(const Basis& basis, const Fragments& fr)
+PairData build_pair_data(const Basis& basis, const Fragments& fr, bool dense)
 {
     const ClassTables& ct = class_tables();
     const auto& sh = basis.shells;
@@ -440,6 +440,7 @@ PairData build_pair_data(const Basis& basis, const Fragments& fr)
     struct PairOut {
         std::vector<PairGeo> geo;
         std::vector<double> epool, rec;
+        int npp = 0;
     };
     std::vector<PairOut> outs(items.size());
     constexpr int kPairsPerUnit = 16;
@@ -455,8 +456,8 @@ PairData build_pair_data(const Basis& basis, const Fragments& fr)
             const int n0 = ncart(l0), n1 = ncart(l1), H = nherm(L);
             const PairClassTab& pt = ct.tab[pair_class(l0, l1)];
             const int nt = L + 1;
-            // All primitive pairs of the shell pair first (geometry, dense E
-            // block, record coefficients), then only those whose largest
+            // All primitive pairs of the shell pair first (geometry, record
+            // coefficients, dense E block where asked for), then only those whose largest
             // Hermite->Cartesian coefficient reaches kPrimPairCut of the shell
             // pair's largest: the others (tight primitives on distant centres,
             // exp(-mu |AB|^2) ~ 0) change no integral by more than ~1e-14 of
@@ -464,7 +465,7 @@ PairData build_pair_data(const Basis& basis, const Fragments& fr)
             // from every class kernel.
             const int np = S0.nprim() * S1.nprim();
             const size_t ne = (size_t)n0 * n1 * H;
-            std::vector<double> pgeo((size_t)np * 4), pe((size_t)np * ne, 0.0), pc((size_t)np * pt.ncoef), pmax(np, 0.0);
+            std::vector<double> pgeo((size_t)np * 4), pe(dense ? (size_t)np * ne : 0, 0.0), pc((size_t)np * pt.ncoef), pmax(np, 0.0);
             std::vector<int> pnc(np, 0);
             double cmax_pair = 0.0;
             for (int i = 0; i < S0.nprim(); ++i)
@@ -488,14 +489,14 @@ PairData build_pair_data(const Basis& basis, const Fragments& fr)
                             int bx, by, bz;
                             component(l1, c1, bx, by, bz);
                             const double w = S0.w[(size_t)c0 * S0.nprim() + i] * S1.w[(size_t)c1 * S1.nprim() + j];
-                            double* row = pe.data() + (size_t)q * ne + (size_t)(c0 * n1 + c1) * H;
+                            double* row = dense ? pe.data() + (size_t)q * ne + (size_t)(c0 * n1 + c1) * H : nullptr;
                             for (int t = 0; t <= ax + bx; ++t)
                                 for (int u2 = 0; u2 <= ay + by; ++u2)
                                     for (int v = 0; v <= az + bz; ++v) {
                                         const double c = w * Ex[((size_t)ax * (l1 + 1) + bx) * nt + t] *
                                                          Ey[((size_t)ay * (l1 + 1) + by) * nt + u2] *
                                                          Ez[((size_t)az * (l1 + 1) + bz) * nt + v];
-                                        row[herm_index(t, u2, v)] = c;
+                                        if (dense) row[herm_index(t, u2, v)] = c;
                                         cq[nc++] = c;
                                         cmax = std::max(cmax, std::fabs(c));
                                     }
@@ -508,8 +509,11 @@ PairData build_pair_data(const Basis& basis, const Fragments& fr)
             PairOut& o = outs[it];
             for (int q = 0; q < np; ++q) {
                 if (pmax[q] < kPrimPairCut * cmax_pair) continue;
-                o.geo.push_back(make_pairgeo(pgeo[4 * q], pgeo[4 * q + 1], pgeo[4 * q + 2], pgeo[4 * q + 3]));
-                o.epool.insert(o.epool.end(), pe.begin() + (size_t)q * ne, pe.begin() + (size_t)(q + 1) * ne);
+                ++o.npp;
+                if (dense) {
+                    o.geo.push_back(make_pairgeo(pgeo[4 * q], pgeo[4 * q + 1], pgeo[4 * q + 2], pgeo[4 * q + 3]));
+                    o.epool.insert(o.epool.end(), pe.begin() + (size_t)q * ne, pe.begin() + (size_t)(q + 1) * ne);
+                }
                 const size_t rb = o.rec.size();
                 o.rec.resize(rb + pt.stride, 0.0);
                 o.rec[rb] = pgeo[4 * q];
@@ -550,7 +554,7 @@ PairData build_pair_data(const Basis& basis, const Fragments& fr)
         hp.same = (A == B);
         hp.pp0 = (int)pd.geo.size();
         hp.e_off = (long long)pd.epool.size();
-        hp.npp = (int)o.geo.size();
+        hp.npp = o.npp;
         const long long rec_off = (long long)pd.rec.size();
         pd.geo.insert(pd.geo.end(), o.geo.begin(), o.geo.end());
         pd.epool.insert(pd.epool.end(), o.epool.begin(), o.epool.end());
@@ -587,7 +591,7 @@ PairData build_pair_data(const Basis& basis, const Fragments& fr)
 // Shell-pair records of the FP32 launches; built for mixed-precision jobs.
 void Job::build_pairs()
 {
-    PairData pd = build_pair_data(basis_, frags_);
+    PairData pd = build_pair_data(basis_, frags_, false);
     // The FP32 tasks are tiles of the records, which their kernels index
     // without a check: the list of shell pairs takes the records' counts.  The
     // super pairs fold both orders of two shells' common exponents and keep
@@ -630,7 +634,6 @@ TeamArgs Job::team_args(const TeamPlanDev& plan, const TeamGroup& g, int* counte
     a.ridx = reinterpret_cast<const uint4*>(d_sridx_.p);
     std::copy(team_ridx().at, team_ridx().at + 49, a.ridx_at);
     a.boys = team_boys_->p;
-    a.slice = g.slice;
     return a;
 }
 
@@ -1280,7 +1283,6 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
     const std::vector<LaunchGroup>& groups = gs.groups;
     const Task* tasks = gs.tasks.p;
     const double* Dsh = nullptr;
-    int K = basis_.K;
     const unsigned char* active = d_active_.p;
     const double* Tsh = nullptr;
     if (dthr > 0.0 && !groups.empty()) {
@@ -1361,14 +1363,14 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
             const int lane = naux - next_aux;
             next_aux = (next_aux + 1) % (naux + 1 - kFp64Lanes);
             SmallArgs<float> a{d_pairs_.p, d_rec32_.p, tasks + g.off, (int)g.n, d_boys32_.p, opt_.screening_threshold,
-                               d_qbf_.p, K, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, d_qbf32_.p, ncopy, cstride};
+                               J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, d_qbf32_.p, ncopy, cstride};
             cuda_check(small_spec_f32(g.pcb, g.pck, nk, (int)g.n, &ks), "small-class kernel");
             void* prm[] = {&a};
             sk.kernel(lane, ks, prm);
         } else {
             cuda_check(warp_spec(nk, g.grid, g.warps_per_cta, g.slice, &ks), "warp kernel");
             WarpArgs<float> a{d_pairs_.p, d_rec32_.p, d_pct_.p, d_abs_.p, d_kh_.p, d_kl_.p, tasks + g.off, (int)g.n,
-                              ctr + gi, d_boys32_.p, opt_.screening_threshold, d_qbf_.p, K, Dj, Dk, Dk2, J, Kx, Kx2,
+                              ctr + gi, d_boys32_.p, opt_.screening_threshold, J, Kx, Kx2,
                               g.slice, g.lane_min_npp, Dsh, dthr, active, Dj32, Dk32, Dk232,
                               d_qbf32_.p, ncopy, cstride};
             void* prm[] = {&a};

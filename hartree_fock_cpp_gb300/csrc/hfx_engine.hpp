@@ -142,7 +142,9 @@ struct Fragments {
 Basis concat_basis(const std::vector<Basis>& mols, Fragments& fr);
 Fragments single_fragment(const Basis& b);
 
-PairData build_pair_data(const Basis& b, const Fragments& fr);
+// Records of the FP32 kernels; `dense`: also the primitive pairs' geometry and
+// dense E blocks (hfx_debug_pair_data).
+PairData build_pair_data(const Basis& b, const Fragments& fr, bool dense = true);
 // Primitive-pair counts of `pd`'s records into a list of the same shell pairs.
 void take_record_counts(std::vector<HostPair>& pairs, const PairData& pd);
 

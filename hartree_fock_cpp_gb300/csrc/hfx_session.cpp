@@ -461,7 +461,6 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
         a.Dsh = Tsh;
         a.active = active;
         a.nk = nk;
-        a.slice = g.slice;
         void* prm[] = {&a};
         sk.kernel((int)(gi % (c.groups.empty() ? naux + 1 : kFp64Lanes)), c.team.specs[gi], prm);
     }
@@ -472,15 +471,15 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
         if (g.kind == 0) {
             const int lane = naux - next_aux;
             next_aux = (next_aux + 1) % (naux + 1 - kFp64Lanes);
-            SmallArgs<float> a{pairs32_.p, anchor32_.p, tasks + g.off, (int)g.n, boys32_.p, thr_, nullptr,
-                               0, Dj, Dk, Dk2, J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p, 1, 0};
+            SmallArgs<float> a{pairs32_.p, anchor32_.p, tasks + g.off, (int)g.n, boys32_.p, thr_,
+                               J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p, 1, 0};
             cuda_check(small_spec_f32(g.pcb, g.pck, nk, (int)g.n, &ks), "session small-class kernel");
             void* prm[] = {&a};
             sk.kernel(lane, ks, prm);
         } else {
             cuda_check(warp_spec(nk, g.grid, g.warps_per_cta, g.slice, &ks), "session warp kernel");
             WarpArgs<float> a{pairs32_.p, anchor32_.p, pct_.p, abs_.p, kh_.p, kl_.p, tasks + g.off, (int)g.n,
-                              ctr + gi, boys32_.p, thr_, nullptr, 0, Dj, Dk, Dk2, J, Kx, Kx2, g.slice,
+                              ctr + gi, boys32_.p, thr_, J, Kx, Kx2, g.slice,
                               g.lane_min_npp, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p, 1, 0};
             void* prm[] = {&a};
             sk.kernel(naux, ks, prm);
@@ -492,6 +491,8 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
     const int* fk = fk_.p;
     const long long* fm = fmoff_.p;
     const int nf = (int)live_.size();
+    // one copy of the accumulators: more were measured on single jobs only
+    // (kAccCopies), not on a session's merged launches
     int ncopy = 1;
     long long cstride = 0;
     if (nk == 1) {

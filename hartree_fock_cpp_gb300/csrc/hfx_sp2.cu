@@ -28,8 +28,6 @@ constexpr int kThreads = 256;       // 64 outputs x 4 slices of the inner dimens
 constexpr double kIdemTol = 1e-10;
 constexpr double kTraceTol = 1e-6;  // tr(D) = nocc: otherwise no gap (fractional occupation)
 
-// Gershgorin bounds of sym(F) = (F + F^T) / 2, one warp per row:
-// bounds[0] = min_i (f_ii - r_i), bounds[1] = max_i (f_ii + r_i).
 // The projections of one run (blockIdx.y).
 struct Sp2Set {
     const double* F;
@@ -42,6 +40,8 @@ struct Sp2Sets {
     Sp2Set s[2];
 };
 
+// Gershgorin bounds of sym(F) = (F + F^T) / 2, one warp per row:
+// bounds[0] = min_i (f_ii - r_i), bounds[1] = max_i (f_ii + r_i).
 __global__ void __launch_bounds__(1024) k_sp2_bounds(int n, Sp2Sets sets)
 {
     const double* __restrict__ F = sets.s[blockIdx.y].F;

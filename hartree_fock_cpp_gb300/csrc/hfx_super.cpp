@@ -226,7 +226,6 @@ SuperData build_super_data(const Basis& b, const Fragments& fr)
         d.nA = A.nfn;
         d.nB = B.nfn;
         d.L = A.L + B.L;
-        sd.maxL = std::max(sd.maxL, d.L);
         d.same = x == y;
         d.kdim = fr.K(it.f);
         d.frag = it.f;

@@ -21,12 +21,14 @@
 
 namespace hfx {
 
-// Most functions of a super shell of several shells (a single shell may have
-// up to ten, f): bounds the Cartesian block of a quartet to 36 x 36, 10 KB of
-// shared memory.
+// Most functions of a super shell of several shells: the Cartesian block of a
+// quartet of such is at most 36 x 36, 10 KB of shared memory.  A single shell
+// may have up to ten functions (f): 100 x 100, 80 KB, in slices of up to 19452
+// doubles (152 KB, NaCl/cc-pVTZ).
 constexpr int kSuperMaxFn = 6;
 
-// Primitive-pair header: p, Px, Py, Pz, sqrt(2 pi^{5/2}) / p, unused.
+// Primitive-pair header: p, Px, Py, Pz, sqrt(2 pi^{5/2}) / p, and a word that
+// keeps its three 16-byte loads aligned.
 constexpr int kTeamHdr = 6;
 
 // Boys table of the team kernel: one row of 8 doubles per (L, k), T_k = k/64:
@@ -111,7 +113,6 @@ struct TeamArgs {
     double* out;            // kTeamDiag: partial sums; kTeamEri: packed integrals
     int nk;                 // exchange matrices (1 or 2)
     int mixed;              // leave out the member quartets below the pairs' cut32: FP32 launches have them
-    int slice;              // shared-memory slice per team, doubles
 };
 
 __host__ __device__ constexpr int team_nherm(int L) { return (L + 1) * (L + 2) * (L + 3) / 6; }
@@ -172,7 +173,6 @@ struct SuperData {
     std::vector<std::vector<int>> member_at; // and their member numbers
     std::vector<std::vector<int>> member_npp;   // and the primitive pairs of each shell pair by itself (build statistics)
     std::vector<int> pbase;             // per molecule: first super pair
-    int maxL = 0;
 };
 
 // Per coefficient of the 16 ordered (la, lb) classes, concatenated: packed

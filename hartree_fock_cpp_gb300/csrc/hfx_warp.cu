@@ -365,18 +365,14 @@ __global__ void __launch_bounds__(256) k_warp_quartet(WarpArgs<T> a)
             __syncwarp();
         }
 
-        // digestion (FP64), into the bra pair's molecule's matrices
+        // digestion into the FP64 matrices of the bra pair's molecule
         const int K = bra.kdim;
-        const double* __restrict__ Qbf = a.Qbf + bra.qoff;
-        const double* __restrict__ Dj = a.Dj + bra.moff;
-        const double* __restrict__ Dk = a.Dk + bra.moff;
-        const double* __restrict__ Dk2 = a.Dk2 + (NK == 2 ? bra.moff : 0);
         double* J = a.J + bra.moff;
         double* Kx = a.Kx + bra.moff;
         double* Kx2 = a.Kx2 + (NK == 2 ? bra.moff : 0);
         // Block digestion: weights in place (0 for non-canonical and
         // BF-screened elements), then one lane per J / K element the
-        // quartet touches sums its contributions (FP32 quartets: float
+        // quartet touches sums its contributions (float
         // products with the float density copies) and adds the sum to the
         // FP64 accumulator: nab + ncd + na nc + na nd + nb nc + nb nd
         // atomics per quartet instead of 6 per integral.
@@ -475,7 +471,7 @@ static cudaError_t warp_spec_t(int nk, int grid, int warps_per_cta, int slice, K
         s->func = (const void*)kern;
         return allow_max_smem(s->func);
     };
-    cudaError_t e = nk == 2 ? pick(k_warp_quartet<T, 2>)  : pick(k_warp_quartet<T, 1>);
+    cudaError_t e = nk == 2 ? pick(k_warp_quartet<T, 2>) : pick(k_warp_quartet<T, 1>);
     s->grid = dim3((unsigned)grid);
     s->block = dim3((unsigned)(32 * warps_per_cta));
     s->smem = kWarpSmemHeader + sizeof(T) * (size_t)slice * warps_per_cta;
