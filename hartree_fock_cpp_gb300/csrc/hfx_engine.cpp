@@ -1267,6 +1267,46 @@ cudaGraphExec_t GraphSink::instantiate()
     return exec;
 }
 
+void place_launches(OpSink& sk, size_t nteam, const std::vector<LaunchGroup>& groups, int lanes,
+                    const std::function<void(int, bool, size_t)>& put)
+{
+    // class kernels, then warp kernels, each by decreasing work
+    std::vector<size_t> order;
+    double flops = 0.0;
+    for (size_t g = 0; g < groups.size(); ++g) {
+        if (groups[g].n == 0) continue;
+        order.push_back(g);
+        if (groups[g].kind == 0) flops += groups[g].flops;
+    }
+    if (nteam > 0 && !order.empty() && flops < kClassesFirstFlops) {
+        // side by side: FP64, the largest first, on lanes of its own; FP32 on
+        // the others, warp kernels on the last
+        for (size_t g = 0; g < nteam; ++g) put((int)(g % kFp64Lanes), true, g);
+        int next = 0;
+        for (size_t g : order) {
+            if (groups[g].kind != 0) {
+                put(lanes - 1, false, g);
+                continue;
+            }
+            put(lanes - 1 - next, false, g);
+            next = (next + 1) % (lanes - kFp64Lanes);
+        }
+        return;
+    }
+    std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) {
+        return groups[x].kind != groups[y].kind ? groups[x].kind < groups[y].kind : groups[x].flops > groups[y].flops;
+    });
+    int next = 0;
+    size_t x = 0;
+    for (; x < order.size() && groups[order[x]].kind == 0; ++x, next = (next + 1) % lanes) put(next, false, order[x]);
+    if (flops >= kClassesFirstFlops && (nteam > 0 || x < order.size())) {
+        sk.join();
+        sk.fork();
+    }
+    for (size_t g = 0; g < nteam; ++g) put((int)(g % lanes), true, g);
+    for (; x < order.size(); ++x, next = (next + 1) % lanes) put(next, false, order[x]);
+}
+
 int Job::acc_copies(bool mixed_plan) const
 {
     return plan(mixed_plan).groups.empty() ? 1 : kAccCopies;
@@ -1332,36 +1372,29 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
     int* ctr = counters ? counters : d_counters_.p;
     sk.zero(0, ctr, sizeof(int) * std::max<size_t>(1, gs.launches()));
     sk.fork();
-    const int naux = (int)aux_.size();
-    // FP64: the team kernel's launches, the largest first
-    const int n64 = groups.empty() ? naux + 1 : kFp64Lanes;
-    for (size_t gi = 0; gi < gs.team.groups.size(); ++gi) {
-        const TeamGroup& g = gs.team.groups[gi];
-        TeamArgs a = team_args(gs.team, g, ctr + groups.size() + gi);
-        a.mode = kTeamFock;
-        a.mixed = mixed_plan && mixed();
-        a.Dj = Dj;
-        a.Dk = Dk;
-        a.Dk2 = Dk2;
-        a.J = J;
-        a.Kx = Kx;
-        a.Kx2 = Kx2;
-        a.Dsh = Tsh;
-        team_thresholds(a, opt_.screening_threshold, dthr);
-        a.active = active;
-        a.nk = nk;
-        void* prm[] = {&a};
-        sk.kernel((int)(gi % n64), gs.team.specs[gi], prm);
-    }
-    // FP32: on the lanes left, warp groups on the last
-    int next_aux = 0;
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
+    place_launches(sk, gs.team.groups.size(), groups, 1 + (int)aux_.size(), [&](int lane, bool fp64, size_t gi) {
+        if (fp64) {
+            const TeamGroup& g = gs.team.groups[gi];
+            TeamArgs a = team_args(gs.team, g, ctr + groups.size() + gi);
+            a.mode = kTeamFock;
+            a.mixed = mixed_plan && mixed();
+            a.Dj = Dj;
+            a.Dk = Dk;
+            a.Dk2 = Dk2;
+            a.J = J;
+            a.Kx = Kx;
+            a.Kx2 = Kx2;
+            a.Dsh = Tsh;
+            team_thresholds(a, opt_.screening_threshold, dthr);
+            a.active = active;
+            a.nk = nk;
+            void* prm[] = {&a};
+            sk.kernel(lane, gs.team.specs[gi], prm);
+            return;
+        }
         const LaunchGroup& g = groups[gi];
-        if (g.n == 0) continue;
         KernelSpec ks;
         if (g.kind == 0) {
-            const int lane = naux - next_aux;
-            next_aux = (next_aux + 1) % (naux + 1 - kFp64Lanes);
             SmallArgs<float> a{d_pairs_.p, d_rec32_.p, tasks + g.off, (int)g.n, d_boys32_.p, opt_.screening_threshold,
                                J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, d_qbf32_.p, ncopy, cstride};
             cuda_check(small_spec_f32(g.pcb, g.pck, nk, (int)g.n, &ks), "small-class kernel");
@@ -1374,9 +1407,9 @@ void Job::launch_jk(OpSink& sk, int nk, const double* Dj, const double* Dk, cons
                               g.slice, g.lane_min_npp, Dsh, dthr, active, Dj32, Dk32, Dk232,
                               d_qbf32_.p, ncopy, cstride};
             void* prm[] = {&a};
-            sk.kernel(naux, ks, prm);
+            sk.kernel(lane, ks, prm);
         }
-    }
+    });
     sk.join();
 }
 

@@ -247,6 +247,23 @@ private:
     std::vector<std::vector<cudaGraphNode_t>> deps_;   // per lane: the nodes its next node depends on
 };
 
+// FP32 class kernels of a build with at least this many algorithmic flops run
+// before everything that uses shared memory.  They live on the L1 cache, whose
+// size an SM sets by the shared memory of what it runs and changes only when it
+// is idle: beside FP64 or warp CTAs they keep the small one to their end. Beside
+// / before, ms, mixed builds at the FP32 cut given: tree of 12 heavy atoms,
+// cc-pVDZ UHF 0.1 (6e11 flops) 45.6 / 31.9, tree of 16, 6-31G* UHF 0.1 (1.5e11)
+// 18.1 / 13.9, tree of 12, 6-31G* UHF 0.1 (8e10) 9.9 / 8.1.  Below it the overlap
+// of both pipes is worth as much: benzene/cc-pVDZ RHF 0.03 (2e10) 4.76 / 4.95,
+// n-decane/6-31G* RHF 0.1 (2.4e10) 2.85 / 2.63, NaCl/6-31G* RHF 0.03 (4e8) 0.34 / 0.36.
+constexpr double kClassesFirstFlops = 4e10;
+
+// Issues the launches of a build, which has forked, on `lanes` lanes, the lane
+// chosen for each: put(lane, true, i) for the i-th FP64 launch, put(lane, false,
+// i) for the i-th FP32 one.
+void place_launches(OpSink& sk, size_t nteam, const std::vector<LaunchGroup>& groups, int lanes,
+                    const std::function<void(int, bool, size_t)>& put);
+
 // What the device SCF needs from a Fock builder: a job of its own, or one
 // molecule's share of a packed job (hfx_batch.cpp).  Builds are synchronous
 // with respect to stream().

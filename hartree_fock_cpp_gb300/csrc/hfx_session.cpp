@@ -436,41 +436,38 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
     sk.zero(0, ctr, sizeof(int) * std::max<size_t>(1, c.launches()));
     sk.fork();
     const Task* tasks = c.tasks.p;
-    const int naux = (int)aux_.size();
-    for (size_t gi = 0; gi < c.team.groups.size(); ++gi) {
-        const TeamGroup& g = c.team.groups[gi];
-        TeamArgs a{};
-        a.pairs = super_.p;
-        a.order = c.team.order.p;
-        a.tasks = c.team.tasks.p + g.off;
-        a.ntasks = (int)g.n;
-        a.counter = ctr + c.groups.size() + gi;
-        a.kcode = scode_.p;
-        a.ridx = reinterpret_cast<const uint4*>(sridx_.p);
-        std::copy(team_ridx().at, team_ridx().at + 49, a.ridx_at);
-        a.boys = team_boys_->p;
-        team_thresholds(a, thr_, dthr);
-        a.mode = kTeamFock;
-        a.mixed = mixed_plan;
-        a.Dj = Dj;
-        a.Dk = Dk;
-        a.Dk2 = Dk2;
-        a.J = J;
-        a.Kx = Kx;
-        a.Kx2 = Kx2;
-        a.Dsh = Tsh;
-        a.active = active;
-        a.nk = nk;
-        void* prm[] = {&a};
-        sk.kernel((int)(gi % (c.groups.empty() ? naux + 1 : kFp64Lanes)), c.team.specs[gi], prm);
-    }
-    int next_aux = 0;
-    for (size_t gi = 0; gi < c.groups.size(); ++gi) {
+    place_launches(sk, c.team.groups.size(), c.groups, 1 + (int)aux_.size(), [&](int lane, bool fp64, size_t gi) {
+        if (fp64) {
+            const TeamGroup& g = c.team.groups[gi];
+            TeamArgs a{};
+            a.pairs = super_.p;
+            a.order = c.team.order.p;
+            a.tasks = c.team.tasks.p + g.off;
+            a.ntasks = (int)g.n;
+            a.counter = ctr + c.groups.size() + gi;
+            a.kcode = scode_.p;
+            a.ridx = reinterpret_cast<const uint4*>(sridx_.p);
+            std::copy(team_ridx().at, team_ridx().at + 49, a.ridx_at);
+            a.boys = team_boys_->p;
+            team_thresholds(a, thr_, dthr);
+            a.mode = kTeamFock;
+            a.mixed = mixed_plan;
+            a.Dj = Dj;
+            a.Dk = Dk;
+            a.Dk2 = Dk2;
+            a.J = J;
+            a.Kx = Kx;
+            a.Kx2 = Kx2;
+            a.Dsh = Tsh;
+            a.active = active;
+            a.nk = nk;
+            void* prm[] = {&a};
+            sk.kernel(lane, c.team.specs[gi], prm);
+            return;
+        }
         const LaunchGroup& g = c.groups[gi];
         KernelSpec ks;
         if (g.kind == 0) {
-            const int lane = naux - next_aux;
-            next_aux = (next_aux + 1) % (naux + 1 - kFp64Lanes);
             SmallArgs<float> a{pairs32_.p, anchor32_.p, tasks + g.off, (int)g.n, boys32_.p, thr_,
                                J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p, 1, 0};
             cuda_check(small_spec_f32(g.pcb, g.pck, nk, (int)g.n, &ks), "session small-class kernel");
@@ -482,9 +479,9 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
                               ctr + gi, boys32_.p, thr_, J, Kx, Kx2, g.slice,
                               g.lane_min_npp, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p, 1, 0};
             void* prm[] = {&a};
-            sk.kernel(naux, ks, prm);
+            sk.kernel(lane, ks, prm);
         }
-    }
+    });
     sk.join();
     int kmax = 0;
     for (int s : live_) kmax = std::max(kmax, slots_[s].job->K());

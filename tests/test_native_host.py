@@ -37,3 +37,52 @@ int main()
 }
 """, tmp_path / "prog")
     assert out.split() == ["1", "5"]
+
+
+def test_every_launch_of_a_build_is_placed_once(tmp_path):
+    """Side by side below the threshold, FP64 and FP32 on lanes of their own;
+    from there on the FP32 class kernels by decreasing work before a join, then
+    the launches that use shared memory; one kind alone on every lane."""
+    out = native_driver.run_driver(r"""
+#include <cstdio>
+#include "hfx_engine.hpp"
+struct Sink final : hfx::OpSink {
+    void zero(int, void*, size_t) override {}
+    void kernel(int, const hfx::KernelSpec&, void**) override {}
+    void fork() override { std::printf("fork "); }
+    void join() override { std::printf("join "); }
+};
+int main()
+{
+    for (double flops : {1e9, hfx::kClassesFirstFlops})
+        for (int team : {0, 13})
+            for (int fp32 = 0; fp32 < 3; ++fp32) {    // none, class kernels, class and warp kernels
+                std::vector<hfx::LaunchGroup> g;
+                for (int k = 0; k < 6 * (fp32 > 0); ++k) {
+                    hfx::LaunchGroup x{};
+                    x.kind = fp32 == 2 && k % 3 == 2;
+                    x.n = k == 4 ? 0 : 1;
+                    x.flops = x.kind ? 1e15 : flops * (k + 1) / 2.0;
+                    g.push_back(x);
+                }
+                Sink sk;
+                hfx::place_launches(sk, team, g, 12, [&](int lane, bool fp64, size_t i) {
+                    std::printf("%s%zu@%d ", fp64 ? "t" : g[i].kind ? "w" : "c", i, lane);
+                });
+                std::printf("\n");
+            }
+}
+""", tmp_path / "prog")
+    team = ["t%d@%%d" % i for i in range(13)]
+    apart = [t % (i % 12) for i, t in enumerate(team)]
+    beside = [t % (i % 8) for i, t in enumerate(team)]
+    small, large = out.splitlines()[:6], out.splitlines()[6:]
+    cls = ["c5@0", "c3@1", "c2@2", "c1@3", "c0@4"]
+    mix = ["c3@0", "c1@1", "c0@2"]
+    assert [x.split() for x in small] == [
+        [], cls, mix + ["w2@3", "w5@4"],
+        apart, beside + ["c0@11", "c1@10", "c2@9", "c3@8", "c5@11"],
+        beside + ["c0@11", "c1@10", "w2@11", "c3@9", "w5@11"]]
+    assert [x.split() for x in large] == [
+        [], cls, mix + ["join", "fork", "w2@3", "w5@4"],
+        apart, cls + ["join", "fork"] + apart, mix + ["join", "fork"] + apart + ["w2@3", "w5@4"]]
