@@ -15,9 +15,7 @@ SCF solve from a zero density.
          measured FP64 FMA-loop peak, and the reference-algorithm CPU baseline
          timed on this host's cores on a bounded sample.
 
---impl reference times the reference's CPU algorithm for the same workload
-(oracle port of integrals.hpp repulsion_tensor + linalg.hpp repulsion_matrix,
-all host threads, bounded sample per step, extrapolated to solves/s).
+--impl reference prints why the reference cannot be run beside the engine.
 Multi-GPU: replicas only (one independent solve stream per rank), launched
 with torchrun; value = solves of all ranks / max time.
 """
@@ -166,17 +164,6 @@ def cpu_baseline(config, basis, iterations, sample_quartets, nthreads, seed=2026
                 seconds_per_solve=t_solve, sample_seconds=t_sample + t_contract + t_schwarz)
 
 
-def load_workloads():
-    """The synthetic workload generators, loaded from their file (numpy only):
-    importing the package would load the engine's library into the process."""
-    import importlib.util
-    spec = importlib.util.spec_from_file_location("hfx_workloads",
-                                                  os.path.join(REPO, "hartree_fock_cpp_gb300", "workloads.py"))
-    mod = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(mod)
-    return mod
-
-
 def reference_iterations():
     """SCF iterations of the headline workload in the reference's own loop:
     the oracle's rhf_diis (scf.hpp:205-419) over the tensor of the reference's
@@ -186,41 +173,22 @@ def reference_iterations():
 
 
 def workload_config(K, ws):
-    """The config dict of the headline workload, the same in both arms."""
+    """The config dict of the headline workload."""
     return {"workload": WORKLOAD, "molecule": "benzene D6h (C r=2.6379, H r=4.68 bohr)", "basis": "cc-pVDZ",
             "K": K, "parallelism": "replicas" if ws > 1 else "single",
-            "l2": "GPU arm: flushed between steps (512 MB write)"}
+            "l2": "flushed between steps (512 MB write)"}
 
 
 def run_reference(args):
-    ws, rank, _ = _dist()
-    if rank != 0:
+    """The reference is CMake C++/CUDA on Eigen (not installed here), no package
+    that could be installed beside the engine, and no checkout of it exists on
+    the GPU machine: there is nothing to time.  The engine's own line reports
+    the restated reference algorithm on a sample of quartets, extrapolated
+    (cpu_baseline); that is no run of the reference."""
+    if _dist()[1] != 0:
         return
-    W = load_workloads()
-    nthreads = os.cpu_count() or 1
-    cfg = W.benzene()
-    iters = reference_iterations()
-    vals = []
-    base = None
-    for s in range(args.warmup + args.steps):
-        b = cpu_baseline(cfg, "cc-pVDZ", iters, sample_quartets=2000 * nthreads, nthreads=nthreads,
-                         seed=20261203 + s)
-        if s >= args.warmup:
-            vals.append(b["seconds_per_solve"])
-            base = b
-    t = float(np.mean(vals))
-    v = 1.0 / t
-    line = {"impl": "reference", "metric": METRIC, "value": v, "unit": UNIT, "n_gpus": ws, "steps": args.steps,
-            "warmup": args.warmup, "ms_per_step": t * 1e3, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "f64", "data": "synthetic",
-            "config": workload_config(base["K"], ws),
-            "reference_impl": "reference CPU algorithm (oracle port of integrals.hpp repulsion_tensor + "
-                              "linalg.hpp repulsion_matrix), host threads, %d SCF iterations of the reference "
-                              "loop" % iters,
-            "cpu_baseline": {"value": v, "unit": UNIT, "cores": nthreads, "kind": base["kind"],
-                             "sample": base["sample"]},
-            "e2e": {"value": v, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
-    print(json.dumps(line), flush=True)
+    print(json.dumps({"impl": "reference", "unavailable": "the reference is a CMake C++/CUDA program on Eigen without a "
+                      "Python package, and the GPU machine has neither Eigen nor a checkout of it"}), flush=True)
 
 
 def run_engine(args):
