@@ -191,6 +191,13 @@ def run_reference(args):
                       "Python package, and the GPU machine has neither Eigen nor a checkout of it"}), flush=True)
 
 
+def copied_bytes(_lib):
+    """Bytes that the library has copied to the device and back so far."""
+    h2d, d2h = ctypes.c_double(), ctypes.c_double()
+    _lib.check(_lib.lib.hfx_debug_copied_bytes(ctypes.byref(h2d), ctypes.byref(d2h)))
+    return h2d.value, d2h.value
+
+
 def run_engine(args):
     import torch
     ws, rank, local = _dist()
@@ -298,15 +305,9 @@ def run_engine(args):
         if k > 0:
             e2e_lat.append(dt)
     e2e_t = max_over_ranks(float(np.mean(e2e_lat)), ws)
-    m = H._lib.MoleculeArgs(cfg, basis)
-    npp = ctypes.c_int()
-    npr = ctypes.c_int()
-    nep = ctypes.c_longlong()
-    _lib.check(_lib.lib.hfx_debug_pair_data(m.ref(), ctypes.byref(npp), ctypes.byref(npr), ctypes.byref(nep), None,
-                                            None, None))
-    setup_bytes = nep.value * 8 + npr.value * 32 + npp.value * 48 + s["quartets"] * 8
-    h2d = int(setup_bytes + r["fock_builds"] * K * K * 8)
-    d2h = int(r["fock_builds"] * K * K * 8 + K * (K + 1) // 2 * 8 + npp.value * 8)
+    moved = copied_bytes(_lib)
+    H.rhf_diis(cfg, basis, **scf_kw)
+    h2d, d2h = (int(b - a) for a, b in zip(moved, copied_bytes(_lib)))
 
     if rank != 0:
         if ws > 1:

@@ -150,6 +150,7 @@ SIGNATURES = {
     "hfx_debug_pair_data": (I, [V, P(I), P(I), P(ctypes.c_longlong), V, V, V]),
     "hfx_debug_packed_pairs": (I, [V, I, P(I), V, V]),
     "hfx_debug_plan": (I, [V, I, P(I), V]),
+    "hfx_debug_copied_bytes": (I, [P(D), P(D)]),
     "hfx_one_electron": (I, [V, V, V, V, P(I)]),
     "hfx_one_electron_gpu": (I, [V, I, V, V, V, P(I)]),
     "hfx_grid_density": (I, [V, I, V, V, D, I, V]),

@@ -533,6 +533,11 @@ hfx_status hfx_debug_plan(const hfx_job* job, int mixed, int* ngroups, double* r
     });
 }
 
+hfx_status hfx_debug_copied_bytes(double* h2d, double* d2h)
+{
+    return guarded([&] { copied_bytes(h2d, d2h); });
+}
+
 hfx_status hfx_one_electron(const hfx_molecule* mol, double* S, double* T, double* V, int* K)
 {
     return guarded([&] {

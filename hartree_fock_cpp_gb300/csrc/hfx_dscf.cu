@@ -241,7 +241,7 @@ void DeviceScf::run_dots()
 void DeviceScf::fetch(double* host, int count)
 {
     run_dots();
-    cuda_check(cudaMemcpyAsync(host, scal_.p, sizeof(double) * count, cudaMemcpyDeviceToHost, st_), "D2H scalars");
+    copy_async(host, scal_.p, sizeof(double) * count, cudaMemcpyDeviceToHost, st_, "D2H scalars");
     cuda_check(cudaStreamSynchronize(st_), "scf sync");
 }
 
@@ -408,7 +408,7 @@ ScfOutput DeviceScf::run(const Basis& b, const ScfSetup& setup, const hfx_scf_op
     for (int s = 0; s < nspin_; ++s) {
         const double* p0 = s == 0 ? P0a : P0b;
         if (p0)
-            cuda_check(cudaMemcpyAsync(P_[s].p, p0, bytes, cudaMemcpyHostToDevice, st_), "H2D P0");
+            copy_async(P_[s].p, p0, bytes, cudaMemcpyHostToDevice, st_, "H2D P0");
         else
             cuda_check(cudaMemsetAsync(P_[s].p, 0, bytes, st_), "memset P");
     }
@@ -603,16 +603,16 @@ ScfOutput DeviceScf::run(const Basis& b, const ScfSetup& setup, const hfx_scf_op
         if (proj_[s]) eigensolve(s, nocc[s], occf, false);
     // results to the host: densities, MO energies, coefficients (row-major)
     out.P.resize(n);
-    cuda_check(cudaMemcpyAsync(out.P.data(), P_[0].p, bytes, cudaMemcpyDeviceToHost, st_), "D2H P");
+    copy_async(out.P.data(), P_[0].p, bytes, cudaMemcpyDeviceToHost, st_, "D2H P");
     out.e.resize(K);
-    cuda_check(cudaMemcpyAsync(out.e.data(), e_[0].p, sizeof(double) * K, cudaMemcpyDeviceToHost, st_), "D2H e");
+    copy_async(out.e.data(), e_[0].p, sizeof(double) * K, cudaMemcpyDeviceToHost, st_, "D2H e");
     std::vector<double> Ccm(n);
-    cuda_check(cudaMemcpyAsync(Ccm.data(), C_[0].p, bytes, cudaMemcpyDeviceToHost, st_), "D2H C");
+    copy_async(Ccm.data(), C_[0].p, bytes, cudaMemcpyDeviceToHost, st_, "D2H C");
     if (nspin_ == 2) {
         out.P2.resize(n);
         out.e2.resize(K);
-        cuda_check(cudaMemcpyAsync(out.P2.data(), P_[1].p, bytes, cudaMemcpyDeviceToHost, st_), "D2H P");
-        cuda_check(cudaMemcpyAsync(out.e2.data(), e_[1].p, sizeof(double) * K, cudaMemcpyDeviceToHost, st_), "D2H e");
+        copy_async(out.P2.data(), P_[1].p, bytes, cudaMemcpyDeviceToHost, st_, "D2H P");
+        copy_async(out.e2.data(), e_[1].p, sizeof(double) * K, cudaMemcpyDeviceToHost, st_, "D2H e");
     }
     cuda_check(cudaStreamSynchronize(st_), "scf results");
     out.C.resize(n);

@@ -114,6 +114,20 @@ void cuda_check(cudaError_t e, const char* what)
     }
 }
 
+static std::atomic<unsigned long long> g_copied[2];   // host to device, device to host
+
+void copy_async(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, cudaStream_t st, const char* what)
+{
+    cuda_check(cudaMemcpyAsync(dst, src, bytes, kind, st), what);
+    g_copied[kind == cudaMemcpyDeviceToHost].fetch_add(bytes, std::memory_order_relaxed);
+}
+
+void copied_bytes(double* h2d, double* d2h)
+{
+    if (h2d) *h2d = (double)g_copied[0].load();
+    if (d2h) *d2h = (double)g_copied[1].load();
+}
+
 static double flops_per_prim(int la, int lb, int lc, int ld)
 {
     // algorithmic MD flop count per primitive quartet (boys + R + ket + bra + prefactor)
@@ -142,7 +156,7 @@ Job::Job(const std::vector<Basis>& mols, const hfx_options& opt) : opt_(opt)
 void Job::set_active(const unsigned char* flags)
 {
     if (!d_active_.p) throw Error(HFX_ERR_INVALID, "set_active: not a packed job");
-    cuda_check(cudaMemcpyAsync(d_active_.p, flags, frags_.count(), cudaMemcpyHostToDevice, stream_), "active flags");
+    copy_async(d_active_.p, flags, frags_.count(), cudaMemcpyHostToDevice, stream_, "active flags");
 }
 
 Basis concat_basis(const std::vector<Basis>& mols, Fragments& fr)
@@ -712,7 +726,7 @@ void Job::compute_schwarz()
         cuda_check(cudaLaunchKernel(ks.func, ks.grid, ks.block, prm, 0, stream_), "Schwarz bounds");
     }
     qbf_.resize(npair_bf);
-    cuda_check(cudaMemcpyAsync(qbf_.data(), d_qbf_.p, npair_bf * sizeof(double), cudaMemcpyDeviceToHost, stream_),
+    copy_async(qbf_.data(), d_qbf_.p, npair_bf * sizeof(double), cudaMemcpyDeviceToHost, stream_,
                "download Q");
     cuda_check(cudaStreamSynchronize(stream_), "schwarz");
     // per shell pair, per super pair: the largest
@@ -1162,7 +1176,7 @@ void Job::build_fp32_groups(GroupSet& gs)
     const auto tp4 = std::chrono::steady_clock::now();
     gs.tasks.alloc(total);
     if (total > 0)
-        cuda_check(cudaMemcpyAsync(gs.tasks.p, all.get(), total * sizeof(Task), cudaMemcpyHostToDevice, stream_),
+        copy_async(gs.tasks.p, all.get(), total * sizeof(Task), cudaMemcpyHostToDevice, stream_,
                    "plan upload");
     // the host array is freed on return: the copy must have read it
     cuda_check(cudaStreamSynchronize(stream_), "plan upload");
@@ -1593,7 +1607,7 @@ double Job::autotune_launch_shape(const double* P, int builds, hfx_launch_shape*
     DevBuf<double> dP, dG;
     dP.alloc(n);
     dG.alloc(n);
-    cuda_check(cudaMemcpyAsync(dP.p, P, n * sizeof(double), cudaMemcpyHostToDevice, stream_), "H2D P");
+    copy_async(dP.p, P, n * sizeof(double), cudaMemcpyHostToDevice, stream_, "H2D P");
     builds = std::max(1, std::min(builds, 10));
     auto trial = [&](const hfx_launch_shape& s) {
         set_launch_shape(s);
@@ -1726,9 +1740,9 @@ void Job::fock_rhf_ex(const double* P, double* G, bool mixed_plan, double dthr)
     size_t n = (size_t)nmat();
     d_D_.alloc(n);
     d_out1_.alloc(n);
-    cuda_check(cudaMemcpyAsync(d_D_.p, P, n * sizeof(double), cudaMemcpyHostToDevice, stream_), "H2D");
+    copy_async(d_D_.p, P, n * sizeof(double), cudaMemcpyHostToDevice, stream_, "H2D");
     fock_rhf_device_ex(d_D_.p, d_out1_.p, mixed_plan, dthr);
-    cuda_check(cudaMemcpyAsync(G, d_out1_.p, n * sizeof(double), cudaMemcpyDeviceToHost, stream_), "D2H");
+    copy_async(G, d_out1_.p, n * sizeof(double), cudaMemcpyDeviceToHost, stream_, "D2H");
     cuda_check(cudaStreamSynchronize(stream_), "D2H");
 }
 
@@ -1747,12 +1761,12 @@ void Job::fock_uhf_ex(const double* Pa, const double* Pb, double* J, double* Ka,
     d_out1_.alloc(n);
     d_out2_.alloc(n);
     d_out3_.alloc(n);
-    cuda_check(cudaMemcpyAsync(d_D_.p, Pa, n * sizeof(double), cudaMemcpyHostToDevice, stream_), "H2D");
-    cuda_check(cudaMemcpyAsync(d_D2_.p, Pb, n * sizeof(double), cudaMemcpyHostToDevice, stream_), "H2D");
+    copy_async(d_D_.p, Pa, n * sizeof(double), cudaMemcpyHostToDevice, stream_, "H2D");
+    copy_async(d_D2_.p, Pb, n * sizeof(double), cudaMemcpyHostToDevice, stream_, "H2D");
     fock_uhf_device_ex(d_D_.p, d_D2_.p, d_out1_.p, d_out2_.p, d_out3_.p, mixed_plan, dthr);
-    cuda_check(cudaMemcpyAsync(J, d_out1_.p, n * sizeof(double), cudaMemcpyDeviceToHost, stream_), "D2H");
-    cuda_check(cudaMemcpyAsync(Ka, d_out2_.p, n * sizeof(double), cudaMemcpyDeviceToHost, stream_), "D2H");
-    cuda_check(cudaMemcpyAsync(Kb, d_out3_.p, n * sizeof(double), cudaMemcpyDeviceToHost, stream_), "D2H");
+    copy_async(J, d_out1_.p, n * sizeof(double), cudaMemcpyDeviceToHost, stream_, "D2H");
+    copy_async(Ka, d_out2_.p, n * sizeof(double), cudaMemcpyDeviceToHost, stream_, "D2H");
+    copy_async(Kb, d_out3_.p, n * sizeof(double), cudaMemcpyDeviceToHost, stream_, "D2H");
     cuda_check(cudaStreamSynchronize(stream_), "D2H");
 }
 
@@ -1770,7 +1784,7 @@ void Job::eri_unique(double thr, double* out)
     TeamPlanDev plan;
     plan.upload(host, nsm_, stream_);
     run_team(plan, kTeamEri, thr, d_out.p);
-    cuda_check(cudaMemcpyAsync(out, d_out.p, nq * sizeof(double), cudaMemcpyDeviceToHost, stream_), "D2H");
+    copy_async(out, d_out.p, nq * sizeof(double), cudaMemcpyDeviceToHost, stream_, "D2H");
     cuda_check(cudaStreamSynchronize(stream_), "eri_unique");
 }
 

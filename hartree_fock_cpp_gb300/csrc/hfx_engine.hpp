@@ -39,6 +39,11 @@ const std::vector<float>& boys_table32_host();
 
 void cuda_check(cudaError_t e, const char* what);
 
+// cudaMemcpyAsync between host and device, its bytes counted
+// (hfx_debug_copied_bytes).
+void copy_async(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, cudaStream_t st, const char* what);
+void copied_bytes(double* h2d, double* d2h);
+
 // Caching device allocator: freed blocks (rounded up to a power of two, up to
 // 256 MB) are kept for reuse instead of being returned with cudaFree, whose
 // implicit device synchronisation would stall every other job in flight when
@@ -78,7 +83,7 @@ struct DevBuf {
     void upload(const std::vector<T>& v, cudaStream_t st)
     {
         alloc(v.size());
-        if (!v.empty()) cuda_check(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st), "upload");
+        if (!v.empty()) copy_async(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st, "upload");
     }
 };
 

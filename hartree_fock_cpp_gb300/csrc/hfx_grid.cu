@@ -164,7 +164,7 @@ void grid_eval(const Basis& b, int device, const double* M, int column, const do
         d_exps.upload(exps, st);
         d_w.upload(w, st);
         d_M.alloc((size_t)K * K);
-        cuda_check(cudaMemcpyAsync(d_M.p, M, sizeof(double) * K * K, cudaMemcpyHostToDevice, st), "upload matrix");
+        copy_async(d_M.p, M, sizeof(double) * K * K, cudaMemcpyHostToDevice, st, "upload matrix");
         const long long chunk = std::min<long long>(n, 8LL << 20);   // 64 MB of values per launch
         d_out.alloc((size_t)std::max<long long>(1, chunk));
         if (xyz) d_xyz.alloc((size_t)3 * std::max<long long>(1, chunk));
@@ -179,7 +179,7 @@ void grid_eval(const Basis& b, int device, const double* M, int column, const do
             a.M = d_M.p;
             a.column = column;
             if (xyz) {
-                cuda_check(cudaMemcpyAsync(d_xyz.p, xyz + 3 * f, sizeof(double) * 3 * m, cudaMemcpyHostToDevice, st),
+                copy_async(d_xyz.p, xyz + 3 * f, sizeof(double) * 3 * m, cudaMemcpyHostToDevice, st,
                            "upload points");
                 a.xyz = d_xyz.p;
             }
@@ -198,7 +198,7 @@ void grid_eval(const Basis& b, int device, const double* M, int column, const do
             const unsigned grid = (unsigned)((m + kTile - 1) / kTile);
             k_grid_eval<<<grid, kGridThreads, smem, st>>>(a);
             cuda_check(cudaGetLastError(), "grid kernel");
-            cuda_check(cudaMemcpyAsync(out + f, d_out.p, sizeof(double) * m, cudaMemcpyDeviceToHost, st), "download");
+            copy_async(out + f, d_out.p, sizeof(double) * m, cudaMemcpyDeviceToHost, st, "download");
             cuda_check(cudaStreamSynchronize(st), "grid evaluation");
         }
     } catch (...) {

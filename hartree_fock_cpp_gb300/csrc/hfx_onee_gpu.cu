@@ -338,9 +338,9 @@ void one_electron_gpu(const Basis& b, std::vector<double>& S, std::vector<double
         S.resize(n);
         T.resize(n);
         V.resize(n);
-        cuda_check(cudaMemcpyAsync(S.data(), d_out.p, n * sizeof(double), cudaMemcpyDeviceToHost, st), "download S");
-        cuda_check(cudaMemcpyAsync(T.data(), d_out.p + n, n * sizeof(double), cudaMemcpyDeviceToHost, st), "T");
-        cuda_check(cudaMemcpyAsync(V.data(), d_out.p + 2 * n, n * sizeof(double), cudaMemcpyDeviceToHost, st), "V");
+        copy_async(S.data(), d_out.p, n * sizeof(double), cudaMemcpyDeviceToHost, st, "download S");
+        copy_async(T.data(), d_out.p + n, n * sizeof(double), cudaMemcpyDeviceToHost, st, "T");
+        copy_async(V.data(), d_out.p + 2 * n, n * sizeof(double), cudaMemcpyDeviceToHost, st, "V");
         cuda_check(cudaStreamSynchronize(st), "one-electron");
     } catch (...) {
         cudaStreamSynchronize(st);

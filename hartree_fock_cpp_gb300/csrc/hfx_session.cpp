@@ -531,7 +531,7 @@ void FockSession::run_locked()
                     cuda_check(cudaMemcpyAsync(in_[1].p + m.moff, r->Pb, bytes, cudaMemcpyDeviceToDevice, stream_),
                                "session stage");
             }
-            cuda_check(cudaMemcpyAsync(active_.p, flags.data(), flags.size(), cudaMemcpyHostToDevice, stream_),
+            copy_async(active_.p, flags.data(), flags.size(), cudaMemcpyHostToDevice, stream_,
                        "session flags");
             cuda_check(cudaEventRecord(ev0_, stream_), "event");
             launch(nspin_, kv.first.first, kv.first.second);

@@ -310,6 +310,11 @@ hfx_status hfx_debug_packed_pairs(const hfx_molecule *mols, int n, int *npairs, 
  * Pass rows = NULL to get ngroups.  No counterpart in the reference. */
 hfx_status hfx_debug_plan(const hfx_job *job, int mixed, int *ngroups, double *rows);
 
+/* Measurement hook: bytes that the library has copied from the host to the
+ * device and back since it was loaded, over all jobs and threads (either
+ * pointer may be NULL).  No counterpart in the reference. */
+hfx_status hfx_debug_copied_bytes(double *h2d, double *d2h);
+
 /* One-electron matrices S, T, V of a molecule (integrals.hpp:10-536), host. */
 hfx_status hfx_one_electron(const hfx_molecule *mol, double *S, double *T, double *V, int *K);
 /* The same matrices computed on CUDA device `device` (one CTA per shell pair;
