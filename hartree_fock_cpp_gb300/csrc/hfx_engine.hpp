@@ -196,12 +196,13 @@ struct GroupSet {
 // benzene/cc-pVDZ 8.10 / 7.84, n-decane/6-31G* mixed 3.20 / 3.02.
 constexpr int kAuxLanes = 11, kFp64Lanes = 8;
 // Copies of the J/K accumulators of a build with FP32 launches (a power of
-// two; CTAs spread over them, the symmetrisation adds them up): the FP32
-// kernels send 600 M FP64 reductions to the L2 for a K = 292 molecule, its
-// busiest slices 50-70% occupied and the average one 30%. 1 / 2 / 4 / 8
-// copies, ms: n-decane/6-31G* mixed 3.07 / 2.94 / 2.89 / 2.89, K = 292 tree
-// 18.0 / 17.6 / 17.5 / 17.4. FP64 builds reduce in the kernel first (1-4%) and
-// keep one.
+// two; CTAs spread over them, the symmetrisation adds them up): with one, the
+// reductions of the FP32 kernels crowd in a few L2 slices; with four the
+// busiest is 58-62% occupied and the average one 38-40% in (ps|ss) and (dp|ps)
+// of n-decane/6-31G*.  1 / 2 / 4 / 8 copies, ms: n-decane mixed at an FP32 cut
+// of 0.1 3.05 / 2.90 / 2.86 / 2.84, tree of 16 heavy atoms in 6-31G* at 0.03
+// 14.3 / 13.8 / 13.7 / 13.6, tree of 12 in cc-pVDZ UHF at 0.1 33.6 / 32.6 /
+// 32.0 / 31.7. FP64 builds reduce in the kernel first (1-4%) and keep one.
 constexpr int kAccCopies = 4;
 
 // Destination of a Fock build's device work.  Lane 0 is the job's main

@@ -8,7 +8,7 @@
 // primitive pairs over the union of the exponents, and every Hermite Coulomb
 // table R_tuv is computed once per pair of primitive pairs for all the member
 // shells, where a shell-by-shell build computes it once per contracted
-// quartet (benzene/cc-pVDZ: 1.6e8 primitive quartets become 2.3e7).
+// quartet (benzene/cc-pVDZ: 1.0e8 primitive quartets become 1.4e7).
 #pragma once
 
 #include <cuda_runtime.h>
