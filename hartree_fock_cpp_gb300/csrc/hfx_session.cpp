@@ -217,7 +217,6 @@ void FockSession::relayout()
     const size_t n = (size_t)nmat_;
     for (int s = 0; s < nspin_; ++s) in_[s].alloc(n);
     if (nspin_ == 2) dj_.alloc(n);
-    for (int s = 0; s < nspin_ + 1; ++s) acc_[s].alloc(n);
     for (int s = 0; s < 2 * nspin_ - 1; ++s) out_[s].alloc(n);
     dsh_.alloc((size_t)std::max(1, npairs_));
     tdsh_.alloc((size_t)std::max(1, nsuper_));
@@ -225,6 +224,9 @@ void FockSession::relayout()
     combine(false, plan64_);
     combine(true, plan_mixed_);
     counters_.alloc(std::max<size_t>(1, std::max(plan64_.launches(), plan_mixed_.launches())));
+    // accumulators: copies of them where any build has FP32 launches
+    const size_t na = std::max(acc_copies(plan64_) * acc_stride(plan64_), acc_copies(plan_mixed_) * acc_stride(plan_mixed_));
+    for (int s = 0; s < nspin_ + 1; ++s) acc_[s].alloc(na);
     cuda_check(cudaStreamSynchronize(stream_), "session layout");
     dirty_ = false;
 }
@@ -372,7 +374,9 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
     const Combined& c = mixed_plan ? plan_mixed_ : plan64_;
     const size_t n = (size_t)nmat_;
     StreamSink sk(stream_, aux_, fork_ev_, aux_ev_);
-    for (int s = 0; s < nk + 1; ++s) sk.zero(0, acc_[s].p, n * sizeof(double));
+    int ncopy = (int)acc_copies(c);
+    long long cstride = (long long)acc_stride(c);
+    for (int s = 0; s < nk + 1; ++s) sk.zero(0, acc_[s].p, ncopy * cstride * sizeof(double));
     const double* Dj = in_[0].p;
     const double* Dk = in_[0].p;
     const double* Dk2 = nullptr;
@@ -469,7 +473,7 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
         KernelSpec ks;
         if (g.kind == 0) {
             SmallArgs<float> a{pairs32_.p, anchor32_.p, tasks + g.off, (int)g.n, boys32_.p, thr_,
-                               J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p, 1, 0};
+                               J, Kx, Kx2, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p, ncopy, cstride};
             cuda_check(small_spec_f32(g.pcb, g.pck, nk, (int)g.n, &ks), "session small-class kernel");
             void* prm[] = {&a};
             sk.kernel(lane, ks, prm);
@@ -477,7 +481,7 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
             cuda_check(warp_spec(nk, g.grid, g.warps_per_cta, g.slice, &ks), "session warp kernel");
             WarpArgs<float> a{pairs32_.p, anchor32_.p, pct_.p, abs_.p, kh_.p, kl_.p, tasks + g.off, (int)g.n,
                               ctr + gi, boys32_.p, thr_, J, Kx, Kx2, g.slice,
-                              g.lane_min_npp, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p, 1, 0};
+                              g.lane_min_npp, Dsh, dthr, active, Dj32, Dk32, Dk232, anchor32_.p, ncopy, cstride};
             void* prm[] = {&a};
             sk.kernel(lane, ks, prm);
         }
@@ -488,10 +492,6 @@ void FockSession::launch(int nk, bool mixed_plan, double dthr)
     const int* fk = fk_.p;
     const long long* fm = fmoff_.p;
     const int nf = (int)live_.size();
-    // one copy of the accumulators: more were measured on single jobs only
-    // (kAccCopies), not on a session's merged launches
-    int ncopy = 1;
-    long long cstride = 0;
     if (nk == 1) {
         const double* jp = acc_[0].p;
         const double* kp = acc_[1].p;

@@ -79,6 +79,9 @@ private:
         size_t launches() const { return groups.size() + team.groups.size(); }
     };
 
+    // accumulator copies of a build (kAccCopies beside FP32 launches) and their distance
+    size_t acc_copies(const Combined& c) const { return c.groups.empty() ? 1 : kAccCopies; }
+    size_t acc_stride(const Combined& c) const { return c.groups.empty() ? (size_t)nmat_ : ((size_t)nmat_ + 31) & ~(size_t)31; }
     void relayout();                      // combined tables of the live members (mu_ held)
     void combine(bool mixed_plan, Combined& c);
     void combine_team(bool mixed_plan, Combined& c);
